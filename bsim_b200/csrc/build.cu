@@ -553,10 +553,23 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     // loops of both phases see every SM
     e.block = e.opt.block_threads > 0 ? e.opt.block_threads : 512;
     if (e.block % 32 != 0 || e.block > 512) return fail(BSIM_ERR_ARG, "block_threads must be a multiple of 32 <= 512");
-    const size_t smem = step_dynamic_smem(a, e.block);
-    if (smem > 0) CK(step_set_smem(e.opt.accumulate, smem));
+    // 4 entry pairs in flight per lane; fewer where that lets two blocks share an SM (or one fit)
     int bps = 0;
-    CK(step_occupancy(e.block, e.opt.accumulate, &bps, smem));
+    for (int depth = 4, best = 0; depth >= 2; depth--) {
+        StepArgs b = a;
+        b.tile_depth = depth;
+        const size_t sm = step_dynamic_smem(b, e.block);
+        int n = 0;
+        if (sm > 0 && step_set_smem(e.opt.accumulate, sm) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        CK(step_occupancy(e.block, e.opt.accumulate, &n, sm));
+        if (n > best) {
+            best = bps = n;
+            a.tile_depth = depth;
+        }
+    }
     if (bps < 1) return fail(BSIM_ERR_LIMIT, "step kernel does not fit on an SM with this tile size");
     e.grid = e.opt.grid_blocks > 0 ? e.opt.grid_blocks : e.sm_count * bps;
     CK(cudaDeviceSynchronize());
@@ -615,23 +628,23 @@ struct TileHost {
     std::vector<int32_t> tile_beg, tile_run_off, tile_units, run_n, run_unit0;
     std::vector<float> tile_scale;
     std::vector<uint32_t> run_src0;
-    std::vector<int64_t> run_pair0;
+    std::vector<int64_t> run_seg0;
     int32_t tile_max = 0;
 };
 
 // Appends a run of sources [src0, src0 + n) to tile q (the last tile so far).
-static void add_run(TileHost &th, uint32_t src0, int32_t n, int64_t pair0, int32_t D)
+static void add_run(TileHost &th, uint32_t src0, int32_t n, int64_t seg0, int32_t D)
 {
     const int32_t q = (int32_t)th.tile_units.size() - 1;
     th.run_src0.push_back(src0);
     th.run_n.push_back(n);
-    th.run_pair0.push_back(pair0);
+    th.run_seg0.push_back(seg0);
     th.run_unit0.push_back(th.tile_units[q]);
     th.tile_units[q] += ((n + 31) / 32) * D;
     th.tile_run_off[q + 1] = (int32_t)th.run_src0.size();
 }
 
-// Uploads the tile tables (pair and entry arrays are uploaded by the caller)
+// Uploads the tile tables (segment and entry arrays are uploaded by the caller)
 // and points the step arguments at them.
 static int upload_tiles(Engine &e, const TileHost &th)
 {
@@ -657,7 +670,7 @@ static int upload_tiles(Engine &e, const TileHost &th)
     if (nr) {
         CK(cudaMemcpy(d_rs, th.run_src0.data(), 4 * nr, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_rn, th.run_n.data(), 4 * nr, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(d_rp, th.run_pair0.data(), 8 * nr, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(d_rp, th.run_seg0.data(), 8 * nr, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_ru, th.run_unit0.data(), 4 * nr, cudaMemcpyHostToDevice));
     }
     a.n_tiles = nt;
@@ -670,35 +683,52 @@ static int upload_tiles(Engine &e, const TileHost &th)
     a.tile_units = d_tu;
     a.run_src0 = d_rs;
     a.run_n = d_rn;
-    a.run_pair0 = d_rp;
+    a.run_seg0 = d_rp;
     a.run_unit0 = d_ru;
     return BSIM_OK;
 }
 
-// Segment starts of every (pair, delay) in 16-byte entry pairs, relative to the
-// first entry pair of the pair's tile (so each tile, not the whole copy, must
-// stay below 2^32 entry pairs), from the pair offsets and the per-delay
-// cumulative counts (all even).
-__global__ void tile_seg0_kernel(const int64_t *pair_base, const int64_t *tile_pair0, int32_t nt, int64_t n_pairs,
-                                 int64_t *tile_seg0)
+// One run of a tile as the set-up kernels see it. The tiled copy is ordered by
+// (tile, run, delay, source): the 32 sources of a work unit have their segment
+// starts in one 128-byte line and their entries next to one another.
+struct TileRun {
+    int64_t pair0;  // (run, source) pairs before the run's
+    int64_t seg0;   // index in seg_off of (delay 1, first source)
+    int64_t base;   // the tile's first 16-byte entry pair
+    int32_t n, D;   // sources, delays (the tile's own network's)
+    int32_t T;      // targets of the tile
+};
+
+static __device__ __forceinline__ int find_run(const TileRun *runs, int n_runs, int64_t k)
 {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nt; q += gridDim.x * blockDim.x)
-        tile_seg0[q] = tile_pair0[q] < n_pairs ? (pair_base[tile_pair0[q]] >> 1) : 0;
+    int lo = 0, hi = n_runs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (runs[mid].pair0 <= k) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
 }
 
-__global__ void pair_seg_kernel(const int64_t *pair_base, const uint16_t *pair_doff, int64_t n_pairs, int D,
-                                const int64_t *tile_pair0, int32_t nt, const int64_t *tile_seg0, uint32_t *pair_seg)
+// Entry pairs of every tile (64 bits) from the segments' counts.
+__global__ void tile_total_kernel(const uint32_t *cnt, const int64_t *tile_idx0, int32_t nt, unsigned long long *total)
 {
-    const int64_t n = n_pairs * (D + 1);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t k = i / (D + 1);
-        int lo = 0, hi = nt - 1;  // the tile whose pair range holds k
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile_pair0[mid] <= k) lo = mid;
-            else hi = mid - 1;
-        }
-        pair_seg[i] = (uint32_t)(((pair_base[k] + pair_doff[i]) >> 1) - tile_seg0[lo]);
+    for (int q = blockIdx.x; q < nt; q += gridDim.x) {
+        unsigned long long s = 0;
+        for (int64_t i = tile_idx0[q] + threadIdx.x; i < tile_idx0[q + 1]; i += blockDim.x) s += cnt[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0 && s) atomicAdd(&total[q], s);
+    }
+}
+
+// The scan over all tiles wraps at 2^32; each tile's starts become relative to its first
+// entry pair, so that each tile (not the whole copy) stays below 2^32 entry pairs.
+__global__ void tile_rebase_kernel(uint32_t *seg_off, const int64_t *tile_idx0, int32_t nt, const int64_t *tile_seg0)
+{
+    for (int q = blockIdx.x; q < nt; q += gridDim.x) {
+        const uint32_t b = (uint32_t)tile_seg0[q];
+        for (int64_t i = tile_idx0[q] + threadIdx.x; i < tile_idx0[q + 1]; i += blockDim.x) seg_off[i] -= b;
     }
 }
 
@@ -709,29 +739,23 @@ __global__ void pair_seg_kernel(const int64_t *pair_base, const uint16_t *pair_d
 // a bank serialise. Each segment of up to TILE_SPREAD_MAX entries is reordered so
 // that its first entries (even positions) and its second entries (odd positions)
 // each cycle through distinct banks: every bank's entries are split between the
-// two halves, and each half is laid out bank by bank in rounds. The counter word
-// of an entry is its target (E) or 2 x tile size + target (I), so the bank is
-// that index mod 32. A padding entry stays last (the second entry of its pair).
+// two halves, and each half is laid out bank by bank in rounds. A padding entry
+// stays last (the second entry of its pair).
 #ifndef TILE_BANK_SPREAD
 #define TILE_BANK_SPREAD 1
 #endif
 #define TILE_SPREAD_MAX 256
 #define SPREAD_WARPS 8
 
-static __device__ __forceinline__ int entry_bank(uint2 v, int T)
-{
-    const float w = __uint_as_float(v.y);
-    return (int)((v.x + (w >= 0.0f ? 0u : 2u * (unsigned)T)) & 31u);
-}
+static __device__ __forceinline__ int entry_bank(uint2 v) { return (int)((v.x >> 2) & 31u); }
 
-// One warp per (tile, source) pair, the lanes working on one segment at a time:
+// One warp per (run, source) pair, the lanes working on one segment at a time:
 // each entry takes a rank within its bank (shared-memory atomics, so the order
 // inside a bank is arbitrary: it changes nothing), lane b splits bank b's entries
 // between the halves, and each entry computes its place from the 32 banks' counts.
-__global__ void __launch_bounds__(32 * SPREAD_WARPS) tile_spread_kernel(uint2 *ent, const int64_t *pair_base,
-                                                                      const uint16_t *pair_doff, int64_t n_pairs,
-                                                                      int D, const int64_t *tile_pair0,
-                                                                      const int32_t *tile_size, int32_t nt)
+__global__ void __launch_bounds__(32 * SPREAD_WARPS) tile_spread_kernel(uint2 *ent, const uint32_t *seg_off,
+                                                                      const TileRun *runs, int32_t n_runs,
+                                                                      int64_t n_pairs)
 {
     __shared__ uint8_t s_bank[SPREAD_WARPS][TILE_SPREAD_MAX];
     __shared__ uint16_t s_rank[SPREAD_WARPS][TILE_SPREAD_MAX];
@@ -743,23 +767,20 @@ __global__ void __launch_bounds__(32 * SPREAD_WARPS) tile_spread_kernel(uint2 *e
     int *cnt = s_cnt[wib], *nes = s_ne[wib];
     for (int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n_pairs;
          k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        int lo = 0, hi = nt - 1;  // the tile whose pair range holds k
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile_pair0[mid] <= k) lo = mid;
-            else hi = mid - 1;
-        }
-        const int T = tile_size[lo];
-        for (int d = 0; d < D; d++) {
-            const int64_t b0 = pair_base[k] + pair_doff[k * (D + 1) + d];
-            const int L = (int)(pair_doff[k * (D + 1) + d + 1] - pair_doff[k * (D + 1) + d]);
+        const TileRun rn = runs[find_run(runs, n_runs, k)];
+        for (int d = 0; d < rn.D; d++) {
+            const int64_t at = rn.seg0 + (int64_t)d * rn.n + (k - rn.pair0);
+            const uint32_t p0 = seg_off[at];
+            const int64_t b0 = 2 * (rn.base + (int64_t)p0);
+            const int64_t L64 = 2 * (int64_t)(seg_off[at + 1] - p0);
+            const int L = (int)(L64 > TILE_SPREAD_MAX ? TILE_SPREAD_MAX + 1 : L64);
             if (L <= 2 || L > TILE_SPREAD_MAX) continue;  // nothing to spread, or kept in target order
-            const int pad = ent[b0 + L - 1].x == TILE_PAD ? 1 : 0;
+            const int pad = ent[b0 + L - 1].y == TILE_PAD_W ? 1 : 0;
             const int nreal = L - pad, half = L / 2;
             cnt[lane] = 0;
             __syncwarp();
             for (int i = lane; i < nreal; i += 32) {
-                const int bk = entry_bank(ent[b0 + i], T);
+                const int bk = entry_bank(ent[b0 + i]);
                 bank[i] = (uint8_t)bk;
                 rank[i] = (uint16_t)atomicAdd(&cnt[bk], 1);
             }
@@ -800,39 +821,28 @@ __global__ void __launch_bounds__(32 * SPREAD_WARPS) tile_spread_kernel(uint2 *e
     }
 }
 
-// tile_pair0: [nt + 1] first pair of each tile (pairs are grouped by tile); tile_beg: [nt + 1]
-// first target of each tile.
-static int make_pair_seg(Engine &e, int64_t n_pairs, const std::vector<int64_t> &tile_pair0,
-                         const std::vector<int32_t> &tile_beg)
+static int spread_tiles(Engine &e, const std::vector<TileRun> &runs, int64_t n_pairs)
 {
-    const int32_t nt = (int32_t)tile_pair0.size() - 1;
-    for (int32_t q = 0; q < nt && q < (int32_t)e.tile_entries.size(); q++)
-        if (e.tile_entries[q] / 2 > (int64_t)UINT32_MAX)
-            return fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries");
-    uint32_t *d_seg;
-    int64_t *d_seg0, *d_tp0;
-    TRY(dalloc(e, &d_seg, (size_t)n_pairs * (e.D + 1)));
-    TRY(dalloc(e, &d_seg0, std::max<int32_t>(nt, 1)));
-    TRY(dalloc(e, &d_tp0, nt + 1));
-    CK(cudaMemcpy(d_tp0, tile_pair0.data(), sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice));
-    if (nt > 0) tile_seg0_kernel<<<e.sm_count, 256, 0, e.stream>>>(e.a.pair_base, d_tp0, nt, n_pairs, d_seg0);
-    if (n_pairs > 0 && nt > 0)
-        pair_seg_kernel<<<e.sm_count * 4, 256, 0, e.stream>>>(e.a.pair_base, e.a.pair_doff, n_pairs, e.D, d_tp0, nt,
-                                                             d_seg0, d_seg);
-    if (TILE_BANK_SPREAD && n_pairs > 0 && nt > 0) {
-        std::vector<int32_t> size(nt);
-        for (int32_t q = 0; q < nt; q++) size[q] = tile_beg[q + 1] - tile_beg[q];
-        int32_t *d_size;
-        TRY(dalloc(e, &d_size, nt));
-        CK(cudaMemcpy(d_size, size.data(), sizeof(int32_t) * nt, cudaMemcpyHostToDevice));
+    if (!TILE_BANK_SPREAD || n_pairs <= 0 || runs.empty()) return BSIM_OK;
+    TileRun *d_runs = nullptr;
+    CK(cudaMalloc((void **)&d_runs, sizeof(TileRun) * runs.size()));
+    cudaError_t st = cudaMemcpy(d_runs, runs.data(), sizeof(TileRun) * runs.size(), cudaMemcpyHostToDevice);
+    if (st == cudaSuccess) {
         tile_spread_kernel<<<e.sm_count * 8, 32 * SPREAD_WARPS, 0, e.stream>>>(
-            const_cast<uint2 *>(e.a.ent), e.a.pair_base, e.a.pair_doff, n_pairs, e.D, d_tp0, d_size, nt);
+            const_cast<uint2 *>(e.a.ent), e.a.seg_off, d_runs, (int32_t)runs.size(), n_pairs);
+        st = cudaStreamSynchronize(e.stream);
     }
-    CK(cudaStreamSynchronize(e.stream));
-    CK(cudaGetLastError());
-    e.a.pair_seg = d_seg;
-    e.a.tile_seg0 = d_seg0;
+    cudaFree(d_runs);
+    if (st == cudaSuccess) st = cudaGetLastError();
+    if (st != cudaSuccess) return fail(BSIM_ERR_CUDA, std::string("tiled copy: ") + cudaGetErrorString(st));
     return BSIM_OK;
+}
+
+// {counter offset, scaled weight} of one synapse onto target `tgt` of a tile of T targets.
+static inline uint2 tile_entry(int64_t tgt, int32_t T, float w, float scale)
+{
+    const float ws = w * scale;  // a power of two
+    return make_uint2(4u * (uint32_t)(tgt + (w >= 0.0f ? 0 : 2 * (int64_t)T)), w == 0.0f ? 0u : f2u(ws));
 }
 
 // Host construction of the tiled copy: target ranges follow population (and
@@ -872,36 +882,9 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
         dm = std::max(dm, delay[k]);
     }
     auto tile_D = [&](int32_t q) { return dmax_inst[inst ? inst[th.tile_beg[q]] : 0]; };
-    std::vector<int64_t> pair_base;
-    std::vector<uint16_t> pair_doff;
-    std::vector<uint2> ent;
-    ent.reserve((size_t)s + (size_t)s / 8 + 16);
-    const uint2 pad = make_uint2(TILE_PAD, TILE_PAD);
-    std::vector<int64_t> cnt(D);
-    int32_t cur_d = -1;
-    auto close_group = [&]() {  // pads the current (pair, delay) segment to even length
-        if (cur_d >= 0 && (cnt[cur_d] & 1)) {
-            ent.push_back(pad);
-            cnt[cur_d]++;
-        }
-        cur_d = -1;
-    };
-    int32_t cur_tile = -1;
-    int64_t cur_src = -1, run_start_src = -1, run_pair0 = 0;
-    bool pair_overflow = false;
-    auto close_pair = [&]() {
-        int64_t c = 0;
-        for (int d = 0; d <= D; d++) {
-            pair_doff.push_back((uint16_t)c);
-            if (d < D) c += cnt[d];
-        }
-        pair_overflow |= c > 65535;
-        std::fill(cnt.begin(), cnt.end(), 0);
-    };
-    auto close_run = [&]() {
-        if (run_start_src >= 0)
-            add_run(th, (uint32_t)run_start_src, (int32_t)(cur_src - run_start_src + 1), run_pair0, tile_D(cur_tile));
-    };
+    // runs of consecutive sources, from the (tile, source) order
+    std::vector<TileRun> runs_d;
+    std::vector<int64_t> tile_idx0(nt + 1, 0);
     auto open_tiles_until = [&](int32_t q) {
         while ((int32_t)th.tile_units.size() <= q) {
             th.tile_units.push_back(0);
@@ -909,58 +892,95 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
             th.tile_run_off[qq + 1] = th.tile_run_off[qq];
         }
     };
-    for (int64_t pos = 0; pos < s; pos++) {
-        const int64_t k = key[pos].second;
+    int64_t n_pairs = 0, n_seg = 0;
+    for (int64_t pos = 0; pos < s;) {
         const int32_t q = (int32_t)(key[pos].first >> 37);
-        if (q != cur_tile || src[k] != cur_src || delay[k] - 1 != cur_d) close_group();
-        if (q != cur_tile || src[k] != cur_src) {
-            if (cur_src >= 0) close_pair();
-            const bool extends = q == cur_tile && src[k] == cur_src + 1;
-            if (!extends) {
-                if (cur_tile >= 0) close_run();
-                open_tiles_until(q);
-                run_start_src = src[k];
-                run_pair0 = (int64_t)pair_base.size();
-            }
-            cur_tile = q;
-            cur_src = src[k];
-            pair_base.push_back((int64_t)ent.size());
+        const int64_t src0 = src[key[pos].second];
+        int64_t last = src0, end = pos + 1;
+        for (; end < s && (int32_t)(key[end].first >> 37) == q; end++) {
+            const int64_t sc = src[key[end].second];
+            if (sc > last + 1) break;
+            last = sc;
         }
-        cur_d = delay[k] - 1;
-        cnt[cur_d]++;
-        ent.push_back(make_uint2((uint32_t)(dst[k] - th.tile_beg[q]), f2u(weight[k])));
+        open_tiles_until(q);
+        const int32_t n_r = (int32_t)(last - src0 + 1), D_r = tile_D(q);
+        TileRun rn{n_pairs, n_seg, 0, n_r, D_r, th.tile_beg[q + 1] - th.tile_beg[q]};
+        runs_d.push_back(rn);
+        add_run(th, (uint32_t)src0, n_r, n_seg, D_r);
+        n_pairs += n_r;
+        n_seg += (int64_t)n_r * D_r + 1;
+        tile_idx0[q + 1] = n_seg;
+        pos = end;
     }
-    close_group();
-    if (cur_src >= 0) {
-        close_pair();
-        close_run();
-    }
-    e.tile_entries.assign(nt, 0);
-    for (int32_t q = 0; q < nt; q++)
-        for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++)
-            for (int32_t i = 0; i < th.run_n[r]; i++)
-                e.tile_entries[q] += pair_doff[(size_t)(th.run_pair0[r] + i) * (D + 1) + D];
     open_tiles_until(nt - 1);
+    for (int32_t q = 0; q < nt; q++) tile_idx0[q + 1] = std::max(tile_idx0[q + 1], tile_idx0[q]);
+    // entries per segment, then starts in 16-byte pairs from the tile's first one
+    std::vector<uint32_t> seg_off(n_seg, 0);
+    auto seg_at = [&](const TileRun &rn, uint32_t src0, int64_t k) {
+        return rn.seg0 + (int64_t)(delay[k] - 1) * rn.n + (src[k] - (int64_t)src0);
+    };
+    auto for_each = [&](auto &&body) {  // synapses in (tile, source, delay) order with their run
+        size_t r = 0;
+        int32_t q = 0;
+        for (int64_t pos = 0; pos < s; pos++) {
+            const int64_t k = key[pos].second;
+            const int32_t qk = (int32_t)(key[pos].first >> 37);
+            while (q < qk) r = (size_t)th.tile_run_off[++q];
+            while ((int64_t)src[k] >= (int64_t)th.run_src0[r] + th.run_n[r]) r++;
+            body(r, q, k);
+        }
+    };
+    for_each([&](size_t r, int32_t, int64_t k) { seg_off[seg_at(runs_d[r], th.run_src0[r], k)]++; });
+    bool pair_overflow = false;
+    for (const TileRun &rn : runs_d)
+        for (int64_t i = 0; i < rn.n; i++) {
+            int64_t c = 0;
+            for (int32_t d = 0; d < rn.D; d++) c += (seg_off[rn.seg0 + (int64_t)d * rn.n + i] + 1) & ~1u;
+            pair_overflow |= c > 65535;
+        }
     if (pair_overflow) return fail(BSIM_ERR_LIMIT, "tiled delivery: a source has more than 65535 synapses into one tile");
-    int64_t *d_pb;
-    uint16_t *d_pd;
-    uint2 *d_ent;
-    TRY(dalloc(e, &d_pb, pair_base.size()));
-    TRY(dalloc(e, &d_pd, pair_doff.size()));
-    TRY(dalloc(e, &d_ent, ent.size()));
-    if (!pair_base.empty()) {
-        CK(cudaMemcpy(d_pb, pair_base.data(), 8 * pair_base.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(d_pd, pair_doff.data(), 2 * pair_doff.size(), cudaMemcpyHostToDevice));
+    std::vector<int64_t> tile_seg0(nt, 0);
+    e.tile_entries.assign(nt, 0);
+    int64_t at = 0;
+    for (int32_t q = 0; q < nt; q++) {
+        tile_seg0[q] = at;
+        for (int64_t i = tile_idx0[q]; i < tile_idx0[q + 1]; i++) {
+            const int64_t pairs = (seg_off[i] + 1) / 2;
+            seg_off[i] = (uint32_t)(at - tile_seg0[q]);
+            at += pairs;
+        }
+        e.tile_entries[q] = 2 * (at - tile_seg0[q]);
+        if (at - tile_seg0[q] > (int64_t)UINT32_MAX)
+            return fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries");
+        for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++) runs_d[r].base = tile_seg0[q];
     }
+    std::vector<uint2> ent(2 * (size_t)at);
+    {
+        int64_t cur_seg = -1, cur = 0;
+        for_each([&](size_t r, int32_t q, int64_t k) {
+            const int64_t sg = seg_at(runs_d[r], th.run_src0[r], k);
+            if (sg != cur_seg) {
+                cur_seg = sg;
+                cur = 2 * (tile_seg0[q] + (int64_t)seg_off[sg]);
+            }
+            const uint2 v = tile_entry(dst[k] - th.tile_beg[q], runs_d[r].T, weight[k], th.tile_scale[q]);
+            ent[cur++] = v;
+            if (cur & 1) ent[cur] = make_uint2(v.x, TILE_PAD_W);  // padding, unless another entry follows
+        });
+    }
+    uint32_t *d_seg;
+    int64_t *d_ts;
+    uint2 *d_ent;
+    TRY(dalloc(e, &d_seg, seg_off.size()));
+    TRY(dalloc(e, &d_ts, nt));
+    TRY(dalloc(e, &d_ent, ent.size()));
+    if (!seg_off.empty()) CK(cudaMemcpy(d_seg, seg_off.data(), 4 * seg_off.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_ts, tile_seg0.data(), 8 * nt, cudaMemcpyHostToDevice));
     if (!ent.empty()) CK(cudaMemcpy(d_ent, ent.data(), sizeof(uint2) * ent.size(), cudaMemcpyHostToDevice));
-    e.a.pair_base = d_pb;
-    e.a.pair_doff = d_pd;
+    e.a.seg_off = d_seg;
+    e.a.tile_seg0 = d_ts;
     e.a.ent = d_ent;
-    // pairs are grouped by tile: a tile's first pair is its first run's
-    std::vector<int64_t> tile_pair0(nt + 1, (int64_t)pair_base.size());
-    for (int32_t q = nt - 1; q >= 0; q--)
-        tile_pair0[q] = th.tile_run_off[q] < th.tile_run_off[q + 1] ? th.run_pair0[th.tile_run_off[q]] : tile_pair0[q + 1];
-    TRY(make_pair_seg(e, (int64_t)pair_base.size(), tile_pair0, th.tile_beg));
+    TRY(spread_tiles(e, runs_d, n_pairs));
     return upload_tiles(e, th);
 }
 
@@ -1135,6 +1155,8 @@ __global__ void gen_pull_kernel(GenDev g, int64_t N, int64_t *col_cnt_or_off, ui
 // population that lie in the tile. Its pairs are pair_start + source index.
 struct TileSeg {
     int64_t pair_start;
+    int64_t seg0;       // index in seg_off of (delay 1, source 0)
+    int64_t base;       // the tile's first 16-byte entry pair (pass 1)
     uint64_t pseed;
     int64_t src_base;   // global id of source 0
     int32_t j0, j1;     // target range, local to the target population
@@ -1143,7 +1165,8 @@ struct TileSeg {
     uint32_t p24, exc24;
     float w_exc, w_inh;
     int32_t d_inst;     // the network's max delay
-    int32_t sign;       // -1: all synapses; 0: excitatory only (w >= 0); 1: inhibitory only
+    int32_t T;          // targets of the tile
+    float scale;        // 2^qexp of the network
 };
 
 static __device__ __forceinline__ int find_seg(const TileSeg *segs, int n_segs, int64_t k)
@@ -1157,13 +1180,11 @@ static __device__ __forceinline__ int find_seg(const TileSeg *segs, int n_segs, 
     return lo;
 }
 
-// One warp per (tile, source) pair. Pass 0: per-delay counts -> cumulative
-// pair_doff and pair_cnt (each delay's segment padded to even length). Pass 1:
-// entries in delay order, targets ascending.
+// One warp per (run, source) pair. Pass 0: entry pairs of each delay's segment (padded to
+// even length). Pass 1: the entries, targets ascending inside a segment, and the padding.
 template <int PASS>
-__global__ void gen_tile_kernel(const TileSeg *segs, int n_segs, int64_t n_pairs, int D,
-                                int64_t *pair_cnt, uint16_t *pair_doff, const int64_t *pair_base,
-                                uint2 *ent)
+__global__ void gen_tile_kernel(const TileSeg *segs, int n_segs, int64_t n_pairs, uint32_t *seg_cnt,
+                                const uint32_t *seg_off, uint2 *ent)
 {
     __shared__ long long s_cur[8][GEN_MAX_DELAY];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1172,35 +1193,37 @@ __global__ void gen_tile_kernel(const TileSeg *segs, int n_segs, int64_t n_pairs
          k += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const TileSeg sg = segs[find_seg(segs, n_segs, k)];
         const int64_t i = k - sg.pair_start;
-        uint16_t *doff = pair_doff + k * (D + 1);
-        for (int d = lane; d < D; d += 32) cur[d] = PASS == 0 ? 0 : pair_base[k] + doff[d];
+        const int64_t at0 = sg.seg0 + i;
+        for (int d = lane; d < sg.d_inst; d += 32)
+            cur[d] = PASS == 0 ? 0 : 2 * (sg.base + (long long)seg_off[at0 + (int64_t)d * sg.n_src]);
         __syncwarp();
         for (int j0 = sg.j0; j0 < sg.j1; j0 += 32) {
             const int j = j0 + lane;
             SynDraw sd;
-            bool conn = j < sg.j1 && draw_pair(sg.pseed, (uint64_t)i, (uint64_t)j, sg.p24, sg.exc24, sg.w_exc,
-                                               sg.w_inh, sg.d_inst, &sd);
-            if (conn && sg.sign >= 0) conn = (sd.w >= 0.0f) == (sg.sign == 0);
+            const bool conn = j < sg.j1 && draw_pair(sg.pseed, (uint64_t)i, (uint64_t)j, sg.p24, sg.exc24, sg.w_exc,
+                                                     sg.w_inh, sg.d_inst, &sd);
             if (!__ballot_sync(0xffffffffu, conn)) continue;
             const unsigned same = __match_any_sync(0xffffffffu, conn ? sd.d : -1);
             if (conn) {
                 const int leader = __ffs(same) - 1;
                 const long long at = cur[sd.d - 1] + __popc(same & ((1u << lane) - 1u));
-                if (PASS == 1) ent[at] = make_uint2((uint32_t)(sg.tgt_off + (j - sg.j0)), __float_as_uint(sd.w));
+                if (PASS == 1) {
+                    const unsigned tgt = (unsigned)(sg.tgt_off + (j - sg.j0));
+                    ent[at] = make_uint2(4u * (tgt + (sd.w >= 0.0f ? 0u : 2u * (unsigned)sg.T)),
+                                         sd.w == 0.0f ? 0u : __float_as_uint(__fmul_rn(sd.w, sg.scale)));
+                }
                 __syncwarp(same);
                 if (lane == leader) cur[sd.d - 1] += __popc(same);
             }
             __syncwarp();
         }
         __syncwarp();
-        if (PASS == 0 && lane == 0) {
-            // segments padded to even length (the padding entries are preset)
-            long long c = 0;
-            for (int d = 0; d <= D; d++) {
-                doff[d] = (uint16_t)c;
-                if (d < D) c += (cur[d] + 1) & ~1ll;
+        for (int d = lane; d < sg.d_inst; d += 32) {
+            if (PASS == 0) {
+                seg_cnt[at0 + (int64_t)d * sg.n_src] = (uint32_t)((cur[d] + 1) >> 1);
+            } else if (cur[d] < 2 * (sg.base + (long long)seg_off[at0 + (int64_t)d * sg.n_src + 1])) {
+                ent[cur[d]] = make_uint2(ent[cur[d] - 1].x, TILE_PAD_W);
             }
-            pair_cnt[k] = c;
         }
         __syncwarp();
     }
@@ -1397,11 +1420,11 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         th.tile_max = tile_max;
         th.tile_scale.resize(nt);
         th.tile_run_off.assign(nt + 1, 0);
-        int64_t pairs = 0;
-        std::vector<int64_t> tile_pair0(nt + 1, 0);
+        int64_t pairs = 0, n_seg = 0;
+        std::vector<int64_t> tile_idx0(nt + 1, 0);
+        std::vector<TileRun> runs_d;
         for (int32_t q = 0; q < nt; q++) {
             const int32_t qu = q;
-            tile_pair0[q] = pairs;
             int k = 0;
             while (k + 1 < ns && gi[k + 1].nbase <= tile_beg[qu]) k++;
             const GenInst &x = gi[k];
@@ -1417,6 +1440,8 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
                 for (int id : pl.in[pp]) {
                     TileSeg sg;
                     sg.pair_start = pairs;
+                    sg.seg0 = n_seg;
+                    sg.base = 0;
                     sg.pseed = pl.proj[id].pseed;
                     sg.src_base = x.nbase + (int64_t)pl.proj[id].src_pop * x.n;
                     sg.j0 = j0;
@@ -1428,52 +1453,73 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
                     sg.w_exc = x.w_exc;
                     sg.w_inh = x.w_inh;
                     sg.d_inst = x.D;
-                    sg.sign = -1;
+                    sg.T = tile_beg[qu + 1] - tile_beg[qu];
+                    sg.scale = th.tile_scale[q];
                     segs.push_back(sg);
-                    add_run(th, (uint32_t)sg.src_base, x.n, pairs, x.D);  // the network's own delay range
+                    runs_d.push_back(TileRun{pairs, n_seg, 0, x.n, x.D, sg.T});
+                    add_run(th, (uint32_t)sg.src_base, x.n, n_seg, x.D);  // the network's own delay range
                     pairs += x.n;
+                    n_seg += (int64_t)x.n * x.D + 1;
                 }
             }
+            tile_idx0[q + 1] = n_seg;
         }
-        tile_pair0[nt] = pairs;
         TileSeg *d_segs;
-        int64_t *d_pcnt;
+        int64_t *d_idx0;
+        unsigned long long *d_total;
         if ((rc = talloc((void **)&d_segs, sizeof(TileSeg) * std::max<size_t>(1, segs.size()))) ||
-            (rc = talloc((void **)&d_pcnt, sizeof(int64_t) * (pairs + 1)))) { free_tmp(); return bail(rc); }
+            (rc = talloc((void **)&d_idx0, sizeof(int64_t) * (nt + 1))) ||
+            (rc = talloc((void **)&d_total, sizeof(unsigned long long) * nt))) { free_tmp(); return bail(rc); }
         if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
-        int64_t *d_pb; uint16_t *d_pd;
-        if ((rc = dalloc(E, &d_pb, pairs + 1)) || (rc = dalloc(E, &d_pd, (size_t)pairs * (D + 1)))) {
-            free_tmp();
-            return bail(rc);
-        }
-        gen_tile_kernel<0><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, D, d_pcnt, d_pd, nullptr,
-                                                    nullptr);
-        cudaMemcpyAsync(d_pb, d_pcnt, sizeof(int64_t) * pairs, cudaMemcpyDeviceToDevice, E.stream);
-        if ((rc = scan(d_pb, pairs))) { free_tmp(); return bail(rc); }
-        int64_t n_ent = 0;
-        cudaMemcpyAsync(&n_ent, d_pb + pairs, 8, cudaMemcpyDeviceToHost, E.stream);
+        cudaMemcpy(d_idx0, tile_idx0.data(), sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice);
+        uint32_t *d_seg;
+        int64_t *d_seg0;
+        if ((rc = dalloc(E, &d_seg, n_seg)) || (rc = dalloc(E, &d_seg0, nt))) { free_tmp(); return bail(rc); }
+        cudaMemsetAsync(d_seg, 0, sizeof(uint32_t) * n_seg, E.stream);
+        cudaMemsetAsync(d_total, 0, sizeof(unsigned long long) * nt, E.stream);
+        gen_tile_kernel<0><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, d_seg, nullptr, nullptr);
+        tile_total_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_total);
+        std::vector<unsigned long long> total(nt, 0);
+        cudaMemcpyAsync(total.data(), d_total, sizeof(unsigned long long) * nt, cudaMemcpyDeviceToHost, E.stream);
         if (cudaStreamSynchronize(E.stream) != cudaSuccess) {
             free_tmp();
             return bail(fail(BSIM_ERR_CUDA, "generator: tiled copy sizes"));
         }
-        uint2 *d_ent;
-        if ((rc = dalloc(E, &d_ent, n_ent))) { free_tmp(); return bail(rc); }
-        cudaMemsetAsync(d_ent, 0xff, sizeof(uint2) * n_ent, E.stream);  // padding: target 0xffffffff
-        gen_tile_kernel<1><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, D, d_pcnt, d_pd, d_pb, d_ent);
-        // entries per tile from the pair offsets at the tiles' first pairs
-        std::vector<int64_t> pb_at(nt + 1, 0);
-        for (int32_t q = 0; q <= nt; q++)
-            cudaMemcpyAsync(&pb_at[q], d_pb + tile_pair0[q], 8, cudaMemcpyDeviceToHost, E.stream);
-        if (cudaStreamSynchronize(E.stream) != cudaSuccess || pb_at[nt] != n_ent) {
-            free_tmp();
-            return bail(fail(BSIM_ERR_CUDA, "generator: tiled copy does not match its sizes"));
-        }
+        std::vector<int64_t> tile_seg0(nt, 0);
+        int64_t ent_pairs = 0;
         E.tile_entries.resize(nt);
-        for (int32_t q = 0; q < nt; q++) E.tile_entries[q] = pb_at[q + 1] - pb_at[q];
-        E.a.pair_base = d_pb;
-        E.a.pair_doff = d_pd;
+        for (int32_t q = 0; q < nt; q++) {
+            if (total[q] > (unsigned long long)UINT32_MAX) {
+                free_tmp();
+                return bail(fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries"));
+            }
+            tile_seg0[q] = ent_pairs;
+            E.tile_entries[q] = 2 * (int64_t)total[q];
+            ent_pairs += (int64_t)total[q];
+            for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++)
+                segs[r].base = runs_d[r].base = tile_seg0[q];
+        }
+        cudaMemcpy(d_seg0, tile_seg0.data(), sizeof(int64_t) * nt, cudaMemcpyHostToDevice);
+        if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
+        if (n_seg > 0) {  // starts from the counts, wrapping at 2^32, then relative to the tile
+            size_t tb = 0;
+            cub::DeviceScan::ExclusiveSum(nullptr, tb, d_seg, d_seg, n_seg, E.stream);
+            void *d_tb;
+            if ((rc = talloc(&d_tb, tb))) { free_tmp(); return bail(rc); }
+            cub::DeviceScan::ExclusiveSum(d_tb, tb, d_seg, d_seg, n_seg, E.stream);
+            tile_rebase_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_seg0);
+        }
+        uint2 *d_ent;
+        if ((rc = dalloc(E, &d_ent, 2 * ent_pairs))) { free_tmp(); return bail(rc); }
+        gen_tile_kernel<1><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, nullptr, d_seg, d_ent);
+        if (cudaStreamSynchronize(E.stream) != cudaSuccess) {
+            free_tmp();
+            return bail(fail(BSIM_ERR_CUDA, "generator: tiled copy"));
+        }
+        E.a.seg_off = d_seg;
+        E.a.tile_seg0 = d_seg0;
         E.a.ent = d_ent;
-        if ((rc = make_pair_seg(E, pairs, tile_pair0, tile_beg))) { free_tmp(); return bail(rc); }
+        if ((rc = spread_tiles(E, runs_d, pairs))) { free_tmp(); return bail(rc); }
         if ((rc = upload_tiles(E, th))) { free_tmp(); return bail(rc); }
     }
     // push rows (not needed when every step uses the tiled copy)
@@ -1984,14 +2030,21 @@ __global__ void pop_in_from_counts_kernel(StepArgs a, const int32_t *indeg, doub
 
 __global__ void pop_degree_tiles_kernel(StepArgs a, double *in_sum, double *out_sum, int want_in, int want_out)
 {
-    // one block per tile: entries per pair give out-degree of the source and in-degree of the tile
+    // one block per tile: entries per (run, source) give out-degree of the source and in-degree of the tile
     for (int q = blockIdx.x; q < a.n_tiles; q += gridDim.x) {
+        const uint2 *ent = a.ent + 2 * a.tile_seg0[q];
         for (int r = a.tile_run_off[q]; r < a.tile_run_off[q + 1]; r++) {
-            for (int i = threadIdx.x; i < a.run_n[r]; i += blockDim.x) {
-                const int64_t k = a.run_pair0[r] + i;
-                const int64_t b = a.pair_base[k], n_e = a.pair_doff[k * (a.D + 1) + a.D];
+            const int n_r = a.run_n[r], chunks = (n_r + 31) >> 5;
+            const int units = (r + 1 < a.tile_run_off[q + 1] ? a.run_unit0[r + 1] : a.tile_units[q]) - a.run_unit0[r];
+            const int D_r = units / chunks;
+            for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
                 int64_t real = 0;
-                for (int64_t x = 0; x < n_e; x++) real += a.ent[b + x].x != TILE_PAD;
+                for (int d = 0; d < D_r; d++) {
+                    const uint32_t *so = a.seg_off + a.run_seg0[r] + (int64_t)d * n_r + i;
+                    const int64_t x1 = 2 * (int64_t)so[1];
+                    const int64_t x0 = 2 * (int64_t)so[0];
+                    if (x1 > x0) real += x1 - x0 - (ent[x1 - 1].y == TILE_PAD_W ? 1 : 0);
+                }
                 const double c = (double)real;
                 const uint32_t src = a.run_src0[r] + i;
                 if (want_out) atomicAdd(&out_sum[a.ctab[a.cls[src]].pop], c);

@@ -11,7 +11,9 @@
 
 namespace bsim {
 
-constexpr uint32_t TILE_PAD = 0xffffffffu;  // target of a padding entry of the tiled copy
+// Weight word of a padding entry of the tiled copy (-0.0f: adds nothing; a synapse's
+// own zero weight is stored as +0.0f there).
+constexpr uint32_t TILE_PAD_W = 0x80000000u;
 
 // One neuron class. For LIF_brian neurons: a folded parameter tuple, the
 // per-population part of LIFENeuron::reset's output (src/neuron/lif/LIFENeuron.cpp:68-112);
@@ -130,17 +132,17 @@ struct StepArgs {
     const int32_t *tile_units;       // [n_tiles] work units: sum over runs of ceil(n/32) * D
     const uint32_t *run_src0;        // [runs] first source
     const int32_t *run_n;            // [runs] sources in the run
-    const int64_t *run_pair0;        // [runs] pair of the first source
+    const int64_t *run_seg0;         // [runs] index in seg_off of the run's (delay 1, first source)
     const int32_t *run_unit0;        // [runs] first work unit, counted within the tile
-    const int64_t *pair_base;        // [P] first entry of each pair
-    const uint16_t *pair_doff;       // [P][D + 1] cumulative entry counts by delay (padded to even)
-    const uint32_t *pair_seg;        // [P][D + 1] each delay's segment start in 16-byte entry pairs,
-                                     // (pair_base + pair_doff) / 2 - tile_seg0[tile]; the last one is
-                                     // the pair's end
+    const uint32_t *seg_off;         // per run [tile's delays][run_n] and one more: start of each (delay,
+                                     // source) segment in 16-byte entry pairs from the tile's first one;
+                                     // a segment ends where the next one starts
     const int64_t *tile_seg0;        // [n_tiles] first 16-byte entry pair of each tile
-    const uint2 *ent;                // [E] {target within the tile, weight bits}; every (pair, delay)
-                                     // segment starts on an even entry and has even length
-                                     // (padding entries have target 0xffffffff)
+    const uint2 *ent;                // [E] {byte offset of the target's low counter word in the tile's
+                                     // counters (E or I by the weight's sign), weight x 2^qexp}; every
+                                     // segment starts on an even entry and has even length (padding
+                                     // entries have the weight word TILE_PAD_W and any offset)
+    int32_t tile_depth;              // 16-byte entry pairs a lane keeps in flight (2..4)
     // firing predictor (needs pop_hist)
     const float *mlp;                // [BSIM_MLP_PARAMS] (NULL: off)
     const int32_t *pop_size;         // [n_pops]

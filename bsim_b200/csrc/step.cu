@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "engine.h"
 
 namespace bsim {
@@ -463,13 +465,26 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // left. The first block to finish a piece of a tile stores its sums into the
 // tile's accumulator plane; the others add theirs after that store.
 //
-// The tile's synapses are grouped by (source, delay) and its sources form runs
-// of consecutive ids. A work unit is (run, delay d, 32-source chunk): one lane
-// reads the chunk's word of the fired bitmap of cycle t-d. Each fired
-// (source, delay) names one segment of 8-byte entries ({target offset in the
-// tile, weight bits}), padded to an even length from an even start; a warp
-// gathers up to TILE_SEGS segments and streams them as one flat range of
-// 16-byte entry pairs, each lane advancing its own segment cursor.
+// The tile's sources form runs of consecutive ids; its synapses are grouped by
+// (run, delay, source). A work unit is (run, delay d, 32-source chunk): one lane
+// reads the chunk's word of the fired bitmap of cycle t-d. Each fired (source,
+// delay) names one segment of 8-byte entries, padded to an even length from an
+// even start. A warp lists up to 32 segments at a time, one per lane, and streams
+// them as one flat range of 16-byte entry pairs: pair k of the range goes to lane
+// k % 32, which finds its segment from the warp's start marks (one warp-wide OR
+// and a population count per 32 pairs), fetches the pair with cp.async into its own
+// slot of a small ring in shared memory, and adds it a few pairs later. The ring
+// keeps copies in flight across listings without holding registers.
+//
+// What bounds it: the entry stream (8 bytes per event) and the issue slots of the
+// additions. An entry holds the byte offset of its counter and its weight already
+// scaled to fixed point, so an addition is a conversion, two shared atomics and a
+// carry; a padding entry adds zero instead of branching. Measured against listing
+// two segments per lane at a time and four register loads per lane with the sign,
+// scale and padding worked out per entry (us per cycle): 50 x 5,000 with 50-step
+// delays 296 -> 171, 16 uneven networks 455 -> 312, 50 x 10,000 with 20-step delays
+// 168 -> 128, 25 x 10,000 106 -> 92, 100 x 10,000 210 -> 201 (bound by HBM while it
+// streams).
 //
 // Exact int64 sums with 32-bit shared atomics: the low word of the fixed-point
 // value is added with an atomic that returns the old word, and the high word
@@ -484,40 +499,57 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 #ifndef TILE_WAIT_SPINS
 #define TILE_WAIT_SPINS (1u << 22)  // ~0.3 s of 64 ns sleeps: far beyond any store phase
 #endif
-#ifndef TILE_SEGS
-#define TILE_SEGS 64  // fired segments a warp lists per round
-#endif
-static_assert(TILE_SEGS >= 32 && TILE_SEGS <= 64, "a round's segment prefix covers two entries per lane");
 #ifndef TILE_CHUNK_PAIRS
 #define TILE_CHUNK_PAIRS 512  // entry pairs a chunk of units should list (from the previous cycle's rate)
 #endif
 #ifndef TILE_MIN_CHUNK
 #define TILE_MIN_CHUNK 8ll  // units per chunk at least
 #endif
-#ifndef TILE_INFLIGHT
-#define TILE_INFLIGHT 4  // 16-byte entry pairs per lane loaded before they are added
-#endif
+// shared memory of one warp: the ring (depth x 32 pairs) and the segments' bases
+#define TILE_WARP_BYTES(depth) ((depth) * 512 + 32 * 4)
 
 // Counters are [4][tile]: E low, E high, I low, I high words (word-major, so
 // lanes adding into scattered targets spread over all shared-memory banks).
-static __device__ __forceinline__ void carry_add(unsigned *lo, int T, long long v)
-{
-    const unsigned long long u = (unsigned long long)v;
-    const unsigned l = (unsigned)u, h = (unsigned)(u >> 32);
-    const unsigned old = atomicAdd(lo, l);
-    atomicAdd(lo + T, h + (old + l < old ? 1u : 0u));
-}
-
 // Two entries at once: both low words first, so the second atomic's latency
 // overlaps the first's (a returned value is waited for only where it is used).
-static __device__ __forceinline__ void carry_add2(unsigned *lo0, long long v0, unsigned *lo1, long long v1, int T)
+static __device__ __forceinline__ void carry_add2(char *acc, uint4 v, int hi)
 {
-    const unsigned long long u0 = (unsigned long long)v0, u1 = (unsigned long long)v1;
+    const unsigned long long u0 = (unsigned long long)__float2ll_rn(__uint_as_float(v.y));
+    const unsigned long long u1 = (unsigned long long)__float2ll_rn(__uint_as_float(v.w));
     const unsigned l0 = (unsigned)u0, l1 = (unsigned)u1;
-    const unsigned o0 = atomicAdd(lo0, l0);
-    const unsigned o1 = atomicAdd(lo1, l1);
-    atomicAdd(lo0 + T, (unsigned)(u0 >> 32) + (o0 + l0 < o0 ? 1u : 0u));
-    atomicAdd(lo1 + T, (unsigned)(u1 >> 32) + (o1 + l1 < o1 ? 1u : 0u));
+    unsigned *p0 = reinterpret_cast<unsigned *>(acc + v.x), *p1 = reinterpret_cast<unsigned *>(acc + v.z);
+    const unsigned o0 = atomicAdd(p0, l0);
+    const unsigned o1 = atomicAdd(p1, l1);
+    atomicAdd(p0 + hi, (unsigned)(u0 >> 32) + (o0 + l0 < o0 ? 1u : 0u));
+    atomicAdd(p1 + hi, (unsigned)(u1 >> 32) + (o1 + l1 < o1 ? 1u : 0u));
+}
+
+// One 16-byte copy to shared memory, past L1 and evict-first in L2 (read once per
+// spike); `bytes` = 0 writes zeros and reads nothing.
+static __device__ __forceinline__ void copy16_async(unsigned dst, const uint4 *src, int bytes, unsigned long long pol)
+{
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst), "l"(src), "r"(bytes),
+                 "l"(pol)
+                 : "memory");
+}
+static __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+static __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The position of the n-th (from 0) set bit of m.
+static __device__ __forceinline__ int nth_set_bit(unsigned m, int n)
+{
+    int b = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc(m & ((1u << w) - 1u));
+        if (n >= c) {
+            n -= c;
+            m >>= w;
+            b += w;
+        }
+    }
+    return b;
 }
 
 static __device__ __forceinline__ long long carry_sum(const unsigned *lo, int T)
@@ -526,13 +558,17 @@ static __device__ __forceinline__ long long carry_sum(const unsigned *lo, int T)
 }
 
 static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &a, unsigned long long t, int pw,
-                                                                unsigned *s_acc, long long *s_start, int *s_cum,
-                                                                int *s_part)
+                                                                unsigned *s_acc, char *s_warp, int *s_part)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int D = a.D;
-    long long *seg_start = s_start + warp * TILE_SEGS;
-    int *seg_cum = s_cum + warp * TILE_SEGS;
+    const int depth = a.tile_depth;
+    char *mine = s_warp + (size_t)warp * TILE_WARP_BYTES(depth);
+    uint4 *ring = reinterpret_cast<uint4 *>(mine) + lane;                   // [depth][32]: this lane's slots
+    unsigned *seg_base = reinterpret_cast<unsigned *>(mine + depth * 512);  // [32]
+    const unsigned ring_sh = (unsigned)__cvta_generic_to_shared(ring);
+    const unsigned lanes_le = 0xffffffffu >> (31 - lane);
+    unsigned long long pol;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
     unsigned long long ev = 0;
     unsigned long long *s_best = reinterpret_cast<unsigned long long *>(s_part + 2);
     // the counters start at zero once per launch; each part's flush clears what it read,
@@ -575,8 +611,7 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
         const int4 part = a.parts[pi];  // {tile, first unit, end unit, part within the tile}
         const int q = part.x, u_end = part.z;
         const int tb = a.tile_beg[q], T = a.tile_beg[q + 1] - tb;
-        const float sc = a.tile_scale[q];
-        const long long seg0 = a.tile_seg0[q];  // the tile's first entry pair
+        const uint4 *ent = reinterpret_cast<const uint4 *>(a.ent) + a.tile_seg0[q];  // the tile's entry pairs
         const int r0 = a.tile_run_off[q], r1 = a.tile_run_off[q + 1];
         // the warps of every block working on the part take chunks of its units as they become
         // free: 32 units (one per lane), fewer where the part listed many entry pairs per unit in
@@ -587,6 +622,16 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                                   : (int)max(TILE_MIN_CHUNK, min(32ll, (long long)TILE_CHUNK_PAIRS * (u_end - part.y) /
                                                                             (long long)prev));
         unsigned listed = 0;
+        int pads = 0;
+        int head = 0, held = 0;  // ring: next slot to fill, slots filled and not yet added
+        auto add_oldest = [&]() {
+            int k = head - held;
+            if (k < 0) k += depth;
+            const uint4 v = ring[k * 32];
+            if (v.y | v.w) carry_add2(reinterpret_cast<char *>(s_acc), v, T);  // zeros past a listing's end add nothing
+            pads += v.w == TILE_PAD_W;
+            held--;
+        };
         for (;;) {
             int ub = 0;
             if (lane == 0) ub = (int)atomicAdd(a.part_next + pi, (unsigned)cs);
@@ -594,17 +639,20 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
             if (ub >= u_end) break;
             const int u = ub + lane;
             unsigned m = 0;
-            int64_t kbase = 0;
-            int d = 1;
+            const uint32_t *off = a.seg_off;  // the unit's 32 segment starts
             if (lane < cs && u < u_end) {
-                int r = r0;
-                while (r + 1 < r1 && a.run_unit0[r + 1] <= u) r++;
-                const int n_r = a.run_n[r], chunks = (n_r + 31) >> 5;
-                const int v = u - a.run_unit0[r];
-                d = v / chunks + 1;
+                int lo = r0, hi = r1 - 1;  // the run that holds unit u
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (a.run_unit0[mid] <= u) lo = mid;
+                    else hi = mid - 1;
+                }
+                const int n_r = a.run_n[lo], chunks = (n_r + 31) >> 5;
+                const int v = u - a.run_unit0[lo];
+                const int d = v / chunks + 1;
                 const int c = v - (d - 1) * chunks;
                 if ((long long)t - d >= 0) {
-                    const int64_t s_first = (int64_t)a.run_src0[r] + 32 * c;
+                    const int64_t s_first = (int64_t)a.run_src0[lo] + 32 * c;
                     const int len = min(32, n_r - 32 * c);
                     const uint32_t *bm = a.bitmap + (int64_t)((t - d) % (unsigned long long)a.R) * a.W;
                     const int64_t wi = s_first >> 5;
@@ -612,103 +660,73 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                     unsigned bits = bm[wi];
                     if (sh) bits = (bits >> sh) | ((wi + 1 < a.W ? bm[wi + 1] : 0u) << (32 - sh));
                     m = len == 32 ? bits : (bits & ((1u << len) - 1u));
-                    kbase = a.run_pair0[r] + 32 * c;
+                    off += a.run_seg0[lo] + (int64_t)(d - 1) * n_r + 32 * c;
                 }
             }
-            while (__any_sync(0xffffffffu, m != 0)) {
-                // this round: up to TILE_SEGS fired (source, delay) segments of the warp
-                const int cnt = __popc(m);
-                int incl = cnt;
+            const int cnt = __popc(m);
+            int incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int nb = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += nb;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            for (int b0 = 0; b0 < total; b0 += 32) {
+                // this lane's segment: fired source number b0 + lane of the chunk
+                const int rank = b0 + lane;
+                int ul = 0;  // the lane whose unit holds it
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, ul + w - 1) <= rank) ul += w;
+                const unsigned mu = __shfl_sync(0xffffffffu, m, ul);
+                const int eu = __shfl_sync(0xffffffffu, incl - cnt, ul);
+                const unsigned long long ou = __shfl_sync(0xffffffffu, (unsigned long long)off, ul);
+                unsigned first = 0;
+                int len = 0;
+                if (rank < total) {
+                    const uint32_t *o = reinterpret_cast<const uint32_t *>(ou) + nth_set_bit(mu, rank - eu);
+                    first = __ldg(o);
+                    len = (int)(__ldg(o + 1) - first);
+                }
+                int excl = len;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const int nb = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += nb;
+                    const int nb = __shfl_up_sync(0xffffffffu, excl, o);
+                    if (lane >= o) excl += nb;
                 }
-                const int excl = incl - cnt;
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                const int take = max(0, min(cnt, TILE_SEGS - excl));
-                // the lane's fired segments, two at a time: both offset loads are issued
-                // before either is used (more at once costs registers the streaming loop needs)
-                for (int i = 0; i < take; i += 2) {
-                    const int b0 = __ffs(m) - 1;
-                    m &= m - 1;
-                    const bool two = i + 1 < take;
-                    const int b1 = two ? __ffs(m) - 1 : b0;
-                    if (two) m &= m - 1;
-                    // in 16-byte units: segments start on an even entry and have even length
-                    const uint32_t *p0 = a.pair_seg + (kbase + b0) * (D + 1) + (d - 1);
-                    const uint32_t *p1 = a.pair_seg + (kbase + b1) * (D + 1) + (d - 1);
-                    const uint32_t x0 = p0[0], y0 = p0[1], x1 = p1[0], y1 = p1[1];
-                    seg_start[excl + i] = seg0 + (long long)x0;
-                    seg_cum[excl + i] = (int)(y0 - x0);  // length for now
-                    if (two) {
-                        seg_start[excl + i + 1] = seg0 + (long long)x1;
-                        seg_cum[excl + i + 1] = (int)(y1 - x1);
-                    }
-                }
-                __syncwarp();
-                const int nseg = min(total, TILE_SEGS);
-                // inclusive prefix of the segment lengths (two per lane)
-                int c0 = lane < nseg ? seg_cum[lane] : 0;
-                int c1 = lane + 32 < nseg ? seg_cum[lane + 32] : 0;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int n0 = __shfl_up_sync(0xffffffffu, c0, o);
-                    const int n1 = __shfl_up_sync(0xffffffffu, c1, o);
-                    if (lane >= o) {
-                        c0 += n0;
-                        c1 += n1;
-                    }
-                }
-                const int half = __shfl_sync(0xffffffffu, c0, 31);
-                __syncwarp();
-                if (lane < nseg) seg_cum[lane] = c0;
-                if (lane + 32 < nseg) seg_cum[lane + 32] = half + c1;
-                __syncwarp();
-                const int n_pairs = seg_cum[nseg - 1];  // 16-byte entry pairs of the round
+                const int n_pairs = __shfl_sync(0xffffffffu, excl, 31);  // 16-byte entry pairs of the round
+                excl -= len;
                 listed += (unsigned)n_pairs;
-                const uint4 *ent2 = reinterpret_cast<const uint4 *>(a.ent);
-                // this lane's segment cursor (its flat positions only grow): the current
-                // segment's end, its first flat position and its first entry pair, in registers
-                int j = 0, seg_end = seg_cum[0], seg_first = 0;
-                long long seg_base = seg_start[0];
-                for (int f0 = 0; f0 < n_pairs; f0 += TILE_INFLIGHT * 32) {
-                    uint4 v[TILE_INFLIGHT];
-#pragma unroll
-                    for (int uu = 0; uu < TILE_INFLIGHT; uu++) {
-                        const int f = f0 + uu * 32 + lane;
-                        if (f < n_pairs) {
-                            while (seg_end <= f) {
-                                seg_first = seg_end;
-                                j++;
-                                seg_end = seg_cum[j];
-                                seg_base = seg_start[j];
-                            }
-                            v[uu] = ld_stream16(ent2 + seg_base + (f - seg_first));
-                        }
-                    }
-#pragma unroll
-                    for (int uu = 0; uu < TILE_INFLIGHT; uu++) {
-                        if (f0 + uu * 32 + lane < n_pairs) {
-                            // the sign routes the input as LIFENeuron::recv does; padding (only
-                            // ever the second entry of a pair) is skipped
-                            const float w0 = __uint_as_float(v[uu].y), w1 = __uint_as_float(v[uu].w);
-                            unsigned *c0 = s_acc + (w0 >= 0.0f ? 0 : 2 * T) + (int)v[uu].x;
-                            const long long q0 = __float2ll_rn(__fmul_rn(w0, sc));
-                            if (v[uu].z != TILE_PAD) {
-                                carry_add2(c0, q0, s_acc + (w1 >= 0.0f ? 0 : 2 * T) + (int)v[uu].z,
-                                           __float2ll_rn(__fmul_rn(w1, sc)), T);
-                                ev += 2;
-                            } else {
-                                carry_add(c0, T, q0);
-                                ev += 1;
-                            }
-                        }
+                // segments that hold entries, in lane order: flat position + base = pair of the tile
+                const unsigned full = __ballot_sync(0xffffffffu, len > 0);
+                __syncwarp();
+                if (len > 0) seg_base[__popc(full & lanes_le) - 1] = first - (unsigned)excl;
+                __syncwarp();
+                if (len == 0) excl = -64;  // marks nothing
+                int seg = -1;              // segments that started before the 32 positions
+                for (int f0 = 0; f0 < n_pairs; f0 += 32) {
+                    const unsigned at = (unsigned)(excl - f0);
+                    const unsigned marks = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+                    const int f = f0 + lane;
+                    const unsigned base = seg_base[seg + __popc(marks & lanes_le)];
+                    seg += __popc(marks);
+                    copy16_async(ring_sh + head * 512, ent + (base + (unsigned)f), f < n_pairs ? 16 : 0, pol);
+                    copy_commit();
+                    if (++head == depth) head = 0;
+                    if (++held == depth) {
+                        if (depth == 4) copy_wait<3>();
+                        else if (depth == 3) copy_wait<2>();
+                        else copy_wait<1>();
+                        add_oldest();
                     }
                 }
-                __syncwarp();
             }
         }
+        copy_wait<0>();
+        while (held > 0) add_oldest();
+        // every listed pair holds two entries, but for the padding
+        if (lane == 0) ev += 2ull * listed;
+        ev -= (unsigned long long)pads;
         if (lane == 0 && listed) atomicAdd(pairs_cnt, listed);
         __syncthreads();
         // Flush into the tile's one accumulator plane. The first block to finish a piece of
@@ -900,14 +918,15 @@ static __device__ __forceinline__ void record_phase(const StepArgs &a, unsigned 
 template <int ACC>
 __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel(const __grid_constant__ StepArgs a)
 {
-    __shared__ long long s_cum[BSIM_MAX_DELAY + 1];
-    __shared__ PushSeg s_seg[MAX_WARPS * PUSH_CHUNK];
     __shared__ int s_wcnt[128];
     __shared__ unsigned long long s_ev;
     __shared__ __align__(8) int s_part[4];  // tiled delivery: the block's part; [2..3] the best part to join
     __shared__ int s_last;
-    // tiled delivery: [4][tile] u32 limb counters (one sign), then per-warp segment lists
+    // tiled delivery: [4][tile] u32 counters, then each warp's ring and segment bases; push: the
+    // warps' segment tables, then the delay window's spike counts (step_dynamic_smem)
     extern __shared__ __align__(16) unsigned long long s_dyn[];
+    PushSeg *s_seg = reinterpret_cast<PushSeg *>(s_dyn);
+    long long *s_cum = reinterpret_cast<long long *>(s_seg + MAX_WARPS * PUSH_CHUNK);
     // a raised error flag stops every later cycle (block-uniform test)
     if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
     const unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
@@ -939,9 +958,8 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     if (push) {
         ev = push_phase(a, t, p ^ 1, s_cum, s_seg);
     } else if (tiled) {
-        long long *starts = reinterpret_cast<long long *>(s_dyn + 2 * a.tile_max);
-        int *cums = reinterpret_cast<int *>(starts + (blockDim.x >> 5) * TILE_SEGS);
-        ev = tile_phase(a, t, p ^ 1, reinterpret_cast<unsigned *>(s_dyn), starts, cums, s_part);
+        ev = tile_phase(a, t, p ^ 1, reinterpret_cast<unsigned *>(s_dyn),
+                        reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part);
     } else {
         ev = pull_phase<ACC>(a, t, p ^ 1);
     }
@@ -1013,12 +1031,14 @@ __global__ void record_flush_kernel(const StepArgs a)
     }
 }
 
-// Dynamic shared memory of the step kernel: the tile accumulators and the
-// per-warp segment lists of tiled delivery (0 when no tiles are built).
+// Dynamic shared memory of the step kernel: push delivery's tables, or the tile
+// counters and the warps' rings where they are larger (one mode runs per cycle).
 size_t step_dynamic_smem(const StepArgs &a, int block)
 {
-    if (a.n_tiles == 0) return 0;
-    return (size_t)4 * a.tile_max * sizeof(unsigned) + (size_t)(block / 32) * TILE_SEGS * (sizeof(long long) + sizeof(int));
+    size_t bytes = MAX_WARPS * PUSH_CHUNK * sizeof(PushSeg) + ((size_t)a.D + 1) * sizeof(long long);
+    if (a.n_tiles > 0)
+        bytes = std::max(bytes, (size_t)4 * a.tile_max * sizeof(unsigned) + (size_t)(block / 32) * TILE_WARP_BYTES(a.tile_depth));
+    return bytes;
 }
 
 // The attribute belongs to the kernel, not to an engine: it only ever grows,
@@ -1054,7 +1074,7 @@ cudaError_t launch_step(Engine &e)
 // One step on explicit arguments (used by the allocation-free entry point).
 cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream_t stream)
 {
-    step_kernel<BSIM_ACC_EXACT><<<grid, block, 0, stream>>>(a);
+    step_kernel<BSIM_ACC_EXACT><<<grid, block, step_dynamic_smem(a, block), stream>>>(a);
     return cudaGetLastError();
 }
 
