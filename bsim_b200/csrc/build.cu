@@ -23,10 +23,18 @@ namespace bsim {
 
 cudaError_t launch_step(Engine &e);
 cudaError_t launch_record_flush(Engine &e);
+int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count);
+cudaError_t launch_loop(Engine &e, int steps);
+cudaError_t launch_loop_enter(Engine &e);
+cudaError_t launch_loop_leave(Engine &e);
 cudaError_t step_occupancy(int block, int accumulate, int *blocks_per_sm);
 cudaError_t step_occupancy(int block, int accumulate, int *blocks_per_sm, size_t smem);
 size_t step_dynamic_smem(const StepArgs &a, int block);
 cudaError_t step_set_smem(int accumulate, size_t bytes);
+
+#ifndef LOOP_STEPS
+#define LOOP_STEPS 4096  // cycles of one many-cycle launch at most
+#endif
 
 static thread_local std::string g_err;
 
@@ -344,7 +352,7 @@ static int create_from_arrays(const float *params, const uint8_t *kind, int64_t 
     int64_t *d_row;
     uint2 *d_syn;
     if ((rc = dalloc(*e, &d_state, n)) || (rc = dalloc(*e, &d_vtmp, n)) || (rc = dalloc(*e, &d_cls, n)) ||
-        (rc = dalloc(*e, &d_row, nrows + 1)) || (rc = dalloc(*e, &d_syn, s))) {
+        (rc = dalloc(*e, &d_row, nrows + 1)) || (rc = dalloc(*e, &d_syn, s + 1))) {  // +1: read in pairs
         free_engine(e);
         return rc;
     }
@@ -448,7 +456,10 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     StepArgs &a = e.a;
     a.N = e.N;
     a.D = e.D;
-    a.R = e.D + 2;
+    // small networks run many cycles per launch, unless the caller fixes the launch shape; the push
+    // form clears two cycles' counters ahead
+    e.loop = e.opt.block_threads > 0 || e.opt.grid_blocks > 0 ? 0 : loop_form(e.opt, e.N, e.D, e.sm_count);
+    a.R = e.D + (e.loop == 1 ? 4 : 2);
     a.cap = e.N;
     a.W = (e.N + 31) / 32;
     ClassParams *d_ctab;
@@ -530,12 +541,20 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     a.fire_count = d_fc;
     a.err = d_err;
     unsigned long long *d_ctr;
-    TRY(dalloc(e, &d_ctr, 4));
-    CK(cudaMemset(d_ctr, 0, sizeof(unsigned long long) * 4));
+    TRY(dalloc(e, &d_ctr, 48));  // the many-cycle launch's counters in cache lines of their own
+    CK(cudaMemset(d_ctr, 0, sizeof(unsigned long long) * 48));
     a.step_ctr = d_ctr;
     a.events = d_ctr + 1;
     a.ticket = reinterpret_cast<unsigned int *>(d_ctr + 2);
     a.part_ctr = reinterpret_cast<unsigned int *>(d_ctr + 3);
+    a.loop_bar = d_ctr + 16;
+    if (e.loop == 1) {
+        a.acc_R = e.D + 3;
+        longlong2 *d_ar;
+        TRY(dalloc(e, &d_ar, (size_t)a.acc_R * e.N));
+        TRY(dalloc(e, &a.loop_ev, a.acc_R));
+        a.acc_ring = d_ar;
+    }
     a.delivery = (e.opt.delivery == BSIM_DELIVERY_PULL || e.opt.delivery == BSIM_DELIVERY_AUTO) ? e.opt.delivery
                                                                                                  : BSIM_DELIVERY_PUSH;
     a.deliv_sel = nullptr;
@@ -1526,7 +1545,7 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
     if (!(tiles && E.opt.delivery == BSIM_DELIVERY_TILE)) {
         const int64_t nrows = N * (int64_t)D;
         int64_t *d_row; uint2 *d_syn;
-        if ((rc = dalloc(E, &d_row, nrows + 1)) || (rc = dalloc(E, &d_syn, S))) { free_tmp(); return bail(rc); }
+        if ((rc = dalloc(E, &d_row, nrows + 1)) || (rc = dalloc(E, &d_syn, S + 1))) { free_tmp(); return bail(rc); }
         gen_push_kernel<0><<<gb, 256, 0, E.stream>>>(gd, N, d_row, nullptr);
         if ((rc = scan(d_row, nrows))) { free_tmp(); return bail(rc); }
         gen_push_kernel<1><<<gb, 256, 0, E.stream>>>(gd, N, d_row, d_syn);
@@ -1656,6 +1675,26 @@ static int check_err(Engine &e)
     return BSIM_OK;
 }
 
+// Between one launch per cycle and many: the spikes in flight move between step_kernel's
+// accumulators and push_loop_kernel's ring. A recording's last cycle is copied out before (the
+// many-cycle launch leaves none pending).
+static int enter_loop(Engine &e)
+{
+    if (e.in_loop) return BSIM_OK;
+    if (e.a.rec && e.a.rec_ids) CK(launch_record_flush(e));
+    if (e.loop == 1) CK(launch_loop_enter(e));
+    e.in_loop = true;
+    return BSIM_OK;
+}
+
+static int leave_loop(Engine &e)
+{
+    if (!e.in_loop) return BSIM_OK;
+    if (e.loop == 1) CK(launch_loop_leave(e));
+    e.in_loop = false;
+    return BSIM_OK;
+}
+
 int bsim_run_async(bsim_engine *eh, int64_t steps)
 {
     if (!eh || steps < 0) return fail(BSIM_ERR_ARG, "bsim_run: invalid arguments");
@@ -1663,6 +1702,17 @@ int bsim_run_async(bsim_engine *eh, int64_t steps)
     CK(cudaSetDevice(e.device));
     int64_t left = steps;
     const int gl = e.opt.graph_steps;
+    const bool ordered = e.opt.accumulate == BSIM_ACC_ORDERED;
+    const bool same_mode = e.loop == 1 ? e.a.delivery == BSIM_DELIVERY_PUSH
+                                       : e.loop == 2 && (ordered || e.a.delivery == BSIM_DELIVERY_PULL);
+    if (left > 0 && gl > 0 && same_mode && !e.a.mlp && !e.a.pstats) {
+        TRY(enter_loop(e));
+        for (int k; left > 0; left -= k) {  // bounded, so that a launch ends within a second
+            k = (int)std::min<int64_t>(left, LOOP_STEPS);
+            CK(launch_loop(e, k));
+        }
+    }
+    if (left > 0) TRY(leave_loop(e));
     if (gl > 0 && left >= gl) {
         if (!e.graph_exec || e.graph_len != gl) {
             if (e.graph_exec) cudaGraphExecDestroy(e.graph_exec);
@@ -2234,6 +2284,8 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
         out->delivery = BSIM_DELIVERY_PULL;
         return BSIM_OK;
     }
+    TRY(leave_loop(e));
+    CK(cudaStreamSynchronize(e.stream));
     if (!e.a.acc_clear) {
         // The trials switch modes, and push adds into the planes: from here on the
         // LIF phase clears them. The parity the next cycle delivers into holds the

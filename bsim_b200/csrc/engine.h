@@ -91,6 +91,11 @@ struct StepArgs {
     unsigned long long *step_ctr;  // current cycle t (device-side, advanced by the last block)
     unsigned int *ticket;          // end-of-step block counter
     unsigned long long *events;    // synaptic events delivered
+    // many cycles per launch (small networks)
+    unsigned long long *loop_bar;     // [2] barrier counters, 128 bytes apart (small networks only)
+    void *acc_ring;                   // [acc_R][N] longlong2: input of cycle c in slot c mod acc_R (push form)
+    unsigned long long *loop_ev;      // [acc_R] events in flight by the cycle that delivers them
+    int32_t acc_R;                    // D + 3
     int32_t *err;                  // device error flag (0 = ok)
     const int32_t *deliv_sel;      // per-step delivery choice written by the predictor (may be NULL)
     int32_t delivery;              // BSIM_DELIVERY_PUSH / _PULL when deliv_sel is NULL
@@ -174,6 +179,10 @@ struct Engine {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     int graph_len = 0;
+    // many cycles per launch: 0 no, 1 push form, 2 pull form; and whether the last cycles ran so
+    // (the push form then has the spikes in flight in acc_ring, not in step_kernel's accumulators)
+    int loop = 0;
+    bool in_loop = false;
     // recording
     int64_t rec_cap_alloc = 0, rec_steps_alloc = 0;
     bool rec_dirty = false;

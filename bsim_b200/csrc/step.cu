@@ -52,8 +52,15 @@ static __device__ __forceinline__ void raise_error(const StepArgs &a, int code) 
 // and reset_poisson_neuron (src/neuron/poisson/poisson.cu:29-31, 9-15). Both
 // ignore their synaptic input, as their recv() does.
 // ---------------------------------------------------------------------------
-static __device__ __forceinline__ void drive_update(const StepArgs &a, int kind, int64_t j, int t,
-                                                 const ClassParams *c, float4 &st, bool &fired)
+// The gap a Poisson neuron draws when it fires at cycle fc.
+static __device__ __forceinline__ int poisson_gap(const StepArgs &a, const ClassParams *c, int64_t j, const float4 &st, int fc)
+{
+    return poisson_draw(poisson_key(a.input_seed, j - __ldg(&c->id_base), fc), st.x, a.vtmp[j], a.ptab);
+}
+
+// gap(fc): what poisson_gap gives for a spike at cycle fc
+template <typename Gap>
+static __device__ __forceinline__ void drive_update(int kind, int t, float4 &st, bool &fired, Gap gap)
 {
     if (kind == BSIM_NEURON_CONSTANT) {
         const int cnt = __float_as_int(st.w);
@@ -65,19 +72,92 @@ static __device__ __forceinline__ void drive_update(const StepArgs &a, int kind,
         const int fc = __float_as_int(st.y);
         if (t == fc && t <= __float_as_int(st.z)) {
             fired = true;
-            const uint64_t key = poisson_key(a.input_seed, j - __ldg(&c->id_base), fc);
-            const long long nxt = (long long)fc + 1 + poisson_draw(key, st.x, a.vtmp[j], a.ptab) +
-                                  __float_as_int(st.w);
+            const long long nxt = (long long)fc + 1 + gap(fc) + __float_as_int(st.w);
             st.y = __int_as_float(nxt > 2147483647LL ? 2147483647 : (int)nxt);
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Phase A: LIF_brian update of a grid-stride share of the neurons.
-// Arithmetic follows LIFENeuron::update term by term with every product and
-// sum rounded on its own (no FMA contraction), as the reference's x86 build
+// Update of one neuron for cycle t with the synaptic input of the cycle.
+// LIF_brian arithmetic follows LIFENeuron::update term by term with every product
+// and sum rounded on its own (no FMA contraction), as the reference's x86 build
 // evaluates it:  v = ((Cm*v + v_tmp) + i_E*C_E) + i_I*C_I.
+// ---------------------------------------------------------------------------
+struct LifConst {
+    float Cm, CE, CI, C_E, C_I, v_thresh, v_reset;
+    int refrac_time;
+};
+static __device__ __forceinline__ LifConst lif_const(const ClassParams *c)
+{
+    return LifConst{__ldg(&c->Cm),  __ldg(&c->CE),       __ldg(&c->CI),      __ldg(&c->C_E),
+                    __ldg(&c->C_I), __ldg(&c->v_thresh), __ldg(&c->v_reset), __ldg(&c->refrac_time)};
+}
+
+static __device__ __forceinline__ void lif_update(const LifConst &k, float vtmp, float inE, float inI, float4 &st,
+                                                  bool &fired)
+{
+    int refrac = __float_as_int(st.w);
+    if (refrac > 0) {
+        refrac -= 1;  // input of this cycle is dropped
+    } else {
+        float v = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(k.Cm, st.x), vtmp), __fmul_rn(st.y, k.C_E)),
+                            __fmul_rn(st.z, k.C_I));
+        float iE = __fmul_rn(k.CE, st.y);
+        float iI = __fmul_rn(k.CI, st.z);
+        if (v >= k.v_thresh) {
+            fired = true;
+            refrac = k.refrac_time - 1;
+            v = k.v_reset;
+        } else {
+            iE = __fadd_rn(iE, inE);
+            iI = __fadd_rn(iI, inI);
+        }
+        st.x = v;
+        st.y = iE;
+        st.z = iI;
+    }
+    st.w = __int_as_float(refrac);
+}
+
+static __device__ __forceinline__ void neuron_update(const StepArgs &a, const ClassParams *c, int64_t j, int t,
+                                                     const float *vtmp, float inE, float inI, float4 &st, bool &fired)
+{
+    const int kind = __ldg(&c->kind);
+    if (kind == BSIM_NEURON_LIF) lif_update(lif_const(c), vtmp[j], inE, inI, st, fired);
+    else  // input is dropped (recv returns 0)
+        drive_update(kind, t, st, fired, [&](int fc) { return poisson_gap(a, c, j, st, fc); });
+}
+
+// The state trace row of cycle t (or -1) and the copy of one neuron into it.
+struct TraceRow {
+    long long k, first, count, steps;
+};
+static __device__ __forceinline__ TraceRow trace_row(const StepArgs &a, unsigned long long t)
+{
+    TraceRow r{-1, 0, 0, 0};
+    if (a.trace) {
+        const TraceCtl tc = *a.trace_ctl;
+        const long long k = (long long)t - tc.t0;
+        if (k >= 0 && k < tc.steps) r = TraceRow{k, tc.first, tc.count, tc.steps};
+    }
+    return r;
+}
+static __device__ __forceinline__ void trace_neuron(const StepArgs &a, const TraceRow &r, int64_t j, const float4 &st,
+                                                    float inE, float inI)
+{
+    if (r.k < 0 || j < r.first || j >= r.first + r.count) return;
+    const int64_t plane = r.steps * r.count;
+    float *row = a.trace + r.k * r.count + (j - r.first);
+    row[0] = st.x;
+    row[plane] = st.y;
+    row[2 * plane] = st.z;
+    row[3 * plane] = inE;
+    row[4 * plane] = inI;
+}
+
+// ---------------------------------------------------------------------------
+// Phase A: update of all neurons, in chunks of one block pass.
 // ---------------------------------------------------------------------------
 // Fired ids are appended to the cycle's ring slot with one global atomic per
 // block and pass: warps publish their ballot counts, warp 0 scans them and
@@ -95,18 +175,7 @@ static __device__ __forceinline__ void lif_phase(const StepArgs &a, unsigned lon
     uint32_t *bm = a.bitmap + (int64_t)cur * a.W;
     int32_t *hist = a.pop_hist ? a.pop_hist + (int64_t)(t % (unsigned long long)a.hist_len) * a.n_pops : nullptr;
     const float *vtmp = (a.drive_half > 0 && ((t / (unsigned long long)a.drive_half) & 1ull)) ? a.vtmp_alt : a.vtmp;
-    // state trace of this cycle: the row, or -1
-    long long tr_k = -1, tr_first = 0, tr_count = 0, tr_steps = 0;
-    if (a.trace) {
-        const TraceCtl tc = *a.trace_ctl;
-        const long long k = (long long)t - tc.t0;
-        if (k >= 0 && k < tc.steps) {
-            tr_k = k;
-            tr_first = tc.first;
-            tr_count = tc.count;
-            tr_steps = tc.steps;
-        }
-    }
+    const TraceRow tr = trace_row(a, t);
     int buf = 0;  // s_wcnt is double-buffered by pass, so a pass needs no closing barrier
     int cb = 0;
     if (threadIdx.x == 0) s_chunk[0] = (long long)atomicAdd(chunk_ctr, (unsigned)blockDim.x);
@@ -126,7 +195,6 @@ static __device__ __forceinline__ void lif_phase(const StepArgs &a, unsigned lon
         int pop = -1;
         if (j < a.N) {
             float4 st = a.state[j];
-            int refrac = __float_as_int(st.w);
             const ClassParams *c = a.ctab + a.cls[j];
             float inE, inI;
             if (ACC == BSIM_ACC_EXACT) {
@@ -148,42 +216,9 @@ static __device__ __forceinline__ void lif_phase(const StepArgs &a, unsigned lon
                 inE = q.x;
                 inI = q.y;
             }
-            const int kind = __ldg(&c->kind);
-            if (kind == BSIM_NEURON_LIF) {
-                if (refrac > 0) {
-                    refrac -= 1;  // input of this cycle is dropped
-                } else {
-                    const float Cm = __ldg(&c->Cm), C_E = __ldg(&c->C_E), C_I = __ldg(&c->C_I);
-                    float v = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(Cm, st.x), vtmp[j]), __fmul_rn(st.y, C_E)),
-                                        __fmul_rn(st.z, C_I));
-                    float iE = __fmul_rn(__ldg(&c->CE), st.y);
-                    float iI = __fmul_rn(__ldg(&c->CI), st.z);
-                    if (v >= __ldg(&c->v_thresh)) {
-                        fired = true;
-                        refrac = __ldg(&c->refrac_time) - 1;
-                        v = __ldg(&c->v_reset);
-                    } else {
-                        iE = __fadd_rn(iE, inE);
-                        iI = __fadd_rn(iI, inI);
-                    }
-                    st.x = v;
-                    st.y = iE;
-                    st.z = iI;
-                }
-                st.w = __int_as_float(refrac);
-            } else {
-                drive_update(a, kind, j, (int)t, c, st, fired);  // input is dropped (recv returns 0)
-            }
+            neuron_update(a, c, j, (int)t, vtmp, inE, inI, st, fired);
             a.state[j] = st;
-            if (tr_k >= 0 && j >= tr_first && j < tr_first + tr_count) {
-                const int64_t plane = tr_steps * tr_count;
-                float *row = a.trace + tr_k * tr_count + (j - tr_first);
-                row[0] = st.x;
-                row[plane] = st.y;
-                row[2 * plane] = st.z;
-                row[3 * plane] = inE;
-                row[4 * plane] = inI;
-            }
+            trace_neuron(a, tr, j, st, inE, inI);
             if (hist) pop = __ldg(&c->pop);
         }
         const unsigned mask = __ballot_sync(0xffffffffu, fired);
@@ -242,6 +277,9 @@ static __device__ __forceinline__ void push_one(const StepArgs &a, unsigned long
 #ifndef PUSH_CHUNK
 #define PUSH_CHUNK 8
 #endif
+#ifndef PUSH_MAX_SPLIT
+#define PUSH_MAX_SPLIT 32  // pieces of one row at most, in cycles with few long rows
+#endif
 // resident blocks of STEP_MAX_THREADS threads the step kernel is compiled for
 // (together they set its register budget: 65,536 / (2 x 512) = 64 per thread)
 #ifndef STEP_MAX_THREADS
@@ -261,15 +299,17 @@ struct PushSeg {
 // s_cum[d] = spikes of cycles t-1 .. t-d (the push work items of delays 1..d).
 // Run by warp 0 before the LIF phase, so its loads overlap the neuron update;
 // the caller's __syncthreads publishes it.
-static __device__ __forceinline__ void delay_window_prefix(const StepArgs &a, unsigned long long t, long long *s_cum)
+template <typename Count>  // Count: spikes of ring slot s
+static __device__ __forceinline__ void delay_window_prefix(const StepArgs &a, unsigned long long t, long long *s_cum,
+                                                           Count count)
 {
     const int lane = threadIdx.x & 31;
-    const int D = a.D;
+    const int D = a.D, cur = (int)(t % (unsigned long long)a.R);
     long long run = 0;
     for (int d0 = 1; d0 <= D; d0 += 32) {
         const int d = d0 + lane;
         long long c = 0;
-        if (d <= D && (long long)t - d >= 0) c = a.ring_cnt[(t - d) % (unsigned long long)a.R];
+        if (d <= D && (long long)t - d >= 0) c = count(cur >= d ? cur - d : cur - d + a.R);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             long long nb = __shfl_up_sync(0xffffffffu, c, o);
@@ -281,30 +321,32 @@ static __device__ __forceinline__ void delay_window_prefix(const StepArgs &a, un
     if (lane == 0) s_cum[0] = 0;
 }
 
+// warp_lin of n_warps: this warp's number among those that deliver; s_seg: the warp's table.
 static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &a, unsigned long long t, int pw,
-                                                                const long long *s_cum, PushSeg *s_seg)
+                                                                const long long *s_cum, PushSeg *seg,
+                                                                long long warp_lin, long long n_warps)
 {
     const int lane = threadIdx.x & 31;
     const int D = a.D;
     const long long total = s_cum[D];
     unsigned long long ev = 0;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc) + 2 * (int64_t)pw * a.n_planes * a.N;
-    const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
     // Segments per warp chunk: PUSH_CHUNK when there are enough for every warp, fewer
     // (down to one) when a cycle has few spikes with long rows, so that more warps
     // share the rows. Chunks go to warps block-interleaved (chunk c to warp c / grid of
     // block c % grid), so a cycle with few chunks still spreads over every SM.
     int pc = PUSH_CHUNK;
     while (pc > 1 && total < (long long)pc * n_warps) pc >>= 1;
-    const long long n_chunks = (total + pc - 1) / pc;
-    const long long warp_lin = (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    // fewer segments than warps: each is cut into `split` pieces of whole pairs
+    const int split = total > 0 && 2 * total <= n_warps ? (int)min(n_warps / total, (long long)PUSH_MAX_SPLIT) : 1;
+    const long long n_chunks = split > 1 ? total * split : (total + pc - 1) / pc;
     for (long long ch = warp_lin; ch < n_chunks; ch += n_warps) {
         // Lanes 0..PUSH_CHUNK-1 each resolve one (spike, delay) segment: its row
         // [r0, r1), split into an odd head entry, 16-byte pairs [p0, p0 + 2*np)
         // and an odd tail entry.
         int64_t r0 = 0, r1 = 0;
         float sc = 0.0f;
-        const long long item = ch * pc + lane;
+        const long long item = split > 1 ? ch / split + lane : ch * pc + lane;
         if (lane < pc && item < total) {
             int lo = 1, hi = D;
             while (lo < hi) {
@@ -314,7 +356,7 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
             }
             const int d = lo;
             const int slot = (int)((t - d) % (unsigned long long)a.R);
-            const int32_t s = a.ring[(int64_t)slot * a.cap + (item - s_cum[d - 1])];
+            const int32_t s = __ldcg(&a.ring[(int64_t)slot * a.cap + (item - s_cum[d - 1])]);
             r0 = a.row_off[(int64_t)s * D + d - 1];
             r1 = a.row_off[(int64_t)s * D + d];
             if (r1 < r0) {  // row offsets not ascending: flag it, skip the row
@@ -322,6 +364,14 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
                 r1 = r0;
             }
             sc = __ldg(&a.ctab[a.cls[s]].scale_up);
+            if (split > 1 && r1 > r0) {  // piece ch % split; inner cuts lie on 16-byte boundaries
+                const int64_t len = r1 - r0, b = r0;
+                const int k = (int)(ch % split);
+                const int64_t lo = (b + len * k / split + 1) & ~1ll, hi = (b + len * (k + 1) / split + 1) & ~1ll;
+                if (k > 0) r0 = lo < r1 ? lo : r1;
+                if (k + 1 < split) r1 = hi < r1 ? hi : r1;
+                if (r0 > r1) r0 = r1;
+            }
             ev += (unsigned long long)(r1 - r0);
         }
         const int64_t p0 = (r0 & 1) && r0 < r1 ? r0 + 1 : r0;  // first entry of the first pair
@@ -334,8 +384,7 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
             const long long nb = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += nb;
         }
-        // the chunk's segment table, in this warp's slice of shared memory
-        PushSeg *seg = s_seg + (threadIdx.x >> 5) * PUSH_CHUNK;
+        // the chunk's segment table, in this warp's slice of shared memory (seg)
         __syncwarp();
         if (lane < PUSH_CHUNK) {
             seg[lane].incl = incl;
@@ -398,13 +447,18 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
 // row order with warp shuffles, so the fp32 sum is formed in exactly the order
 // of the reference's loop over pSynapses.
 // ---------------------------------------------------------------------------
+// bitmap: [R][W] fired flags (global memory, or a copy of them in shared memory);
+// warp_lin of n_warps: this warp's number among those that deliver.
 template <int ACC>
-static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &a, unsigned long long t, int pw)
+static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &a, unsigned long long t, int pw,
+                                                                const uint32_t *bitmap, long long warp_lin,
+                                                                long long n_warps)
 {
     const int lane = threadIdx.x & 31;
-    const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int W = (int)a.W, R = a.R, cur = (int)(t % (unsigned long long)a.R);
+    const int d_max = (long long)t < a.D ? (int)t : a.D;  // cycles before the first fired nothing
     unsigned long long ev = 0;
-    for (long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < a.N; j += n_warps) {
+    for (long long j = warp_lin; j < a.N; j += n_warps) {
         const int64_t c0 = a.col_off[j], c1 = a.col_off[j + 1];
         const float sc = (ACC == BSIM_ACC_EXACT) ? __ldg(&a.ctab[a.cls[j]].scale_up) : 0.0f;
         long long sE = 0, sI = 0;
@@ -417,9 +471,9 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
                 const uint32_t s = __ldcs(a.csc_src + e);
                 const int d = (int)__ldcs(a.csc_d + e) + 1;
                 w = __ldcs(a.csc_w + e);
-                if ((long long)t - d >= 0) {
-                    const int slot = (int)((t - d) % (unsigned long long)a.R);
-                    act = (a.bitmap[(int64_t)slot * a.W + (s >> 5)] >> (s & 31)) & 1u;
+                if (d <= d_max) {
+                    const int slot = cur >= d ? cur - d : cur - d + R;
+                    act = (bitmap[(int64_t)slot * W + (s >> 5)] >> (s & 31)) & 1u;
                 }
             }
             unsigned m = __ballot_sync(0xffffffffu, act);
@@ -905,14 +959,27 @@ static __device__ __forceinline__ void record_phase(const StepArgs &a, unsigned 
     const long long k = ts - rc.t0;
     if (k < 0 || k >= rc.steps || rc.next != ts) return;
     const int slot = (int)(ts % a.R);
-    const int64_t n = a.ring_cnt[slot];
-    const int64_t base = a.rec_off[k];
+    const int64_t n = __ldcg(&a.ring_cnt[slot]);
+    const int64_t base = __ldcg(&a.rec_off[k]);
     int64_t room = rc.cap - base;
     if (room < 0) room = 0;
     const int64_t ncopy = n < room ? n : room;
     const int32_t *src = a.ring + (int64_t)slot * a.cap;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncopy; i += (int64_t)gridDim.x * blockDim.x)
-        a.rec_ids[base + i] = src[i];
+        a.rec_ids[base + i] = __ldcg(&src[i]);
+}
+
+// End of a cycle, by one thread of the last block: recording offsets.
+static __device__ __forceinline__ void record_advance(const StepArgs &a, unsigned long long t)
+{
+    if (!a.rec || t == 0) return;
+    volatile RecCtl *rc = a.rec;
+    const long long k = (long long)t - 1 - rc->t0;
+    if (k >= 0 && k < rc->steps && rc->next == (long long)t - 1) {
+        const int64_t n = __ldcg(&a.ring_cnt[(t - 1) % (unsigned long long)a.R]);
+        a.rec_off[k + 1] = __ldcg(&a.rec_off[k]) + n;
+        rc->next = (long long)t;
+    }
 }
 
 template <int ACC>
@@ -943,7 +1010,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     const bool push = ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_PUSH;
     const bool tiled = ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_TILE;
     if (threadIdx.x == 0) s_ev = 0;
-    if (push && threadIdx.x < 32) delay_window_prefix(a, t, s_cum);
+    if (push && threadIdx.x < 32) delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // slot t+1 is neither written (LIF writes slot t) nor read (delivery reads t-1..t-D) now
         a.ring_cnt[(t + 1) % (unsigned long long)a.R] = 0;
@@ -956,12 +1023,15 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     __syncthreads();  // publishes s_cum and s_ev
     unsigned long long ev;
     if (push) {
-        ev = push_phase(a, t, p ^ 1, s_cum, s_seg);
+        ev = push_phase(a, t, p ^ 1, s_cum, s_seg + (threadIdx.x >> 5) * PUSH_CHUNK,
+                        (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x,
+                        ((long long)gridDim.x * blockDim.x) >> 5);
     } else if (tiled) {
         ev = tile_phase(a, t, p ^ 1, reinterpret_cast<unsigned *>(s_dyn),
                         reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part);
     } else {
-        ev = pull_phase<ACC>(a, t, p ^ 1);
+        ev = pull_phase<ACC>(a, t, p ^ 1, a.bitmap, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                             ((long long)gridDim.x * blockDim.x) >> 5);
     }
     if (ev) atomicAdd(&s_ev, ev);
     lif_phase<ACC>(a, t, p, cur, s_wcnt);
@@ -989,21 +1059,552 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
                 a.part_pairs[(int64_t)((t + 1ull) & 1ull) * a.n_parts + i] = 0u;
         if (threadIdx.x == 0) {
             // advance the cycle
-            if (a.rec && t > 0) {
-                RecCtl *rc = a.rec;
-                const long long k = (long long)t - 1 - rc->t0;
-                if (k >= 0 && k < rc->steps && rc->next == (long long)t - 1) {
-                    const int64_t n = a.ring_cnt[(t - 1) % (unsigned long long)a.R];
-                    a.rec_off[k + 1] = a.rec_off[k] + n;
-                    rc->next = (long long)t;
-                }
-            }
+            record_advance(a, t);
             *a.ticket = 0u;
             *(a.ticket + 1) = 0u;  // the update's chunk counter
             if (a.part_ctr) *a.part_ctr = 0u;
             *a.step_ctr = t + 1;
             __threadfence();
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small networks: many cycles in one cooperative launch.
+//
+// A cycle of a network of a few thousand neurons moves little; one launch per cycle
+// spends its ~10 us on the launch and on a chain of dependent reads (error flag,
+// cycle counter, spike counts, ids, rows, entries, then the update's chunk counter,
+// state, class, ring position). In one launch the blocks meet at a grid barrier
+// instead (~4,000 clocks with the release of the sums, whatever the grid), so the
+// work is laid out to need few of them:
+//
+//   * Push: neurons have owners for the whole launch (state in registers), and a
+//     block delivers its own neurons' spikes at once, with all delays, into a ring
+//     of input accumulators, one per future cycle (acc_ring: cycle c in slot c mod
+//     acc_R). A spike of cycle t reaches no update before cycle t + 2, so two cycles
+//     are run between barriers: both updates, then the rows of both cycles' spikes.
+//     Owners take groups of eight consecutive neurons dealt out over all blocks, so
+//     that a population that fires together spreads over the GPU.
+//     10 x 1,000 neurons (100 Hz): 10.2 -> 3.3 us per cycle; 5,000 neurons behind
+//     Poisson drives 13.7 -> 3.9; 20 x 1,000 all-to-all 18.1 -> 6.2.
+//   * Pull (and the ORDERED sums): one cycle per barrier; the update's owners and
+//     the target rows run side by side, with the delay window's fired flags in
+//     shared memory. 10 x 1,000 neurons: 12.8 -> 10.0 us per cycle.
+//
+// The fire ring, its counts and the fired flags are kept as step_kernel keeps them,
+// so the two can follow one another (loop_enter_kernel, loop_leave_kernel). Data that
+// another block wrote during the launch is read past L1 (ld.cg).
+//
+// The barrier is the launch's only wait: every block adds itself to a counter, with an
+// error bit when the device error flag is set, and waits until all have. Two counters
+// alternate, so one that a block still reads is not added to for the next barrier, and
+// every block sees the same error bits and leaves after the same cycle. The wait is
+// bounded (BSIM_DEVERR_TIMEOUT). The launch is cooperative: its blocks are resident at
+// the same time.
+// ---------------------------------------------------------------------------
+// Threads per block. Push: the rows of a few spikes per block, so more warps only make the
+// block's own barriers longer (10 x 1,000 neurons, us per cycle: 256 threads 4.3, 512 4.3,
+// 1,024 5.1; 20 x 1,000 all-to-all with bursts 11.7, 7.2, 7.3). Pull: every synapse is scanned,
+// so all the warps that fit (18.6, 12.8, 10.0 on the same network).
+#define LOOP_THREADS 512
+#define PULL_LOOP_THREADS 1024
+#define LOOP_WARPS (LOOP_THREADS / 32)
+#define PULL_LOOP_WARPS (PULL_LOOP_THREADS / 32)
+#define LOOP_MAX_DELAY 64
+#define LOOP_CYCLES 2  // between barriers of the push form: the shortest delay (1 step) + 1
+#ifndef LOOP_WAIT_SPINS
+#define LOOP_WAIT_SPINS (1u << 22)  // seconds: a cycle takes microseconds
+#endif
+#define LOOP_MAX_SMEM ((size_t)160 * 1024)  // pull: bitmaps kept in shared memory
+#define LOOP_ERR (1ull << 40)  // one block's error in a barrier counter; arrivals are below
+
+static __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+static __device__ __forceinline__ void red_release(unsigned long long *p, unsigned long long v)
+{
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// The recording during a launch: every block follows the offsets (block 0 writes them).
+struct LoopRec {
+    long long t0, steps, cap;
+    int64_t off;  // spikes recorded so far
+    bool on;
+};
+static __device__ __forceinline__ LoopRec loop_record_begin(const StepArgs &a, unsigned long long t)
+{
+    LoopRec r{0, 0, 0, 0, false};
+    if (a.rec) {
+        const volatile RecCtl *rc = a.rec;
+        r.t0 = rc->t0;
+        r.steps = rc->steps;
+        r.cap = rc->cap;
+        const long long k = (long long)t - r.t0;
+        r.on = k >= 0 && k < r.steps && rc->next == (long long)t;
+        if (r.on) r.off = __ldcg(&a.rec_off[k]);
+    }
+    return r;
+}
+
+// Copies the spikes of cycles [t, t_end), complete, into the recording (slot: ring slot of t).
+static __device__ __forceinline__ void loop_record(const StepArgs &a, LoopRec &r, unsigned long long t,
+                                                   unsigned long long t_end, int slot)
+{
+    for (; r.on && t < t_end; t++) {
+        const long long k = (long long)t - r.t0;
+        if (k >= r.steps) {
+            r.on = false;
+            break;
+        }
+        const int64_t count = __ldcg(&a.ring_cnt[slot]);
+        const int64_t n = min(count, max((int64_t)0, (int64_t)r.cap - r.off));
+        const int32_t *src = a.ring + (int64_t)slot * a.cap;
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+            a.rec_ids[r.off + i] = __ldcg(&src[i]);
+        r.off += count;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.rec_off[k + 1] = r.off;
+            a.rec->next = (long long)t + 1;
+        }
+        if (++slot == a.R) slot = 0;
+    }
+}
+
+// Barrier number k of the launch. `base`: the counter's value when none of this barrier's blocks
+// had arrived (blocks leave a counter at a multiple of the grid). Returns whether the launch stops
+// here. The block's last warp (which owns no neurons) arrives and waits; meanwhile the others may
+// do `shadow`.
+struct LoopBar {
+    unsigned long long base[2];
+    int k;
+};
+static __device__ __forceinline__ LoopBar loop_bar_begin(const StepArgs &a)
+{
+    LoopBar b{{0, 0}, 0};
+    if (threadIdx.x == blockDim.x - 32)
+        for (int i = 0; i < 2; i++) {
+            const unsigned long long v = ld_acquire(a.loop_bar + 16 * i);  // this block has not arrived yet
+            b.base[i] = v - (v & (LOOP_ERR - 1)) % gridDim.x;
+        }
+    return b;
+}
+template <typename Shadow>
+static __device__ __forceinline__ bool loop_barrier(const StepArgs &a, LoopBar &b, const bool *s_err, bool *s_stop,
+                                                    Shadow shadow)
+{
+    __syncthreads();
+    if (threadIdx.x != blockDim.x - 32) {
+        shadow();
+    } else {
+        const int p = b.k & 1;
+        unsigned long long *ctr = a.loop_bar + 16 * p;
+        red_release(ctr, 1ull + (*s_err ? LOOP_ERR : 0ull));
+        const unsigned long long all = (b.base[p] & (LOOP_ERR - 1)) + gridDim.x;
+        unsigned long long w;
+        unsigned spins = 0;
+        bool stop = false;
+        while (((w = ld_acquire(ctr)) & (LOOP_ERR - 1)) != all) {
+            if (++spins > LOOP_WAIT_SPINS) {
+                raise_error(a, BSIM_DEVERR_TIMEOUT);
+                stop = true;
+                break;
+            }
+        }
+        *s_stop = stop || (w / LOOP_ERR) != (b.base[p] / LOOP_ERR);
+        b.base[p] = w;
+    }
+    b.k++;
+    __syncthreads();
+    return *s_stop;
+}
+
+// The counters of the n cycles from t on, t in ring slot `slot` (what they held is not read any more).
+static __device__ __forceinline__ void loop_clear_counts(const StepArgs &a, unsigned long long t, int slot, int n)
+{
+    const int lane = threadIdx.x & 31;
+    for (int c = 0; c < n; c++) {
+        if (lane == 0) a.ring_cnt[slot] = 0;
+        if (a.pop_hist) {
+            int32_t *nxt = a.pop_hist + (int64_t)((t + c) % (unsigned long long)a.hist_len) * a.n_pops;
+            for (int i = lane; i < a.n_pops; i += 32) nxt[i] = 0;
+        }
+        if (++slot == a.R) slot = 0;
+    }
+}
+
+// Reserves a warp's places in the fire ring of cycle t (mask: the lanes that fired), and, later,
+// fills them: the reservation's latency is not waited for in between.
+static __device__ __forceinline__ int loop_reserve(const StepArgs &a, int slot, unsigned mask)
+{
+    int at = 0;
+    if (mask && (threadIdx.x & 31) == 0) at = atomicAdd(&a.ring_cnt[slot], __popc(mask));
+    return at;
+}
+static __device__ __forceinline__ void loop_append(const StepArgs &a, unsigned long long t, int slot, unsigned mask, int at,
+                                                   int64_t j, int pop)
+{
+    if (!mask) return;
+    const int lane = threadIdx.x & 31;
+    const bool fired = (mask >> lane) & 1u;
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (fired) a.ring[(int64_t)slot * a.cap + at + __popc(mask & ((1u << lane) - 1u))] = (int32_t)j;
+    if (a.pop_hist) {
+        // one atomic per (warp, population) with spikes
+        int32_t *hist = a.pop_hist + (int64_t)(t % (unsigned long long)a.hist_len) * a.n_pops;
+        const unsigned same = __match_any_sync(0xffffffffu, fired ? pop : -1);
+        if (fired && lane == __ffs(same) - 1) atomicAdd(&hist[pop], __popc(same));
+    }
+}
+
+static __device__ __forceinline__ const float *drive_vtmp(const StepArgs &a, unsigned long long t)
+{
+    return (a.drive_half > 0 && ((t / (unsigned long long)a.drive_half) & 1ull)) ? a.vtmp_alt : a.vtmp;
+}
+
+struct LoopSpike {
+    int who, cycle;  // owner thread's number in the block, cycle within the interval
+    float scale;     // 2^qexp of the source's network
+};
+
+// Dynamic shared memory of the push form: each owner thread's row start and its D + 1 delay
+// segments' starts within the row.
+static __host__ __device__ __forceinline__ size_t push_loop_smem(int64_t N, int D, int grid)
+{
+    const int64_t octets = (N + 7) / 8, owner_warps = (octets + 4 * (int64_t)grid - 1) / (4 * (int64_t)grid);
+    return (size_t)owner_warps * 32 * (sizeof(int64_t) + sizeof(unsigned) * (size_t)(D + 1));
+}
+
+__global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid_constant__ StepArgs a, int steps)
+{
+    __shared__ LoopSpike s_spike[LOOP_CYCLES * LOOP_THREADS / 2];  // at most half the warps own neurons
+    __shared__ unsigned long long s_ev[LOOP_MAX_DELAY + 3];        // events by the cycle that delivers them
+    __shared__ int s_n;
+    __shared__ bool s_stop, s_err;
+    extern __shared__ __align__(16) unsigned long long s_dyn[];  // rows (push_loop_smem)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int D = a.D, Ra = a.acc_R;
+    if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
+    unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
+    // owners: four groups of eight neurons per warp, dealt out over all owning warps
+    const int64_t octets = (a.N + 7) / 8;
+    const int owner_warps = (int)((octets + 4 * (int64_t)gridDim.x - 1) / (4 * (int64_t)gridDim.x));
+    const bool owner = warp < owner_warps;
+    const int64_t octet = (int64_t)(lane >> 3) * owner_warps * gridDim.x + (int64_t)warp * gridDim.x + blockIdx.x;
+    const int64_t j = octet * 8 + (lane & 7);
+    const bool mine = owner && j < a.N;
+    longlong2 *acc = reinterpret_cast<longlong2 *>(a.acc_ring);
+    const ClassParams *c = a.ctab;
+    float4 st = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float scale_down = 0.0f, scale_up = 0.0f, vt = 0.0f, vt_alt = 0.0f;
+    int pop = -1, fires = 0, kind = BSIM_NEURON_LIF;
+    // The barrier's acquire empties L1, so what a cycle needs of the class, the drive and the
+    // rows' bounds is kept in registers and shared memory.
+    LifConst lif{};
+    int64_t *s_row0 = reinterpret_cast<int64_t *>(s_dyn);
+    unsigned *s_seg0 = reinterpret_cast<unsigned *>(s_row0 + owner_warps * 32);
+    if (mine) {
+        c += a.cls[j];
+        st = a.state[j];
+        scale_down = __ldg(&c->scale_down);
+        scale_up = __ldg(&c->scale_up);
+        pop = __ldg(&c->pop);
+        kind = __ldg(&c->kind);
+        lif = lif_const(c);
+        vt = a.vtmp[j];
+        if (a.drive_half > 0) vt_alt = a.vtmp_alt[j];
+        const int64_t *row = a.row_off + j * D;
+        const int64_t r0 = __ldg(row);
+        s_row0[threadIdx.x] = r0;
+        for (int d = 0; d <= D; d++) s_seg0[threadIdx.x * (D + 1) + d] = (unsigned)(__ldg(row + d) - r0);
+    }
+    int gap = -1;  // a Poisson neuron's gap after its next spike, drawn ahead while the barrier waits
+    if (threadIdx.x == 0) {
+        s_n = 0;
+        s_err = false;
+    }
+    if (threadIdx.x < Ra) {  // spikes in flight when the launch starts: counted by block 0
+        s_ev[threadIdx.x] = blockIdx.x == 0 ? a.loop_ev[threadIdx.x] : 0ull;
+        if (blockIdx.x == 0) a.loop_ev[threadIdx.x] = 0ull;
+    }
+    __syncthreads();
+    unsigned long long ev = 0;  // thread 0: events delivered
+    int slot = (int)(t % (unsigned long long)Ra);         // accumulator slot of cycle t
+    int rslot = (int)(t % (unsigned long long)a.R);       // ring slot of cycle t
+    LoopBar bar = loop_bar_begin(a);
+    LoopRec rec = loop_record_begin(a, t);
+    bool stop = false;
+    for (int k = 0; k < steps && !stop;) {
+        const int m = min(LOOP_CYCLES, steps - k);
+        const int rslot1 = rslot + 1 < a.R ? rslot + 1 : 0;  // of cycle t + 1
+        unsigned mask[LOOP_CYCLES];
+        int place[LOOP_CYCLES];
+        // ---- the updates of cycles t .. t+m-1: their inputs are complete
+        if (owner) {
+            longlong2 in[LOOP_CYCLES];
+#pragma unroll
+            for (int i = 0; i < LOOP_CYCLES; i++) {
+                in[i] = make_longlong2(0, 0);
+                if (mine && i < m) {
+                    longlong2 *q = acc + (int64_t)(slot + i < Ra ? slot + i : slot + i - Ra) * a.N + j;
+                    in[i] = __ldcg(q);
+                    __stcg(q, make_longlong2(0, 0));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < LOOP_CYCLES; i++) {
+                bool fired = false;
+                if (mine && i < m) {
+                    const float inE = __fmul_rn(__ll2float_rn(in[i].x), scale_down);
+                    const float inI = __fmul_rn(__ll2float_rn(in[i].y), scale_down);
+                    if (kind == BSIM_NEURON_LIF) {
+                        const bool alt = a.drive_half > 0 && (((t + i) / (unsigned long long)a.drive_half) & 1ull);
+                        lif_update(lif, alt ? vt_alt : vt, inE, inI, st, fired);
+                    } else {
+                        drive_update(kind, (int)(t + i), st, fired, [&](int fc) {
+                            const int g = gap >= 0 ? gap : poisson_gap(a, c, j, st, fc);
+                            gap = -1;
+                            return g;
+                        });
+                    }
+                    if (a.trace) trace_neuron(a, trace_row(a, t + i), j, st, inE, inI);
+                }
+                mask[i] = __ballot_sync(0xffffffffu, fired);
+                if (mask[i]) {
+                    int at = 0;
+                    if (lane == 0) at = atomicAdd(&s_n, __popc(mask[i]));
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (fired) {
+                        s_spike[at + __popc(mask[i] & ((1u << lane) - 1u))] = LoopSpike{(int)threadIdx.x, i, scale_up};
+                        fires++;
+                    }
+                }
+                place[i] = i < m ? loop_reserve(a, i == 0 ? rslot : rslot1, mask[i]) : 0;
+            }
+        }
+        __syncthreads();
+        // ---- the rows of this block's spikes, all delays: a spike of cycle t+i with delay d is
+        // input of cycle t+i+d+1. With fewer spikes than warps each row is cut into pieces.
+        const int n = s_n;
+        const int split = n > 0 && 2 * n <= LOOP_WARPS ? LOOP_WARPS / n : 1;
+        for (int it = warp; it < n * split; it += LOOP_WARPS) {
+            const LoopSpike sp = s_spike[it / split];
+            const unsigned *off = s_seg0 + sp.who * (D + 1);
+            const int64_t r0 = s_row0[sp.who];
+            int64_t lo = r0, hi = r0 + off[D];
+            if (split > 1) {  // inner cuts lie on 16-byte boundaries
+                const int64_t len = hi - lo, b = lo;
+                const int piece = it % split;
+                const int64_t cut0 = (b + len * piece / split + 1) & ~1ll, cut1 = (b + len * (piece + 1) / split + 1) & ~1ll;
+                if (piece > 0) lo = min(cut0, hi);
+                if (piece + 1 < split) hi = min(cut1, hi);
+            }
+            int slot0 = slot + sp.cycle + 2;  // of delay 1
+            if (slot0 >= Ra) slot0 -= Ra;
+            auto add = [&](int64_t e, uint32_t tgt, uint32_t wbits) {
+                if ((int64_t)tgt >= a.N) {  // a target outside the network: flag it, touch nothing
+                    raise_error(a, BSIM_DEVERR_TARGET);
+                    s_err = true;
+                    return;
+                }
+                const unsigned x = (unsigned)(e - r0);
+                int d = 0, top = D - 1;  // delay - 1: the segment that holds entry x
+                while (d < top) {
+                    const int mid = (d + top + 1) >> 1;
+                    if (off[mid] <= x) d = mid;
+                    else top = mid - 1;
+                }
+                int sl = slot0 + d;
+                if (sl >= Ra) sl -= Ra;
+                const float w = __uint_as_float(wbits);
+                const long long q = __float2ll_rn(__fmul_rn(w, sp.scale));
+                red_add_u64(reinterpret_cast<unsigned long long *>(acc + (int64_t)sl * a.N + tgt) + (w >= 0.0f ? 0 : 1),
+                            (unsigned long long)q);
+            };
+            if (it % split == 0)  // delivered in cycle t+i+d: counted when that cycle has run
+                for (int d = lane; d < D; d += 32) {
+                    int sl = slot + sp.cycle + 1 + d;
+                    if (sl >= Ra) sl -= Ra;
+                    if (off[d + 1] != off[d]) atomicAdd(&s_ev[sl], (unsigned long long)(off[d + 1] - off[d]));
+                }
+            // pairs of entries from even positions; the rows are read again within cycles, so they
+            // stay in L2 (the array has room for the pair that holds its last entry)
+            for (int64_t e0 = (lo & ~1ll) + 2 * lane; e0 < hi; e0 += 4 * 64) {
+                uint4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (e0 + u * 64 < hi) v[u] = __ldg(reinterpret_cast<const uint4 *>(a.syn + e0 + u * 64));
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int64_t e = e0 + u * 64;
+                    if (e < hi && e >= lo) add(e, v[u].x, v[u].y);
+                    if (e + 1 < hi) add(e + 1, v[u].z, v[u].w);
+                }
+            }
+        }
+        // ---- history: fired flags and the fire ring (not read by this launch's delivery)
+        if (owner) {
+            for (int i = 0; i < m; i++) {
+                const unsigned mk = i == 0 ? mask[0] : mask[1];
+                const int rs = i == 0 ? rslot : rslot1;
+                if ((lane & 7) == 0 && octet < octets)
+                    reinterpret_cast<uint8_t *>(a.bitmap + (int64_t)rs * a.W)[octet] = (uint8_t)(mk >> lane);
+                loop_append(a, t + i, rs, mk, i == 0 ? place[0] : place[1], j, pop);
+            }
+        }
+        if (blockIdx.x == 0 && warp == LOOP_WARPS - 1) loop_clear_counts(a, t + m, (rslot + m) % a.R, LOOP_CYCLES);
+        stop = loop_barrier(a, bar, &s_err, &s_stop, [&] {
+            if (kind == BSIM_NEURON_POISSON && gap < 0) gap = poisson_gap(a, c, j, st, __float_as_int(st.y));
+        });
+        if (threadIdx.x == 0) {
+            s_n = 0;
+            for (int i = 0; i < m; i++) {
+                const int sl = slot + i < Ra ? slot + i : slot + i - Ra;
+                ev += s_ev[sl];
+                s_ev[sl] = 0ull;
+            }
+        }
+        if (rec.on) loop_record(a, rec, t, t + m, rslot);
+        t += m;
+        k += m;
+        slot = (slot + m) % Ra;
+        rslot = (rslot + m) % a.R;
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.step_ctr = t;
+    if (threadIdx.x < Ra && s_ev[threadIdx.x]) atomicAdd(&a.loop_ev[threadIdx.x], s_ev[threadIdx.x]);  // still in flight
+    if (mine) {
+        a.state[j] = st;
+        if (fires) a.fire_count[j] += fires;
+    }
+    if (ev) atomicAdd(a.events, ev);
+}
+
+template <int ACC>
+__global__ void __launch_bounds__(PULL_LOOP_THREADS, 1) pull_loop_kernel(const __grid_constant__ StepArgs a, int steps)
+{
+    __shared__ bool s_stop, s_err;
+    extern __shared__ __align__(16) unsigned long long s_dyn[];  // [R][W] the fired flags
+    uint32_t *s_bm = reinterpret_cast<uint32_t *>(s_dyn);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
+    unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
+    // owners: warp w of block b owns word w * grid + b of the fired flags, if there is one
+    const int64_t word = (int64_t)warp * gridDim.x + blockIdx.x;
+    const bool owner = word < a.W;
+    const int64_t j = word * 32 + lane;
+    const bool mine = owner && j < a.N;
+    const ClassParams *c = a.ctab;
+    float4 st = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float scale_down = 0.0f;
+    int pop = -1, fires = 0;
+    if (mine) {
+        c += a.cls[j];
+        st = a.state[j];
+        scale_down = __ldg(&c->scale_down);
+        pop = __ldg(&c->pop);
+    }
+    if (threadIdx.x == 0) s_err = false;
+    for (int64_t i = threadIdx.x; i < (int64_t)a.R * a.W; i += PULL_LOOP_THREADS) s_bm[i] = a.bitmap[i];
+    unsigned long long ev = 0;
+    LoopBar bar = loop_bar_begin(a);
+    LoopRec rec = loop_record_begin(a, t);
+    bool stop = false;
+    for (int k = 0; k < steps && !stop; k++) {
+        const int p = (int)(t & 1ull);
+        const int cur = (int)(t % (unsigned long long)a.R);
+        if (blockIdx.x == 0 && warp == PULL_LOOP_WARPS - 1) loop_clear_counts(a, t + 1, cur + 1 < a.R ? cur + 1 : 0, 1);
+        if (owner) {
+            bool fired = false;
+            if (mine) {
+                float inE, inI;
+                if (ACC == BSIM_ACC_EXACT) {
+                    longlong2 *q = reinterpret_cast<longlong2 *>(a.acc) + (int64_t)p * a.N + j;
+                    const longlong2 in = __ldcg(q);
+                    if (a.acc_clear) __stcg(q, make_longlong2(0, 0));  // as step_kernel leaves it
+                    inE = __fmul_rn(__ll2float_rn(in.x), scale_down);
+                    inI = __fmul_rn(__ll2float_rn(in.y), scale_down);
+                } else {
+                    const float2 in = __ldcg(reinterpret_cast<const float2 *>(a.acc) + (int64_t)p * a.N + j);
+                    inE = in.x;
+                    inI = in.y;
+                }
+                neuron_update(a, c, j, (int)t, drive_vtmp(a, t), inE, inI, st, fired);
+                if (a.trace) trace_neuron(a, trace_row(a, t), j, st, inE, inI);
+                fires += fired;
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, fired);
+            if (lane == 0) a.bitmap[(int64_t)cur * a.W + word] = mask;
+            loop_append(a, t, cur, mask, loop_reserve(a, cur, mask), j, pop);
+        }
+        if (k > 0) {  // the previous cycle's fired flags
+            const int prev = cur > 0 ? cur - 1 : a.R - 1;
+            for (int64_t i = threadIdx.x; i < a.W; i += PULL_LOOP_THREADS)
+                s_bm[(int64_t)prev * a.W + i] = __ldcg(&a.bitmap[(int64_t)prev * a.W + i]);
+        }
+        __syncthreads();
+        ev += pull_phase<ACC>(a, t, p ^ 1, s_bm, (long long)warp * gridDim.x + blockIdx.x,
+                              (long long)PULL_LOOP_WARPS * gridDim.x);
+        stop = loop_barrier(a, bar, &s_err, &s_stop, [] {});
+        if (rec.on) loop_record(a, rec, t, t + 1, cur);
+        t++;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.step_ctr = t;
+    if (mine) {
+        a.state[j] = st;
+        if (fires) a.fire_count[j] += fires;
+    }
+    if (ev) atomicAdd(a.events, ev);
+}
+
+// From step_kernel's input accumulators to the ring of push_loop_kernel: the input of the next
+// cycle, and the spikes in flight (a spike of cycle s with delay d >= t - s is still to be delivered).
+__global__ void loop_enter_kernel(const __grid_constant__ StepArgs a)
+{
+    if (*reinterpret_cast<volatile int32_t *>(a.err) != 0) return;
+    const unsigned long long t = *a.step_ctr;
+    const int D = a.D;
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc_ring);
+    const longlong2 *now = reinterpret_cast<const longlong2 *>(a.acc) + (int64_t)(t & 1ull) * a.N;
+    // (the ring was zeroed before this launch; slots of later cycles are added to below)
+    if (blockIdx.x == 0 && threadIdx.x < 32) loop_clear_counts(a, t + 1, (int)((t + 1) % (unsigned long long)a.R), 1);  // step_kernel cleared t's
+    longlong2 *first = reinterpret_cast<longlong2 *>(a.acc_ring) + (int64_t)(t % (unsigned long long)a.acc_R) * a.N;
+    for (int64_t i = tid; i < a.N; i += nt) first[i] = now[i];
+    const int lane = threadIdx.x & 31;
+    for (int age = 1; age <= D && (long long)t - age >= 0; age++) {
+        const unsigned long long s = t - age;
+        const int slot = (int)(s % (unsigned long long)a.R);
+        const int n = a.ring_cnt[slot];
+        for (int64_t i = tid >> 5; i < n; i += nt >> 5) {
+            const int id = a.ring[(int64_t)slot * a.cap + i];
+            const float sc = a.ctab[a.cls[id]].scale_up;
+            for (int d = age; d <= D; d++) {
+                unsigned long long *q = acc + 2 * (int64_t)((s + d + 1) % (unsigned long long)a.acc_R) * a.N;
+                const int64_t r0 = a.row_off[(int64_t)id * D + d - 1], r1 = a.row_off[(int64_t)id * D + d];
+                if (lane == 0 && r1 > r0)
+                    atomicAdd(&a.loop_ev[(s + d) % (unsigned long long)a.acc_R], (unsigned long long)(r1 - r0));
+                for (int64_t e = r0 + lane; e < r1; e += 32)
+                    push_one(a, q, a.syn[e].x, a.syn[e].y, sc);
+            }
+        }
+    }
+}
+
+// And back: the next cycle's input; the other parity is delivered into next.
+__global__ void loop_leave_kernel(const __grid_constant__ StepArgs a)
+{
+    const unsigned long long t = *a.step_ctr;
+    if (blockIdx.x == 0 && threadIdx.x < a.acc_R) a.loop_ev[threadIdx.x] = 0ull;  // step_kernel counts them
+    longlong2 *acc = reinterpret_cast<longlong2 *>(a.acc);
+    const longlong2 *now = reinterpret_cast<const longlong2 *>(a.acc_ring) + (int64_t)(t % (unsigned long long)a.acc_R) * a.N;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.N; i += (int64_t)gridDim.x * blockDim.x) {
+        acc[(int64_t)(t & 1ull) * a.N + i] = now[i];
+        acc[(int64_t)((t & 1ull) ^ 1ull) * a.N + i] = make_longlong2(0, 0);
     }
 }
 
@@ -1075,6 +1676,54 @@ cudaError_t launch_step(Engine &e)
 cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream_t stream)
 {
     step_kernel<BSIM_ACC_EXACT><<<grid, block, step_dynamic_smem(a, block), stream>>>(a);
+    return cudaGetLastError();
+}
+
+// Whether an engine of these sizes can run many cycles per launch (0: no, 1: push form, 2: pull
+// form): half of a block's warps own neurons at most. Tiled and AUTO delivery and longer delays
+// take one launch per cycle.
+int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
+{
+    const int64_t W = (N + 31) / 32;
+    if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
+    if (o.accumulate != BSIM_ACC_ORDERED && o.delivery == BSIM_DELIVERY_PUSH)
+        return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
+    const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + 2) * W;
+    return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps <= LOOP_MAX_SMEM ? 2 : 0;
+}
+
+cudaError_t launch_loop(Engine &e, int steps)
+{
+    void *args[] = {&e.a, &steps};
+    if (e.loop == 1)
+    {
+        const cudaError_t st = cudaFuncSetAttribute((const void *)push_loop_kernel,
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOOP_MAX_SMEM);
+        if (st != cudaSuccess) return st;
+        return cudaLaunchCooperativeKernel((const void *)push_loop_kernel, dim3(e.sm_count), dim3(LOOP_THREADS), args,
+                                           push_loop_smem(e.N, e.D, e.sm_count), e.stream);
+    }
+    const void *f = e.opt.accumulate == BSIM_ACC_ORDERED ? (const void *)pull_loop_kernel<BSIM_ACC_ORDERED>
+                                                         : (const void *)pull_loop_kernel<BSIM_ACC_EXACT>;
+    const cudaError_t st = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOOP_MAX_SMEM);
+    if (st != cudaSuccess) return st;
+    return cudaLaunchCooperativeKernel(f, dim3(e.sm_count), dim3(PULL_LOOP_THREADS), args,
+                                       sizeof(uint32_t) * (size_t)e.a.R * e.a.W, e.stream);
+}
+
+cudaError_t launch_loop_enter(Engine &e)
+{
+    cudaError_t st = cudaMemsetAsync(e.a.acc_ring, 0, sizeof(longlong2) * (size_t)e.a.acc_R * e.N, e.stream);
+    if (st == cudaSuccess)
+        st = cudaMemsetAsync(e.a.loop_ev, 0, sizeof(unsigned long long) * e.a.acc_R, e.stream);
+    if (st != cudaSuccess) return st;
+    loop_enter_kernel<<<e.sm_count, 512, 0, e.stream>>>(e.a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_loop_leave(Engine &e)
+{
+    loop_leave_kernel<<<e.sm_count, 512, 0, e.stream>>>(e.a);
     return cudaGetLastError();
 }
 
