@@ -439,17 +439,6 @@ static int create_from_arrays(const float *params, const uint8_t *kind, int64_t 
     return BSIM_OK;
 }
 
-#ifndef MAX_PLANES
-#define MAX_PLANES 8  // parts per tile at most
-#endif
-#ifndef TILE_PARTS_PER_SM
-#define TILE_PARTS_PER_SM 3.4  // parts over all tiles per SM, about two per resident block (measured:
-                               // 2 parts per tile on 300 tiles and 3 on 148 tiles beat 1 / 4 and 4)
-#endif
-#ifndef MIN_PLANES
-#define MIN_PLANES 1  // parts per tile at least (blocks that run out of parts help the others)
-#endif
-
 // Ring, bitmaps, accumulators, counters; launch shape. Shared by both builders.
 static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
 {
@@ -466,60 +455,8 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     TRY(dalloc(e, &d_ctab, ctab.size()));
     CK(cudaMemcpy(d_ctab, ctab.data(), sizeof(ClassParams) * ctab.size(), cudaMemcpyHostToDevice));
     a.ctab = d_ctab;
-    // tiled delivery: each tile's work units in P parts (TILE_PARTS_PER_SM parts per SM
-    // over all tiles, MIN_PLANES..MAX_PLANES per tile); all parts of a tile (and the
-    // blocks helping them) sum into one accumulator plane: the first to finish stores
-    // its sums, the others add theirs once that store is done. One plane per parity for
-    // every delivery mode (the step kernel keeps the plane count a runtime value: with
-    // the count folded away its code generation measured 1-15 % slower)
-    a.n_planes = 1;
-    a.n_parts = 0;
-    a.parts = nullptr;
-    a.part_next = nullptr;
-    a.part_pairs = nullptr;
-    a.tile_arrive = nullptr;
-    if (a.n_tiles > 0) {
-        const int nt = a.n_tiles;
-        const double want = (double)TILE_PARTS_PER_SM * e.sm_count / nt;
-        const int P = (int)std::max((double)MIN_PLANES, std::min((double)MAX_PLANES, std::floor(want + 0.5)));
-        unsigned int *d_arrive;
-        TRY(dalloc(e, &d_arrive, 2 * (size_t)nt));  // [2][n_tiles]: finishers so far, first store done
-        CK(cudaMemset(d_arrive, 0, sizeof(unsigned int) * 2 * nt));
-        a.tile_arrive = d_arrive;
-        std::vector<int4> parts;
-        for (int q = 0; q < nt; q++) {
-            const int U = q < (int)e.tile_units.size() ? e.tile_units[q] : 0;
-            for (int k = 0; k < P; k++)
-                parts.push_back(make_int4(q, (int)((int64_t)U * k / P), (int)((int64_t)U * (k + 1) / P), k));
-        }
-        // largest expected work first, so the queue ends with small parts
-        std::stable_sort(parts.begin(), parts.end(), [&](const int4 &x, const int4 &y) {
-            const int64_t ex = x.x < (int)e.tile_entries.size() ? e.tile_entries[x.x] : 0;
-            const int64_t ey = y.x < (int)e.tile_entries.size() ? e.tile_entries[y.x] : 0;
-            return ex > ey;
-        });
-        int4 *d_parts;
-        unsigned int *d_next;
-        std::vector<unsigned int> next(parts.size());
-        for (size_t i = 0; i < parts.size(); i++) next[i] = (unsigned)parts[i].y;
-        TRY(dalloc(e, &d_parts, parts.size()));
-        TRY(dalloc(e, &d_next, parts.size()));
-        CK(cudaMemcpy(d_parts, parts.data(), sizeof(int4) * parts.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(d_next, next.data(), sizeof(unsigned int) * parts.size(), cudaMemcpyHostToDevice));
-        unsigned int *d_help;
-        TRY(dalloc(e, &d_help, parts.size()));
-        CK(cudaMemset(d_help, 0, sizeof(unsigned int) * parts.size()));
-        a.part_help = d_help;
-        unsigned int *d_pairs;
-        TRY(dalloc(e, &d_pairs, 2 * parts.size()));
-        CK(cudaMemset(d_pairs, 0, sizeof(unsigned int) * 2 * parts.size()));
-        a.part_pairs = d_pairs;
-        a.parts = d_parts;
-        a.part_next = d_next;
-        a.n_parts = (int32_t)parts.size();
-    }
     const size_t acc_elem = e.opt.accumulate == BSIM_ACC_ORDERED ? sizeof(float2) : sizeof(longlong2);
-    const size_t acc_count = 2 * (size_t)a.n_planes * (size_t)e.N;
+    const size_t acc_count = 2 * (size_t)e.N;
     char *d_acc;
     TRY(dalloc(e, &d_acc, acc_elem * acc_count));
     CK(cudaMemset(d_acc, 0, acc_elem * acc_count));
@@ -546,7 +483,6 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     a.step_ctr = d_ctr;
     a.events = d_ctr + 1;
     a.ticket = reinterpret_cast<unsigned int *>(d_ctr + 2);
-    a.part_ctr = reinterpret_cast<unsigned int *>(d_ctr + 3);
     a.loop_bar = d_ctr + 16;
     if (e.loop == 1) {
         a.acc_R = e.D + 3;
@@ -591,6 +527,20 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     }
     if (bps < 1) return fail(BSIM_ERR_LIMIT, "step kernel does not fit on an SM with this tile size");
     e.grid = e.opt.grid_blocks > 0 ? e.opt.grid_blocks : e.sm_count * bps;
+    if (a.n_tiles > 0) {
+        // parts are numbered block + tile, for any grid the engine may take (the autotuner's too)
+        const size_t cap = (size_t)std::max(e.grid, e.sm_count * 64) + a.n_tiles;
+        TRY(dalloc(e, &a.part_word, cap));
+        TRY(dalloc(e, &a.part_tile, cap));
+        TRY(dalloc(e, &a.part_help, cap));
+        TRY(dalloc(e, &a.tile_pairs, 2 * (size_t)a.n_tiles));
+        TRY(dalloc(e, &a.tile_arrive, 2 * (size_t)a.n_tiles));  // finishers so far, first store done
+        CK(cudaMemset(a.part_word, 0, sizeof(unsigned long long) * cap));
+        CK(cudaMemset(a.part_tile, 0, sizeof(int) * cap));
+        CK(cudaMemset(a.part_help, 0, sizeof(unsigned) * cap));
+        CK(cudaMemset(a.tile_pairs, 0, sizeof(unsigned) * 2 * a.n_tiles));
+        CK(cudaMemset(a.tile_arrive, 0, sizeof(unsigned) * 2 * a.n_tiles));
+    }
     CK(cudaDeviceSynchronize());
     return BSIM_OK;
 }
@@ -617,21 +567,18 @@ static int plan_tiles(const std::vector<int64_t> &run_beg, int64_t tile, std::ve
 }
 
 // 16 bytes of shared counters per target (two words per E and I sum): tiles of
-// <= 5000 targets let two 512-thread blocks share an SM. Every tile scans the
-// fire bitmaps of its sources for each delay (a cost of tiles x D), while a
-// source's segment into a tile shrinks with the tile; blocks that run out of
-// parts help the others, so a few hundred tiles balance the GPU. Measured on the
-// generator's networks at their steady rates: ~300 tiles of ~3,300 targets best for
-// 1e6 neurons at D = 6 (7 % faster than 400 of 2,500), 5,000 targets for 2e6
-// neurons, ~1,700 targets at D = 6 for smaller ones, >= 5,000 at D = 50: so the
-// larger of N / (2 x SMs) and 1,700 x sqrt(D / 6), and small networks are cut
-// into at least SMs / 2 tiles (the parts split them further).
+// <= 5000 targets let two 512-thread blocks share an SM. A source's segment into a
+// tile shrinks with the tile, and every tile scans its sources' fire bitmaps for each
+// delay, so tiles are large where segments are short (long delays) and where there are
+// enough of them; a small network is cut finer, since each block flushes a whole tile
+// for its share. Measured on the generator's networks (us per cycle; 2,500 / 5,000
+// targets): 1e6 neurons, 6-step delays 188 / 164; 500,000, 20 steps 118 / 102; 250,000,
+// 50 steps 163 / 128; 250,000, 6 steps 84 / 94 (2,000: 82).
 static int64_t auto_tile_size(const bsim_options &o, int64_t N, int sm_count, int32_t D)
 {
     if (o.tile_size > 0) return std::min<int64_t>(o.tile_size, 12288);
-    int64_t t = std::max<int64_t>((int64_t)std::ceil((double)N / (2.0 * sm_count)),
-                                  (int64_t)(1700.0 * std::sqrt((double)D / 6.0)));
-    t = std::min<int64_t>(t, (2 * N + sm_count - 1) / sm_count);
+    int64_t t = std::max<int64_t>(N / 100, (int64_t)(2000.0 * std::sqrt((double)D / 6.0)));
+    t = std::min<int64_t>(t, (3 * N + sm_count - 1) / sm_count);
     return std::max<int64_t>(256, std::min<int64_t>(5000, t));
 }
 
@@ -692,9 +639,44 @@ static int upload_tiles(Engine &e, const TileHost &th)
         CK(cudaMemcpy(d_rp, th.run_seg0.data(), 8 * nr, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(d_ru, th.run_unit0.data(), 4 * nr, cudaMemcpyHostToDevice));
     }
+    // cost items: runs of a tile, cut into ranges of delays where they are large and merged where
+    // they are small, about eight per resident block
+    int64_t all_units = 0;
+    for (int32_t q = 0; q < nt; q++) all_units += th.tile_units[q];
+    const int32_t target = (int32_t)std::max<int64_t>(64, all_units / (16 * (int64_t)e.sm_count));
+    std::vector<int4> items;
+    std::vector<int2> run_item(std::max<size_t>(nr, 1));
+    for (int32_t q = 0; q < nt; q++) {
+        const int32_t first = (int32_t)items.size();
+        for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++) {
+            const int32_t u0 = th.run_unit0[r], chunks = (th.run_n[r] + 31) / 32;
+            const int32_t u1 = r + 1 < th.tile_run_off[q + 1] ? th.run_unit0[r + 1] : th.tile_units[q];
+            const int32_t D_r = (u1 - u0) / chunks, k = std::max(1, std::min(D_r, (u1 - u0) / target));
+            const int32_t per = (D_r + k - 1) / k;  // delays per item
+            if (k == 1 && (int32_t)items.size() > first && items.back().z < target) {
+                items.back().z += u1 - u0;
+                run_item[r] = make_int2((int32_t)items.size() - 1, D_r);
+                continue;
+            }
+            run_item[r] = make_int2((int32_t)items.size(), per);
+            for (int32_t d = 0; d < D_r; d += per)
+                items.push_back(make_int4(q, u0 + d * chunks, (std::min(d + per, D_r) - d) * chunks, 0));
+        }
+        if ((int32_t)items.size() == first) items.push_back(make_int4(q, 0, 1, 0));  // a tile without sources
+        items[first].w = th.tile_beg[q + 1] - th.tile_beg[q];
+    }
+    int4 *d_items;
+    int2 *d_ri;
+    TRY(dalloc(e, &d_items, items.size()));
+    TRY(dalloc(e, &d_ri, run_item.size()));
+    TRY(dalloc(e, &a.item_clocks, 2 * items.size()));
+    CK(cudaMemcpy(d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_ri, run_item.data(), sizeof(int2) * run_item.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemset(a.item_clocks, 0, sizeof(unsigned) * 2 * items.size()));
+    a.n_items = (int32_t)items.size();
+    a.items = d_items;
+    a.run_item = d_ri;
     a.n_tiles = nt;
-    a.n_tiles_u = th.n_u;
-    e.tile_units = th.tile_units;
     a.tile_max = th.tile_max;
     a.tile_beg = d_tb;
     a.tile_scale = d_ts;
@@ -959,7 +941,6 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
         }
     if (pair_overflow) return fail(BSIM_ERR_LIMIT, "tiled delivery: a source has more than 65535 synapses into one tile");
     std::vector<int64_t> tile_seg0(nt, 0);
-    e.tile_entries.assign(nt, 0);
     int64_t at = 0;
     for (int32_t q = 0; q < nt; q++) {
         tile_seg0[q] = at;
@@ -968,7 +949,6 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
             seg_off[i] = (uint32_t)(at - tile_seg0[q]);
             at += pairs;
         }
-        e.tile_entries[q] = 2 * (at - tile_seg0[q]);
         if (at - tile_seg0[q] > (int64_t)UINT32_MAX)
             return fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries");
         for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++) runs_d[r].base = tile_seg0[q];
@@ -1506,14 +1486,12 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         }
         std::vector<int64_t> tile_seg0(nt, 0);
         int64_t ent_pairs = 0;
-        E.tile_entries.resize(nt);
         for (int32_t q = 0; q < nt; q++) {
             if (total[q] > (unsigned long long)UINT32_MAX) {
                 free_tmp();
                 return bail(fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries"));
             }
             tile_seg0[q] = ent_pairs;
-            E.tile_entries[q] = 2 * (int64_t)total[q];
             ent_pairs += (int64_t)total[q];
             for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++)
                 segs[r].base = runs_d[r].base = tile_seg0[q];
@@ -2292,7 +2270,7 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
         // input consumed by the last cycle; zero it (the other parity is unread input).
         unsigned long long t_next = 0;
         CK(cudaMemcpy(&t_next, e.a.step_ctr, sizeof(t_next), cudaMemcpyDeviceToHost));
-        const size_t plane_set = (size_t)e.a.n_planes * (size_t)e.N;
+        const size_t plane_set = (size_t)e.N;
         CK(cudaMemset(reinterpret_cast<longlong2 *>(e.a.acc) + ((t_next & 1ull) ^ 1ull) * plane_set, 0,
                       sizeof(longlong2) * plane_set));
         e.a.acc_clear = 1;

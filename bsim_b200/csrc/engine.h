@@ -74,10 +74,8 @@ struct StepArgs {
     uint64_t input_seed;    // seed of the Poisson neurons' draws
     const uint16_t *cls;       // [N] class of each neuron
     const ClassParams *ctab;   // [n_cls]
-    void *acc;                 // [2][n_planes][N] longlong2 (EXACT) or [2][N] float2 (ORDERED): input
-                               // for the next step; a target's input is the sum over its planes
-    int32_t n_planes;          // accumulator planes per parity (1 in every configuration)
-    int32_t acc_clear;         // the LIF phase zeroes the planes it read (0: every cycle overwrites them)
+    void *acc;                 // [2][N] longlong2 (EXACT) or [2][N] float2 (ORDERED): input for the next step
+    int32_t acc_clear;         // the LIF phase zeroes the input it read (0: every cycle overwrites it)
     uint32_t *bitmap;          // [R][W] fired flags of each step in the ring
     int32_t *ring;             // [R][cap] fired ids of each step in the ring
     int32_t *ring_cnt;         // [R]
@@ -112,21 +110,22 @@ struct StepArgs {
     // target-tiled delivery (BSIM_DELIVERY_TILE). A tile is a target range whose
     // excitatory and inhibitory sums are formed in shared memory. Its sources form
     // runs of consecutive neuron ids; every source of a run owns one (tile, source)
-    // pair. A tile's work units are split into parts, handed to blocks by a per-cycle
-    // queue. A block that finds the queue empty joins the part with the most units
-    // left. Every block that worked on a tile stores (the first to finish) or adds (the
-    // others, once that store is done) its sums into the one accumulator plane.
+    // pair. The work units of all tiles in a row are cut into one share per block, of equal
+    // cost; the part of a share that lies in one tile has number block + tile. Every block that
+    // worked on a tile stores (the first to finish) or adds (the others, once that store is
+    // done) its sums into the accumulator plane.
     int32_t n_tiles;                 // tiles (0: no tiled copy)
-    int32_t n_tiles_u;               // = n_tiles (target ranges)
-    int32_t n_parts;                 // parts over all tiles
-    const int4 *parts;               // [n_parts] {tile, first unit, end unit, part within the tile},
-                                     // largest first
-    unsigned int *part_ctr;          // next part to hand out (reset by the last block of a cycle)
-    unsigned int *part_help;         // [n_parts] blocks helping each part this cycle
-    unsigned int *part_next;         // [n_parts] next unit of each part: any block may take chunks
-                                     // of any part (reset to the first unit by the last block)
-    unsigned int *part_pairs;        // [2][n_parts] entry pairs listed per part, by cycle parity;
-                                     // the previous cycle's count sizes the part's chunks
+    unsigned long long *part_word;   // [part_cap] end unit (high half) and next unit of each part: any block may
+                                     // take chunks of any part
+    int *part_tile;                  // [part_cap] its tile
+    unsigned int *part_help;         // [part_cap] blocks helping it
+    unsigned int *tile_pairs;        // [2][n_tiles] entry pairs listed per tile, by cycle parity; the previous
+                                     // cycle's count sizes the tile's chunks
+    int32_t n_items;                 // cost items: ranges of work units of a tile (delays of a run, or small runs), in
+                                     // tile order
+    const int4 *items;               // [n_items] {tile, first unit, units, targets of the tile (its first item)}
+    const int2 *run_item;            // [runs] first item of each run, delays per item
+    unsigned int *item_clocks;       // [2][n_items] warp clocks spent, by cycle parity
     unsigned int *tile_arrive;       // [2][n_tiles]: blocks that finished a piece of the tile this
                                      // cycle, and whether the first one's store is done (reset by
                                      // the last block)
@@ -201,9 +200,6 @@ struct Engine {
     float *mlp_mem = nullptr;
     // population statistics (device arrays in a: pop_size, pop_indeg, pop_outdeg)
     bool pop_info_ready = false;
-    // tiled copy, host side: synapses and work units per tile (planning the parts)
-    std::vector<int64_t> tile_entries;
-    std::vector<int32_t> tile_units;
 };
 
 }  // namespace bsim

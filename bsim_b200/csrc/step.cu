@@ -198,16 +198,9 @@ static __device__ __forceinline__ void lif_phase(const StepArgs &a, unsigned lon
             const ClassParams *c = a.ctab + a.cls[j];
             float inE, inI;
             if (ACC == BSIM_ACC_EXACT) {
-                // the target's input is the (two's-complement) sum over the planes
-                longlong2 *acc = reinterpret_cast<longlong2 *>(a.acc) + (int64_t)p * a.n_planes * a.N + j;
-                longlong2 q = acc[0];
-                for (int k = 1; k < a.n_planes; k++) {
-                    const longlong2 r = acc[(int64_t)k * a.N];
-                    q.x = (long long)((unsigned long long)q.x + (unsigned long long)r.x);
-                    q.y = (long long)((unsigned long long)q.y + (unsigned long long)r.y);
-                }
-                if (a.acc_clear)
-                    for (int k = 0; k < a.n_planes; k++) acc[(int64_t)k * a.N] = make_longlong2(0, 0);
+                longlong2 *acc = reinterpret_cast<longlong2 *>(a.acc) + (int64_t)p * a.N + j;
+                const longlong2 q = *acc;
+                if (a.acc_clear) *acc = make_longlong2(0, 0);
                 const float sd = __ldg(&c->scale_down);
                 inE = __fmul_rn(__ll2float_rn(q.x), sd);
                 inI = __fmul_rn(__ll2float_rn(q.y), sd);
@@ -330,7 +323,7 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
     const int D = a.D;
     const long long total = s_cum[D];
     unsigned long long ev = 0;
-    unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc) + 2 * (int64_t)pw * a.n_planes * a.N;
+    unsigned long long *acc = reinterpret_cast<unsigned long long *>(a.acc) + 2 * (int64_t)pw * a.N;
     // Segments per warp chunk: PUSH_CHUNK when there are enough for every warp, fewer
     // (down to one) when a cycle has few spikes with long rows, so that more warps
     // share the rows. Chunks go to warps block-interleaved (chunk c to warp c / grid of
@@ -501,7 +494,7 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
                 sI += __shfl_xor_sync(0xffffffffu, sI, o);
             }
             if (lane == 0)
-                reinterpret_cast<longlong2 *>(a.acc)[(int64_t)pw * a.n_planes * a.N + j] = make_longlong2(sE, sI);
+                reinterpret_cast<longlong2 *>(a.acc)[(int64_t)pw * a.N + j] = make_longlong2(sE, sI);
         } else {
             if (lane == 0) reinterpret_cast<float2 *>(a.acc)[(int64_t)pw * a.N + j] = make_float2(fE, fI);
         }
@@ -513,11 +506,23 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // Phase B, tiled: the exact E and I sums of a tile of target neurons are formed
 // in shared memory, so no per-event global atomic is issued. Tiles follow
 // population boundaries and hold up to a few thousand targets (16 bytes of
-// counters each), so each source's row into a tile stays a long segment. A
-// tile's work units are cut into parts; blocks take parts from a per-cycle queue
-// (largest first) and, once it is empty, help the parts with the most work
-// left. The first block to finish a piece of a tile stores its sums into the
-// tile's accumulator plane; the others add theirs after that store.
+// counters each), so each source's row into a tile stays a long segment. The first
+// block to finish a piece of a tile stores its sums into the accumulator plane; the
+// others add theirs after that store.
+//
+// Every block works on one contiguous share of the cycle: the tiles in a row, each cut
+// into items (a run's sources and a few delays: populations fire at different rates and
+// in bursts) with the warp clocks spent on them in the previous cycle, are cut into
+// shares of equal cost, so a block touches one or two tiles, flushes as often, and the
+// blocks end together. Each block finds its share by itself from the items' costs. The
+// units of a share are taken in chunks from a counter, so a block that is done can help
+// where the activity changed since the previous cycle and much is left. Measured against
+// parts of a tile taken from a queue, two per resident block, with the additions below
+// through generic addresses (us per cycle): 100 x 10,000 201 -> 164, 25 x 10,000 92 -> 84,
+// 50 x 10,000 with 20-step delays 128 -> 102, 50 x 5,000 with 50-step delays 171 -> 128,
+// 16 uneven networks 312 -> 309. A cost of a tile by its pairs alone left blocks idle (a
+// tile's runs differ, cold tiles scan fast: 206 on the first network); item clocks that
+// include the flush made shares chase their own splits (178).
 //
 // The tile's sources form runs of consecutive ids; its synapses are grouped by
 // (run, delay, source). A work unit is (run, delay d, 32-source chunk): one lane
@@ -547,8 +552,15 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // every carry is counted once); the fixed-point exponent keeps every sum below
 // 2^61, so the high word cannot overflow.
 // ---------------------------------------------------------------------------
-#ifndef TILE_HELP_MIN
-#define TILE_HELP_MIN 64  // units a part must have left per helping block for another block to join
+// costs in warp clocks: scanning one work unit (at least), one part of a tile, flushing one target
+#ifndef TILE_UNIT_CLOCKS
+#define TILE_UNIT_CLOCKS 16
+#endif
+#ifndef TILE_PART_CLOCKS
+#define TILE_PART_CLOCKS 131072
+#endif
+#ifndef TILE_FLUSH_CLOCKS
+#define TILE_FLUSH_CLOCKS 16
 #endif
 #ifndef TILE_WAIT_SPINS
 #define TILE_WAIT_SPINS (1u << 22)  // ~0.3 s of 64 ns sleeps: far beyond any store phase
@@ -566,16 +578,45 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // lanes adding into scattered targets spread over all shared-memory banks).
 // Two entries at once: both low words first, so the second atomic's latency
 // overlaps the first's (a returned value is waited for only where it is used).
-static __device__ __forceinline__ void carry_add2(char *acc, uint4 v, int hi)
+// acc: shared-memory address of the counters; hi: bytes from a low word to its high word. The
+// addresses are 32-bit shared-memory ones throughout: through a generic pointer the compiler
+// emits both kinds of atomic and a compare-and-swap loop, ten shared accesses per addition.
+static __device__ __forceinline__ unsigned atom_add_shared(unsigned p, unsigned v)
+{
+    unsigned old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(p), "r"(v) : "memory");
+    return old;
+}
+static __device__ __forceinline__ void red_add_shared(unsigned p, unsigned v)
+{
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+}
+static __device__ __forceinline__ void carry_add2(unsigned acc, uint4 v, unsigned hi)
 {
     const unsigned long long u0 = (unsigned long long)__float2ll_rn(__uint_as_float(v.y));
     const unsigned long long u1 = (unsigned long long)__float2ll_rn(__uint_as_float(v.w));
     const unsigned l0 = (unsigned)u0, l1 = (unsigned)u1;
-    unsigned *p0 = reinterpret_cast<unsigned *>(acc + v.x), *p1 = reinterpret_cast<unsigned *>(acc + v.z);
-    const unsigned o0 = atomicAdd(p0, l0);
-    const unsigned o1 = atomicAdd(p1, l1);
-    atomicAdd(p0 + hi, (unsigned)(u0 >> 32) + (o0 + l0 < o0 ? 1u : 0u));
-    atomicAdd(p1 + hi, (unsigned)(u1 >> 32) + (o1 + l1 < o1 ? 1u : 0u));
+    const unsigned p0 = acc + v.x, p1 = acc + v.z;
+    const unsigned o0 = atom_add_shared(p0, l0);
+    const unsigned o1 = atom_add_shared(p1, l1);
+    red_add_shared(p0 + hi, (unsigned)(u0 >> 32) + (o0 + l0 < o0 ? 1u : 0u));
+    red_add_shared(p1 + hi, (unsigned)(u1 >> 32) + (o1 + l1 < o1 ? 1u : 0u));
+}
+static __device__ __forceinline__ uint4 ld_shared16(unsigned p)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(p) : "memory");
+    return v;
+}
+static __device__ __forceinline__ unsigned ld_shared4(unsigned p)
+{
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+static __device__ __forceinline__ void st_shared4(unsigned p, unsigned v)
+{
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
 }
 
 // One 16-byte copy to shared memory, past L1 and evict-first in L2 (read once per
@@ -611,42 +652,127 @@ static __device__ __forceinline__ long long carry_sum(const unsigned *lo, int T)
     return (long long)(((unsigned long long)lo[T] << 32) | (unsigned long long)lo[0]);
 }
 
+// A place in the row of all tiles' work units.
+struct TilePlace {
+    int q;       // tile
+    unsigned u;  // unit
+};
+
+static __device__ __forceinline__ unsigned tile_unit_count(const StepArgs &a, int q)
+{
+    return (unsigned)max(a.tile_units[q], 1);  // a tile without sources is flushed all the same
+}
+// Cost of an item in warp clocks: what its chunks took in the previous cycle, a floor for its units'
+// scan, and for a tile's first item the start, the last warp and the flush of one part.
+static __device__ __forceinline__ unsigned long long item_cost(const StepArgs &a, const unsigned *prev, int i)
+{
+    const int4 it = a.items[i];  // {tile, first unit, units, targets of the tile in its first item}
+    return (unsigned long long)prev[i] + (unsigned long long)(TILE_UNIT_CLOCKS * it.z) +
+           (it.w ? (unsigned long long)(TILE_PART_CLOCKS + TILE_FLUSH_CLOCKS * it.w) : 0ull);
+}
+
+// This block's share [share[0], share[1]) of the units. Every block computes the same costs, so the
+// shares meet. s_scan: one word per warp. Ends with a block barrier.
+static __device__ __forceinline__ void tile_share(const StepArgs &a, const unsigned *prev, unsigned long long *s_scan,
+                                                  TilePlace *share)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (a.n_items + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int i0 = min((int)threadIdx.x * per, a.n_items), i1 = min(i0 + per, a.n_items);
+    unsigned long long sum = 0;
+    for (int i = i0; i < i1; i++) sum += item_cost(a, prev, i);
+    unsigned long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long nb = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += nb;
+    }
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    unsigned long long before = incl - sum, total = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        if (w < warp) before += s_scan[w];
+        total += s_scan[w];
+    }
+    for (int k = 0; k < 2; k++) {
+        const unsigned long long x = (unsigned long long)((double)total * (double)(blockIdx.x + k) / (double)gridDim.x);
+        if (blockIdx.x + k == gridDim.x) {
+            if (threadIdx.x == 0) share[k] = TilePlace{a.n_tiles - 1, tile_unit_count(a, a.n_tiles - 1)};
+        } else if (x >= before && x < before + sum) {
+            unsigned long long c = before;
+            for (int i = i0; i < i1; i++) {
+                const unsigned long long cost = item_cost(a, prev, i);
+                if (x < c + cost) {
+                    const int4 it = a.items[i];
+                    share[k] = TilePlace{it.x, (unsigned)it.y + (unsigned)((float)it.z * ((float)(x - c) / (float)cost))};
+                    break;
+                }
+                c += cost;
+            }
+        }
+    }
+    __syncthreads();
+}
+
 static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &a, unsigned long long t, int pw,
-                                                                unsigned *s_acc, char *s_warp, int *s_part)
+                                                                unsigned *s_acc, char *s_warp, int *s_part,
+                                                                unsigned long long *s_scan, TilePlace *s_share)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int depth = a.tile_depth;
-    char *mine = s_warp + (size_t)warp * TILE_WARP_BYTES(depth);
-    uint4 *ring = reinterpret_cast<uint4 *>(mine) + lane;                   // [depth][32]: this lane's slots
-    unsigned *seg_base = reinterpret_cast<unsigned *>(mine + depth * 512);  // [32]
-    const unsigned ring_sh = (unsigned)__cvta_generic_to_shared(ring);
+    const unsigned acc_sh = (unsigned)__cvta_generic_to_shared(s_acc);
+    const unsigned warp_sh = (unsigned)__cvta_generic_to_shared(s_warp) + warp * TILE_WARP_BYTES(depth);
+    const unsigned ring_sh = warp_sh + 16 * lane;      // [depth][32] pairs: this lane's slots
+    const unsigned seg_sh = warp_sh + depth * 512;     // [32] segment bases
     const unsigned lanes_le = 0xffffffffu >> (31 - lane);
     unsigned long long pol;
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
     unsigned long long ev = 0;
     unsigned long long *s_best = reinterpret_cast<unsigned long long *>(s_part + 2);
-    // the counters start at zero once per launch; each part's flush clears what it read,
-    // so the next part (any tile size up to tile_max) finds them zero
+    // the counters start at zero once per launch; each flush clears what it read, so the next
+    // tile (of any size up to tile_max) finds them zero
     for (int i = threadIdx.x; i < 4 * a.tile_max; i += blockDim.x) s_acc[i] = 0u;
+    const unsigned *prev = a.tile_pairs + (int64_t)((t & 1ull) ^ 1ull) * a.n_tiles;
+    unsigned *clocks = a.item_clocks + (int64_t)(t & 1ull) * a.n_items;
+    tile_share(a, a.item_clocks + (int64_t)((t & 1ull) ^ 1ull) * a.n_items, s_scan, s_share);
+    const TilePlace from = s_share[0], to = s_share[1];
+    // this block's parts, one per tile of its share: number block + tile, unique as shares follow
+    // one another. The word holds the part's end (high half) and its next unit (low half).
+    for (int q = from.q + (int)threadIdx.x; q <= to.q; q += blockDim.x) {
+        const int id = (int)blockIdx.x + q;
+        const unsigned b = q == from.q ? from.u : 0u, e = q == to.q ? to.u : tile_unit_count(a, q);
+        a.part_help[id] = 0u;
+        a.part_tile[id] = q;
+        __threadfence();  // a helper that sees the word sees its tile
+        *reinterpret_cast<volatile unsigned long long *>(a.part_word + id) = ((unsigned long long)e << 32) | min(b, e);
+    }
+    int q_own = from.q;
     for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned q = atomicAdd(a.part_ctr, 1u);
-            s_part[0] = q < (unsigned)a.n_parts ? (int)q : -1;
-            *s_best = 0ull;
+        __syncthreads();  // the parts are published; the last flush has read s_part[1]
+        int id = -1;
+        while (q_own <= to.q && id < 0) {
+            const unsigned b = q_own == from.q ? from.u : 0u, e = q_own == to.q ? to.u : tile_unit_count(a, q_own);
+            if (b < e) id = (int)blockIdx.x + q_own;
+            q_own++;
         }
-        __syncthreads();
-        int pi = s_part[0];
-        const bool helper = pi < 0;
-        if (helper) {
-            // the queue is empty: join the part with the most units left per block already
-            // helping it (at least two chunks each), so that helpers spread over the parts
+        if (id < 0) {
+            // the share is done: join the part with the most left per block already helping it, if
+            // that is more than what another flush of the tile costs
+            if (threadIdx.x == 0) *s_best = 0ull;
+            __syncthreads();
             unsigned long long best = 0ull;
-            for (int i = threadIdx.x; i < a.n_parts; i += blockDim.x) {
-                const unsigned nx = *reinterpret_cast<volatile unsigned *>(a.part_next + i);
-                const unsigned end = (unsigned)a.parts[i].z;
+            for (int i = threadIdx.x; i < (int)gridDim.x + a.n_tiles; i += blockDim.x) {
+                const unsigned long long w = *reinterpret_cast<volatile unsigned long long *>(a.part_word + i);
+                const unsigned nx = (unsigned)w, end = (unsigned)(w >> 32);
+                if (nx >= end) continue;
+                __threadfence();
+                const int q = *reinterpret_cast<volatile int *>(a.part_tile + i);
                 const unsigned hp = *reinterpret_cast<volatile unsigned *>(a.part_help + i);
-                const unsigned left = (nx < end ? end - nx : 0u) / (hp + 1u);
-                const unsigned long long key = ((unsigned long long)left << 32) | (unsigned)i;
+                // entry pairs left, about 8 per unit to scan, for each block then on it
+                const unsigned flush = (unsigned)(a.tile_beg[q + 1] - a.tile_beg[q]);
+                const float left = (float)(end - nx) * ((float)prev[q] / (float)tile_unit_count(a, q) + 8.0f) / (float)(hp + 2u);
+                if (left < (float)flush) continue;
+                const unsigned long long key = ((unsigned long long)__float2uint_rz(left) << 32) | (unsigned)i;
                 best = key > best ? key : best;
             }
 #pragma unroll
@@ -657,44 +783,50 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
             if (lane == 0 && best) atomicMax(s_best, best);
             __syncthreads();
             const unsigned long long b = *s_best;
-            pi = (b >> 32) >= (unsigned long long)TILE_HELP_MIN ? (int)(b & 0xffffffffull) : -1;
-            if (pi >= 0 && threadIdx.x == 0) atomicAdd(a.part_help + pi, 1u);
+            if (b == 0ull) break;
+            id = (int)(b & 0xffffffffull);
+            if (threadIdx.x == 0) atomicAdd(a.part_help + id, 1u);
         }
-        __syncthreads();  // every thread has read s_part / s_best before they are written again
-        if (pi < 0) break;
-        const int4 part = a.parts[pi];  // {tile, first unit, end unit, part within the tile}
-        const int q = part.x, u_end = part.z;
+        const int q = *reinterpret_cast<volatile int *>(a.part_tile + id);
+        unsigned long long *word = a.part_word + id;
         const int tb = a.tile_beg[q], T = a.tile_beg[q + 1] - tb;
         const uint4 *ent = reinterpret_cast<const uint4 *>(a.ent) + a.tile_seg0[q];  // the tile's entry pairs
         const int r0 = a.tile_run_off[q], r1 = a.tile_run_off[q + 1];
         // the warps of every block working on the part take chunks of its units as they become
-        // free: 32 units (one per lane), fewer where the part listed many entry pairs per unit in
+        // free: 32 units (one per lane), fewer where the tile listed many entry pairs per unit in
         // the previous cycle, so that a hot chunk does not hold up the block for long
-        unsigned *pairs_cnt = a.part_pairs + (int64_t)(t & 1ull) * a.n_parts + pi;
-        const unsigned prev = a.part_pairs[(int64_t)((t & 1ull) ^ 1ull) * a.n_parts + pi];
-        const int cs = prev == 0u ? 32
-                                  : (int)max(TILE_MIN_CHUNK, min(32ll, (long long)TILE_CHUNK_PAIRS * (u_end - part.y) /
-                                                                            (long long)prev));
+        unsigned *pairs_cnt = a.tile_pairs + (int64_t)(t & 1ull) * a.n_tiles + q;
+        const int cs = prev[q] == 0u ? 32
+                                     : (int)max(TILE_MIN_CHUNK, min(32ll, (long long)TILE_CHUNK_PAIRS * a.tile_units[q] /
+                                                                              (long long)prev[q]));
         unsigned listed = 0;
         int pads = 0;
         int head = 0, held = 0;  // ring: next slot to fill, slots filled and not yet added
+        int item = -1;           // of the last chunk's first unit
+        unsigned since = 0;
         auto add_oldest = [&]() {
             int k = head - held;
             if (k < 0) k += depth;
-            const uint4 v = ring[k * 32];
-            if (v.y | v.w) carry_add2(reinterpret_cast<char *>(s_acc), v, T);  // zeros past a listing's end add nothing
+            const uint4 v = ld_shared16(ring_sh + k * 512);
+            if (v.y | v.w) carry_add2(acc_sh, v, 4u * T);  // zeros past a listing's end add nothing
             pads += v.w == TILE_PAD_W;
             held--;
         };
         for (;;) {
-            int ub = 0;
-            if (lane == 0) ub = (int)atomicAdd(a.part_next + pi, (unsigned)cs);
-            ub = __shfl_sync(0xffffffffu, ub, 0);
+            unsigned long long w = 0;
+            if (lane == 0) w = atomicAdd(word, (unsigned long long)cs);
+            w = __shfl_sync(0xffffffffu, w, 0);
+            const int ub = (int)(unsigned)w, u_end = (int)(w >> 32);
+            {   // the clocks since the last chunk go to that chunk's item
+                const unsigned now = (unsigned)clock();
+                if (item >= 0 && lane == 0) atomicAdd(clocks + item, now - since);
+                since = now;
+            }
             if (ub >= u_end) break;
             const int u = ub + lane;
             unsigned m = 0;
             const uint32_t *off = a.seg_off;  // the unit's 32 segment starts
-            if (lane < cs && u < u_end) {
+            if (lane < cs && u < u_end && r0 < r1) {
                 int lo = r0, hi = r1 - 1;  // the run that holds unit u
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
@@ -704,6 +836,10 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                 const int n_r = a.run_n[lo], chunks = (n_r + 31) >> 5;
                 const int v = u - a.run_unit0[lo];
                 const int d = v / chunks + 1;
+                if (lane == 0) {
+                    const int2 it = a.run_item[lo];
+                    item = it.x + (d - 1) / it.y;
+                }
                 const int c = v - (d - 1) * chunks;
                 if ((long long)t - d >= 0) {
                     const int64_t s_first = (int64_t)a.run_src0[lo] + 32 * c;
@@ -754,7 +890,7 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                 // segments that hold entries, in lane order: flat position + base = pair of the tile
                 const unsigned full = __ballot_sync(0xffffffffu, len > 0);
                 __syncwarp();
-                if (len > 0) seg_base[__popc(full & lanes_le) - 1] = first - (unsigned)excl;
+                if (len > 0) st_shared4(seg_sh + 4 * (__popc(full & lanes_le) - 1), first - (unsigned)excl);
                 __syncwarp();
                 if (len == 0) excl = -64;  // marks nothing
                 int seg = -1;              // segments that started before the 32 positions
@@ -762,7 +898,7 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                     const unsigned at = (unsigned)(excl - f0);
                     const unsigned marks = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
                     const int f = f0 + lane;
-                    const unsigned base = seg_base[seg + __popc(marks & lanes_le)];
+                    const unsigned base = ld_shared4(seg_sh + 4 * (seg + __popc(marks & lanes_le)));
                     seg += __popc(marks);
                     copy16_async(ring_sh + head * 512, ent + (base + (unsigned)f), f < n_pairs ? 16 : 0, pol);
                     copy_commit();
@@ -815,14 +951,15 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
             if (threadIdx.x == 0) atomicExch(a.tile_arrive + a.n_tiles + q, 1u);
         } else {
             unsigned long long *g = reinterpret_cast<unsigned long long *>(a.acc) + 2 * ((int64_t)pw * a.N + tb);
-            for (int i = threadIdx.x; i < T; i += blockDim.x) {
-                const long long e = carry_sum(s_acc + i, T), v = carry_sum(s_acc + 2 * T + i, T);
-                s_acc[i] = s_acc[T + i] = s_acc[2 * T + i] = s_acc[3 * T + i] = 0u;
-                if (e) red_add_u64(g + 2 * i, (unsigned long long)e);
-                if (v) red_add_u64(g + 2 * i + 1, (unsigned long long)v);
+            // consecutive lanes add consecutive words (E, I, E, I, ...), so that each 32-byte sector
+            // is added to once
+            for (int w = threadIdx.x; w < 2 * T; w += blockDim.x) {
+                unsigned *lo = s_acc + (w >> 1) + (w & 1) * 2 * T;
+                const long long v = carry_sum(lo, T);
+                lo[0] = lo[T] = 0u;
+                if (v) red_add_u64(g + w, (unsigned long long)v);
             }
         }
-        // the next part's queue read (two barriers) orders the flush before the counters' reuse
     }
     return ev;
 }
@@ -987,7 +1124,11 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 {
     __shared__ int s_wcnt[128];
     __shared__ unsigned long long s_ev;
-    __shared__ __align__(8) int s_part[4];  // tiled delivery: the block's part; [2..3] the best part to join
+    // tiled delivery: whether the block is a tile's first finisher ([1]), the best part to join ([2..3]),
+    // the share's scan and bounds
+    __shared__ __align__(8) int s_part[4];
+    __shared__ unsigned long long s_scan[32];
+    __shared__ TilePlace s_share[2];
     __shared__ int s_last;
     // tiled delivery: [4][tile] u32 counters, then each warp's ring and segment bases; push: the
     // warps' segment tables, then the delay window's spike counts (step_dynamic_smem)
@@ -1028,7 +1169,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
                         ((long long)gridDim.x * blockDim.x) >> 5);
     } else if (tiled) {
         ev = tile_phase(a, t, p ^ 1, reinterpret_cast<unsigned *>(s_dyn),
-                        reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part);
+                        reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part, s_scan, s_share);
     } else {
         ev = pull_phase<ACC>(a, t, p ^ 1, a.bitmap, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                              ((long long)gridDim.x * blockDim.x) >> 5);
@@ -1044,25 +1185,19 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     }
     __syncthreads();
     if (s_last) {
-        // every other block has finished this cycle: the parts' unit counters and the
-        // tiles' finisher counts start over
-        if (tiled) {
-            for (int i = threadIdx.x; i < a.n_parts; i += blockDim.x) {
-                a.part_next[i] = (unsigned)a.parts[i].y;
-                a.part_help[i] = 0u;
-            }
+        // every other block has finished this cycle: the tiles' finisher counts start over, and the
+        // next cycle counts its listed pairs from zero (whichever delivery this cycle used)
+        if (tiled)
             for (int i = threadIdx.x; i < 2 * a.n_tiles; i += blockDim.x) a.tile_arrive[i] = 0u;
-        }
-        // the next cycle counts its listed pairs from zero (whichever delivery this cycle used)
-        if (a.part_pairs)
-            for (int i = threadIdx.x; i < a.n_parts; i += blockDim.x)
-                a.part_pairs[(int64_t)((t + 1ull) & 1ull) * a.n_parts + i] = 0u;
+        for (int i = threadIdx.x; i < a.n_tiles; i += blockDim.x)
+            a.tile_pairs[(int64_t)((t + 1ull) & 1ull) * a.n_tiles + i] = 0u;
+        for (int i = threadIdx.x; i < a.n_items; i += blockDim.x)
+            a.item_clocks[(int64_t)((t + 1ull) & 1ull) * a.n_items + i] = 0u;
         if (threadIdx.x == 0) {
             // advance the cycle
             record_advance(a, t);
             *a.ticket = 0u;
             *(a.ticket + 1) = 0u;  // the update's chunk counter
-            if (a.part_ctr) *a.part_ctr = 0u;
             *a.step_ctr = t + 1;
             __threadfence();
         }
