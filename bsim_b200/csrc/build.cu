@@ -32,6 +32,9 @@ cudaError_t step_occupancy(int block, int accumulate, int *blocks_per_sm, size_t
 size_t step_dynamic_smem(const StepArgs &a, int block);
 cudaError_t step_set_smem(int accumulate, size_t bytes);
 
+#ifndef TILE_MAX_DEPTH
+#define TILE_MAX_DEPTH 3
+#endif
 #ifndef LOOP_STEPS
 #define LOOP_STEPS 4096  // cycles of one many-cycle launch at most
 #endif
@@ -439,15 +442,21 @@ static int create_from_arrays(const float *params, const uint8_t *kind, int64_t 
     return BSIM_OK;
 }
 
+// Whether the engine runs many cycles per launch, and in which form (loop_form); a caller who fixes the
+// launch shape gets one launch per cycle.
+static int many_cycles(const Engine &e)
+{
+    return e.opt.block_threads > 0 || e.opt.grid_blocks > 0 ? 0 : loop_form(e.opt, e.N, e.D, e.sm_count);
+}
+
 // Ring, bitmaps, accumulators, counters; launch shape. Shared by both builders.
 static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
 {
     StepArgs &a = e.a;
     a.N = e.N;
     a.D = e.D;
-    // small networks run many cycles per launch, unless the caller fixes the launch shape; the push
-    // form clears two cycles' counters ahead
-    e.loop = e.opt.block_threads > 0 || e.opt.grid_blocks > 0 ? 0 : loop_form(e.opt, e.N, e.D, e.sm_count);
+    // small networks run many cycles per launch; the push form clears two cycles' counters ahead
+    e.loop = many_cycles(e);
     a.R = e.D + (e.loop == 1 ? 4 : 2);
     a.cap = e.N;
     a.W = (e.N + 31) / 32;
@@ -508,9 +517,9 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     // loops of both phases see every SM
     e.block = e.opt.block_threads > 0 ? e.opt.block_threads : 512;
     if (e.block % 32 != 0 || e.block > 512) return fail(BSIM_ERR_ARG, "block_threads must be a multiple of 32 <= 512");
-    // 4 entry pairs in flight per lane; fewer where that lets two blocks share an SM (or one fit)
+    // 2 ring slots per warp (4 entry pairs per lane); one where that lets two blocks share an SM, or one fit
     int bps = 0;
-    for (int depth = 4, best = 0; depth >= 2; depth--) {
+    for (int depth = TILE_MAX_DEPTH, best = 0; depth >= 1; depth--) {
         StepArgs b = a;
         b.tile_depth = depth;
         const size_t sm = step_dynamic_smem(b, e.block);
@@ -545,15 +554,23 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     return BSIM_OK;
 }
 
-// Target tiles: contiguous neuron ranges that never straddle two networks, of
-// near-equal size <= tile (so one shared-memory accumulator array fits them).
-static int plan_tiles(const std::vector<int64_t> &run_beg, int64_t tile, std::vector<int32_t> &tile_beg,
-                      int32_t &tile_max)
+// Target tiles: contiguous neuron ranges of at most `tile` neurons (so one shared-memory
+// accumulator array fits them) that never straddle two networks. run_beg: the first neuron of
+// each population and the end; net: each population's network. A population larger than a tile
+// is cut into near-equal parts; consecutive small ones share a tile (each tile costs a part's
+// start and flush: 16 networks with populations of 539 to 7,379 neurons, 311 -> 303 us per
+// cycle).
+static int plan_tiles(const std::vector<int64_t> &run_beg, const std::vector<int32_t> &net, int64_t tile,
+                      std::vector<int32_t> &tile_beg, int32_t &tile_max)
 {
     tile_beg.clear();
     tile_max = 0;
-    for (size_t r = 0; r + 1 < run_beg.size(); r++) {
-        const int64_t b = run_beg[r], len = run_beg[r + 1] - b;
+    const size_t n = run_beg.size() - 1;
+    for (size_t r = 0; r < n;) {
+        size_t e = r + 1;
+        while (e < n && net[e] == net[r] && run_beg[e + 1] - run_beg[r] <= tile) e++;
+        const int64_t b = run_beg[r], len = run_beg[e] - b;
+        r = e;
         if (len <= 0) continue;
         const int64_t k = (len + tile - 1) / tile;
         for (int64_t i = 0; i < k; i++) {
@@ -857,9 +874,11 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
     std::vector<int64_t> runs = {0};
     for (int64_t i = 1; i < n; i++)
         if ((inst && inst[i] != inst[i - 1]) || (pop && pop[i] != pop[i - 1])) runs.push_back(i);
+    std::vector<int32_t> net;
+    for (int64_t b : runs) net.push_back(inst ? inst[b] : 0);
     runs.push_back(n);
     TileHost th;
-    plan_tiles(runs, auto_tile_size(e.opt, n, e.sm_count, D), th.tile_beg, th.tile_max);
+    plan_tiles(runs, net, auto_tile_size(e.opt, n, e.sm_count, D), th.tile_beg, th.tile_max);
     th.n_u = (int32_t)th.tile_beg.size() - 1;
     const int32_t nu = th.n_u, nt = nu;
     std::vector<int32_t> tile_of(n);
@@ -1405,12 +1424,16 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
     if (tiles) {
         // target ranges follow population boundaries
         std::vector<int64_t> runs;
+        std::vector<int32_t> net;
         for (int k = 0; k < ns; k++)
-            for (int pp = 0; pp < gi[k].P; pp++) runs.push_back(gi[k].nbase + (int64_t)pp * gi[k].n);
+            for (int pp = 0; pp < gi[k].P; pp++) {
+                runs.push_back(gi[k].nbase + (int64_t)pp * gi[k].n);
+                net.push_back(k);
+            }
         runs.push_back(N);
         std::vector<int32_t> tile_beg;
         int32_t tile_max = 0;
-        plan_tiles(runs, auto_tile_size(E.opt, N, E.sm_count, D), tile_beg, tile_max);
+        plan_tiles(runs, net, auto_tile_size(E.opt, N, E.sm_count, D), tile_beg, tile_max);
         const int32_t nu = (int32_t)tile_beg.size() - 1, nt = nu;
         std::vector<TileSeg> segs;
         TileHost th;
@@ -1520,7 +1543,7 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         if ((rc = upload_tiles(E, th))) { free_tmp(); return bail(rc); }
     }
     // push rows (not needed when every step uses the tiled copy)
-    if (!(tiles && E.opt.delivery == BSIM_DELIVERY_TILE)) {
+    if (!(tiles && E.opt.delivery == BSIM_DELIVERY_TILE) || many_cycles(E) == 1) {
         const int64_t nrows = N * (int64_t)D;
         int64_t *d_row; uint2 *d_syn;
         if ((rc = dalloc(E, &d_row, nrows + 1)) || (rc = dalloc(E, &d_syn, S + 1))) { free_tmp(); return bail(rc); }
@@ -1681,7 +1704,7 @@ int bsim_run_async(bsim_engine *eh, int64_t steps)
     int64_t left = steps;
     const int gl = e.opt.graph_steps;
     const bool ordered = e.opt.accumulate == BSIM_ACC_ORDERED;
-    const bool same_mode = e.loop == 1 ? e.a.delivery == BSIM_DELIVERY_PUSH
+    const bool same_mode = e.loop == 1 ? e.a.delivery == BSIM_DELIVERY_PUSH || e.a.delivery == BSIM_DELIVERY_TILE
                                        : e.loop == 2 && (ordered || e.a.delivery == BSIM_DELIVERY_PULL);
     if (left > 0 && gl > 0 && same_mode && !e.a.mlp && !e.a.pstats) {
         TRY(enter_loop(e));
@@ -1736,6 +1759,8 @@ int bsim_stall_tile(bsim_engine *eh, int32_t tile)
     if (!e.a.tile_arrive || tile < 0 || tile >= e.a.n_tiles)
         return fail(BSIM_ERR_ARG, "bsim_stall_tile: the engine has no such tile");
     CK(cudaSetDevice(e.device));
+    TRY(leave_loop(e));  // the wait is in the cycle-by-cycle form: a small engine keeps to it from here on
+    e.loop = 0;
     CK(cudaStreamSynchronize(e.stream));
     // the tile's finisher count of the running cycle (reset by the cycle's last block)
     const unsigned int one = 1u;

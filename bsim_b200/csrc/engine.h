@@ -146,7 +146,7 @@ struct StepArgs {
                                      // counters (E or I by the weight's sign), weight x 2^qexp}; every
                                      // segment starts on an even entry and has even length (padding
                                      // entries have the weight word TILE_PAD_W and any offset)
-    int32_t tile_depth;              // 16-byte entry pairs a lane keeps in flight (2..4)
+    int32_t tile_depth;              // ring slots per warp, of two 16-byte entry pairs per lane (1..3)
     // firing predictor (needs pop_hist)
     const float *mlp;                // [BSIM_MLP_PARAMS] (NULL: off)
     const int32_t *pop_size;         // [n_pops]

@@ -529,11 +529,12 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // reads the chunk's word of the fired bitmap of cycle t-d. Each fired (source,
 // delay) names one segment of 8-byte entries, padded to an even length from an
 // even start. A warp lists up to 32 segments at a time, one per lane, and streams
-// them as one flat range of 16-byte entry pairs: pair k of the range goes to lane
-// k % 32, which finds its segment from the warp's start marks (one warp-wide OR
-// and a population count per 32 pairs), fetches the pair with cp.async into its own
-// slot of a small ring in shared memory, and adds it a few pairs later. The ring
-// keeps copies in flight across listings without holding registers.
+// them as one flat range of 16-byte entry pairs, 64 at a time: two per lane, which
+// finds their segments from the warp's start marks (a warp-wide OR and a population
+// count per 32 pairs), fetches them with cp.async into its own places of a slot of
+// the warp's ring in shared memory, and adds a whole slot's four entries per lane one
+// or two slots later. A listing continues the slot that the last one left open, so
+// the ring stays full across listings without holding registers.
 //
 // What bounds it: the entry stream (8 bytes per event) and the issue slots of the
 // additions. An entry holds the byte offset of its counter and its weight already
@@ -542,8 +543,9 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 // two segments per lane at a time and four register loads per lane with the sign,
 // scale and padding worked out per entry (us per cycle): 50 x 5,000 with 50-step
 // delays 296 -> 171, 16 uneven networks 455 -> 312, 50 x 10,000 with 20-step delays
-// 168 -> 128, 25 x 10,000 106 -> 92, 100 x 10,000 210 -> 201 (bound by HBM while it
-// streams).
+// 168 -> 128, 25 x 10,000 106 -> 92, 100 x 10,000 210 -> 201; slots of 64 pairs carried
+// across listings instead of 32: 25 x 10,000 82 -> 79, 100 x 10,000 164 -> 160 (more slots
+// in flight are level, and 1 is 30 % slower).
 //
 // Exact int64 sums with 32-bit shared atomics: the low word of the fixed-point
 // value is added with an atomic that returns the old word, and the high word
@@ -571,8 +573,8 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 #ifndef TILE_MIN_CHUNK
 #define TILE_MIN_CHUNK 8ll  // units per chunk at least
 #endif
-// shared memory of one warp: the ring (depth x 32 pairs) and the segments' bases
-#define TILE_WARP_BYTES(depth) ((depth) * 512 + 32 * 4)
+// shared memory of one warp: the ring (depth x 64 pairs), the segments' bases, the units that fired
+#define TILE_WARP_BYTES(depth) ((depth) * 1024 + 32 * 4 + 32)
 
 // Counters are [4][tile]: E low, E high, I low, I high words (word-major, so
 // lanes adding into scattered targets spread over all shared-memory banks).
@@ -591,16 +593,21 @@ static __device__ __forceinline__ void red_add_shared(unsigned p, unsigned v)
 {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
 }
-static __device__ __forceinline__ void carry_add2(unsigned acc, uint4 v, unsigned hi)
+// Four entries: all low words first, so that the atomics' latencies overlap (a returned value is
+// waited for only where it is used).
+static __device__ __forceinline__ void carry_add4(unsigned acc, uint4 v, uint4 w, unsigned hi)
 {
-    const unsigned long long u0 = (unsigned long long)__float2ll_rn(__uint_as_float(v.y));
-    const unsigned long long u1 = (unsigned long long)__float2ll_rn(__uint_as_float(v.w));
-    const unsigned l0 = (unsigned)u0, l1 = (unsigned)u1;
-    const unsigned p0 = acc + v.x, p1 = acc + v.z;
-    const unsigned o0 = atom_add_shared(p0, l0);
-    const unsigned o1 = atom_add_shared(p1, l1);
-    red_add_shared(p0 + hi, (unsigned)(u0 >> 32) + (o0 + l0 < o0 ? 1u : 0u));
-    red_add_shared(p1 + hi, (unsigned)(u1 >> 32) + (o1 + l1 < o1 ? 1u : 0u));
+    const unsigned x[4] = {acc + v.x, acc + v.z, acc + w.x, acc + w.z};
+    const unsigned long long u[4] = {(unsigned long long)__float2ll_rn(__uint_as_float(v.y)),
+                                     (unsigned long long)__float2ll_rn(__uint_as_float(v.w)),
+                                     (unsigned long long)__float2ll_rn(__uint_as_float(w.y)),
+                                     (unsigned long long)__float2ll_rn(__uint_as_float(w.w))};
+    unsigned o[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) o[i] = atom_add_shared(x[i], (unsigned)u[i]);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        red_add_shared(x[i] + hi, (unsigned)(u[i] >> 32) + (o[i] + (unsigned)u[i] < o[i] ? 1u : 0u));
 }
 static __device__ __forceinline__ uint4 ld_shared16(unsigned p)
 {
@@ -614,38 +621,43 @@ static __device__ __forceinline__ unsigned ld_shared4(unsigned p)
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
     return v;
 }
+static __device__ __forceinline__ void st_shared16_zero(unsigned p)
+{
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(p), "r"(0) : "memory");
+}
+static __device__ __forceinline__ void st_shared1(unsigned p, int v)
+{
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+}
+static __device__ __forceinline__ int ld_shared1(unsigned p)
+{
+    int v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
 static __device__ __forceinline__ void st_shared4(unsigned p, unsigned v)
 {
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
 }
 
-// One 16-byte copy to shared memory, past L1 and evict-first in L2 (read once per
-// spike); `bytes` = 0 writes zeros and reads nothing.
-static __device__ __forceinline__ void copy16_async(unsigned dst, const uint4 *src, int bytes, unsigned long long pol)
+// One 16-byte copy to shared memory, past L1 and evict-first in L2 (read once per spike).
+static __device__ __forceinline__ void copy16_async(unsigned dst, const uint4 *src, unsigned long long pol, bool on)
 {
-    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst), "l"(src), "r"(bytes),
-                 "l"(pol)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+                 "@p cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n\t}" ::"r"(dst),
+                 "l"(src), "l"(pol), "r"((unsigned)on)
                  : "memory");
+}
+// 1 << n, 0 for n of 32 and more (also those that were negative).
+static __device__ __forceinline__ unsigned bit_or_none(unsigned n)
+{
+    unsigned v;
+    asm("shl.b32 %0, 1, %1;" : "=r"(v) : "r"(n));
+    return v;
 }
 static __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 static __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// The position of the n-th (from 0) set bit of m.
-static __device__ __forceinline__ int nth_set_bit(unsigned m, int n)
-{
-    int b = 0;
-#pragma unroll
-    for (int w = 16; w > 0; w >>= 1) {
-        const int c = __popc(m & ((1u << w) - 1u));
-        if (n >= c) {
-            n -= c;
-            m >>= w;
-            b += w;
-        }
-    }
-    return b;
-}
 
 static __device__ __forceinline__ long long carry_sum(const unsigned *lo, int T)
 {
@@ -722,8 +734,9 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
     const int depth = a.tile_depth;
     const unsigned acc_sh = (unsigned)__cvta_generic_to_shared(s_acc);
     const unsigned warp_sh = (unsigned)__cvta_generic_to_shared(s_warp) + warp * TILE_WARP_BYTES(depth);
-    const unsigned ring_sh = warp_sh + 16 * lane;      // [depth][32] pairs: this lane's slots
-    const unsigned seg_sh = warp_sh + depth * 512;     // [32] segment bases
+    const unsigned ring_sh = warp_sh + 16 * lane;   // [depth][2][32] pairs: this lane's places
+    const unsigned seg_sh = warp_sh + depth * 1024;  // [32] segment bases
+    const unsigned unit_sh = seg_sh + 128;           // [32] lanes of the units that fired
     const unsigned lanes_le = 0xffffffffu >> (31 - lane);
     unsigned long long pol;
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -801,15 +814,16 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                                                                               (long long)prev[q]));
         unsigned listed = 0;
         int pads = 0;
-        int head = 0, held = 0;  // ring: next slot to fill, slots filled and not yet added
-        int item = -1;           // of the last chunk's first unit
+        // ring: the slot being filled and how far (64 pairs: two per lane), slots filled and not yet added
+        int head = 0, filled = 0, held = 0;
+        int item = -1;  // of the last chunk's first unit
         unsigned since = 0;
         auto add_oldest = [&]() {
             int k = head - held;
             if (k < 0) k += depth;
-            const uint4 v = ld_shared16(ring_sh + k * 512);
-            if (v.y | v.w) carry_add2(acc_sh, v, 4u * T);  // zeros past a listing's end add nothing
-            pads += v.w == TILE_PAD_W;
+            const uint4 v = ld_shared16(ring_sh + k * 1024), w = ld_shared16(ring_sh + k * 1024 + 512);
+            carry_add4(acc_sh, v, w, 4u * T);
+            pads += (v.w == TILE_PAD_W) + (w.w == TILE_PAD_W);
             held--;
         };
         for (;;) {
@@ -861,20 +875,27 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                 if (lane >= o) incl += nb;
             }
             const int total = __shfl_sync(0xffffffffu, incl, 31);
+            // the units that fired, in order; rank + start finds a fired source's unit
+            const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+            __syncwarp();
+            if (cnt > 0) st_shared1(unit_sh + __popc(some & lanes_le) - 1, lane);
+            __syncwarp();
+            int unit = -1;  // units that started before the 32 ranks
             for (int b0 = 0; b0 < total; b0 += 32) {
                 // this lane's segment: fired source number b0 + lane of the chunk
                 const int rank = b0 + lane;
-                int ul = 0;  // the lane whose unit holds it
-#pragma unroll
-                for (int w = 16; w > 0; w >>= 1)
-                    if (__shfl_sync(0xffffffffu, incl, ul + w - 1) <= rank) ul += w;
-                const unsigned mu = __shfl_sync(0xffffffffu, m, ul);
-                const int eu = __shfl_sync(0xffffffffu, incl - cnt, ul);
+                const unsigned start = (unsigned)(incl - cnt - b0);
+                const unsigned um = __reduce_or_sync(0xffffffffu, cnt > 0 ? bit_or_none(start) : 0u);
+                const int ul = ld_shared1(unit_sh + unit + __popc(um & lanes_le));  // the lane whose unit holds it
+                unit += __popc(um);
+                unsigned mu = __shfl_sync(0xffffffffu, m, ul);
+                int nth = rank - __shfl_sync(0xffffffffu, incl - cnt, ul);
                 const unsigned long long ou = __shfl_sync(0xffffffffu, (unsigned long long)off, ul);
                 unsigned first = 0;
                 int len = 0;
                 if (rank < total) {
-                    const uint32_t *o = reinterpret_cast<const uint32_t *>(ou) + nth_set_bit(mu, rank - eu);
+                    for (; nth > 0; nth--) mu &= mu - 1u;  // its source is the nth set bit
+                    const uint32_t *o = reinterpret_cast<const uint32_t *>(ou) + (__ffs(mu) - 1);
                     first = __ldg(o);
                     len = (int)(__ldg(o + 1) - first);
                 }
@@ -892,25 +913,42 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                 __syncwarp();
                 if (len > 0) st_shared4(seg_sh + 4 * (__popc(full & lanes_le) - 1), first - (unsigned)excl);
                 __syncwarp();
-                if (len == 0) excl = -64;  // marks nothing
-                int seg = -1;              // segments that started before the 32 positions
-                for (int f0 = 0; f0 < n_pairs; f0 += 32) {
+                // the round's pairs follow the last round's in the slot being filled
+                excl = len == 0 ? -128 : excl + filled;  // (-128: marks nothing)
+                const int end = filled + n_pairs;
+                int seg = -1;  // segments that started before the 32 positions
+                for (int f0 = 0; f0 < end; f0 += 64) {
                     const unsigned at = (unsigned)(excl - f0);
-                    const unsigned marks = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
-                    const int f = f0 + lane;
-                    const unsigned base = ld_shared4(seg_sh + 4 * (seg + __popc(marks & lanes_le)));
-                    seg += __popc(marks);
-                    copy16_async(ring_sh + head * 512, ent + (base + (unsigned)f), f < n_pairs ? 16 : 0, pol);
+                    const unsigned m0 = __reduce_or_sync(0xffffffffu, bit_or_none(at));
+                    const unsigned m1 = __reduce_or_sync(0xffffffffu, bit_or_none(at - 32u));
+                    const int s1 = seg + __popc(m0);
+                    const unsigned b0 = ld_shared4(seg_sh + 4 * (seg + __popc(m0 & lanes_le)));
+                    const unsigned b1 = ld_shared4(seg_sh + 4 * (s1 + __popc(m1 & lanes_le)));
+                    seg = s1 + __popc(m1);
+                    const int p = f0 + lane;
+                    const unsigned dst = ring_sh + head * 1024;
+                    copy16_async(dst, ent + (b0 + (unsigned)(p - filled)), pol, p >= filled && p < end);
+                    copy16_async(dst + 512, ent + (b1 + (unsigned)(p + 32 - filled)), pol, p + 32 >= filled && p + 32 < end);
+                    if (f0 + 64 > end) break;
                     copy_commit();
                     if (++head == depth) head = 0;
                     if (++held == depth) {
-                        if (depth == 4) copy_wait<3>();
-                        else if (depth == 3) copy_wait<2>();
-                        else copy_wait<1>();
+                        if (depth == 2) copy_wait<1>();
+                        else if (depth == 1) copy_wait<0>();
+                        else copy_wait<2>();
                         add_oldest();
                     }
                 }
+                filled = end & 63;
             }
+        }
+        // the rest of the ring; places past the last pair hold zeros, which add nothing
+        if (filled > 0) {
+            const unsigned dst = ring_sh + head * 1024;
+            if (lane >= filled) st_shared16_zero(dst);
+            if (lane + 32 >= filled) st_shared16_zero(dst + 512);
+            if (++head == depth) head = 0;
+            held++;
         }
         copy_wait<0>();
         while (held > 0) add_oldest();
@@ -1122,12 +1160,10 @@ static __device__ __forceinline__ void record_advance(const StepArgs &a, unsigne
 template <int ACC>
 __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel(const __grid_constant__ StepArgs a)
 {
-    __shared__ int s_wcnt[128];
     __shared__ unsigned long long s_ev;
     // tiled delivery: whether the block is a tile's first finisher ([1]), the best part to join ([2..3]),
     // the share's scan and bounds
     __shared__ __align__(8) int s_part[4];
-    __shared__ unsigned long long s_scan[32];
     __shared__ TilePlace s_share[2];
     __shared__ int s_last;
     // tiled delivery: [4][tile] u32 counters, then each warp's ring and segment bases; push: the
@@ -1135,6 +1171,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     extern __shared__ __align__(16) unsigned long long s_dyn[];
     PushSeg *s_seg = reinterpret_cast<PushSeg *>(s_dyn);
     long long *s_cum = reinterpret_cast<long long *>(s_seg + MAX_WARPS * PUSH_CHUNK);
+    int *s_wcnt = reinterpret_cast<int *>(s_dyn);  // [128] the update's, after the delivery
     // a raised error flag stops every later cycle (block-uniform test)
     if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
     const unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
@@ -1169,7 +1206,8 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
                         ((long long)gridDim.x * blockDim.x) >> 5);
     } else if (tiled) {
         ev = tile_phase(a, t, p ^ 1, reinterpret_cast<unsigned *>(s_dyn),
-                        reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part, s_scan, s_share);
+                        reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part,
+                        s_dyn + 2 * a.tile_max, s_share);  // (the share's scan is done before the rings are used)
     } else {
         ev = pull_phase<ACC>(a, t, p ^ 1, a.bitmap, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                              ((long long)gridDim.x * blockDim.x) >> 5);
@@ -1815,13 +1853,15 @@ cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream
 }
 
 // Whether an engine of these sizes can run many cycles per launch (0: no, 1: push form, 2: pull
-// form): half of a block's warps own neurons at most. Tiled and AUTO delivery and longer delays
+// form): half of a block's warps own neurons at most. An engine asked to deliver tiled takes the push
+// form too: the spikes are the same, and at these sizes a tiled cycle is a launch and a chain of
+// dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.3). AUTO delivery and longer delays
 // take one launch per cycle.
 int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
 {
     const int64_t W = (N + 31) / 32;
     if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
-    if (o.accumulate != BSIM_ACC_ORDERED && o.delivery == BSIM_DELIVERY_PUSH)
+    if (o.accumulate != BSIM_ACC_ORDERED && (o.delivery == BSIM_DELIVERY_PUSH || o.delivery == BSIM_DELIVERY_TILE))
         return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
     const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + 2) * W;
     return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps <= LOOP_MAX_SMEM ? 2 : 0;

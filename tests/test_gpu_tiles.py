@@ -43,7 +43,8 @@ def test_tiled_listing_edges(tile_size, block):
     n, steps = 2300, 150
     params, src, dst, w, d = network(n, seed=tile_size + block)
     eng = B.Engine.from_arrays(params, src, dst, w, d, DT,
-                               opts=B.options(delivery=B.DELIVERY_TILE, tile_size=tile_size, block_threads=block))
+                               opts=B.options(delivery=B.DELIVERY_TILE, tile_size=tile_size, block_threads=block,
+                                              graph_steps=0))  # cycle by cycle: the tiled kernel at this size
     eng.record(steps, n * steps)
     eng.run(steps)
     ref = oracle.run(params, src, dst, w, d, DT, steps, record_steps=steps, acc_mode=oracle.ACC_FIXED,
@@ -64,10 +65,47 @@ def test_largest_tile_fits():
     params[:, 9] = rng.uniform(5e-9, 40e-9, n)
     src, dst = rng.integers(0, n, 20 * n).astype(np.int32), rng.integers(0, n, 20 * n).astype(np.int32)
     w, d = rng.uniform(-2e-10, 2e-10, 20 * n).astype(np.float32), rng.integers(1, 4, 20 * n).astype(np.int32)
-    eng = B.Engine.from_arrays(params, src, dst, w, d, DT, opts=B.options(delivery=B.DELIVERY_TILE, tile_size=12288))
+    eng = B.Engine.from_arrays(params, src, dst, w, d, DT, opts=B.options(delivery=B.DELIVERY_TILE, tile_size=12288, graph_steps=0))
     eng.run(steps)
     ref = oracle.run(params, src, dst, w, d, DT, steps, acc_mode=oracle.ACC_FIXED, qexp=int(eng.qexp()[0]))
     assert np.array_equal(eng.fire_count(), ref["fire_count"])
     assert np.array_equal(eng.state()["v"], ref["final_state"][:, 0])
     assert eng.info().events_total == ref["events_per_step"].sum() > 0
     eng.close()
+
+
+@pytest.mark.parametrize("length", [1, 3, 255, 256, 257, 300])
+def test_segment_lengths_and_small_populations_in_one_tile(length):
+    """Segments around the bank ordering's limit, populations of 7 to 90 neurons sharing tiles, a
+    population without sources, two networks in one engine (tiles do not straddle them)."""
+    sizes, nets = [7, 30, 90, 41, 12, 60, 700], [0, 0, 0, 0, 1, 1, 1]
+    n, steps = sum(sizes), 120
+    rng = np.random.default_rng(length)
+    pop = np.repeat(np.arange(7), sizes).astype(np.int32)
+    inst = np.repeat(nets, sizes).astype(np.int32)
+    params = np.tile(np.array(LIF, np.float32), (n, 1))
+    params[:, 9] = rng.uniform(2e-9, 30e-9, n)
+    src, dst, w, d = [], [], [], []
+    for a, b in ((0, 1), (0, 2), (1, 2), (2, 3), (4, 5), (5, 6), (6, 6)):
+        s, t = np.nonzero(pop == a)[0], np.nonzero(pop == b)[0]
+        for x in s:
+            k = min(length, len(t))
+            src += [x] * k
+            dst += rng.choice(t, k, replace=False).tolist()
+            d += [1 + x % 3] * k
+    w = rng.uniform(-2e-10, 2e-10, len(src)).astype(np.float32)
+    src, dst, d = (np.asarray(v, np.int32) for v in (src, dst, d))
+    eng = B.Engine.from_arrays(params, src, dst, w, d, DT, pop=pop, instance=inst,
+                               opts=B.options(delivery=B.DELIVERY_TILE, tile_size=600, graph_steps=0))
+    eng.run(steps)
+    q = eng.qexp()
+    ref = oracle.run(params, src, dst, w, d, DT, steps, acc_mode=oracle.ACC_FIXED, qexp=q[inst], instance=inst)
+    assert np.array_equal(eng.fire_count(), ref["fire_count"]) and ref["fire_count"].sum() > 0
+    assert np.array_equal(eng.state()["v"], ref["final_state"][:, 0])
+    assert eng.info().events_total == ref["events_per_step"].sum()
+    # the many-cycle launch gives the same
+    loop = B.Engine.from_arrays(params, src, dst, w, d, DT, pop=pop, instance=inst,
+                                opts=B.options(delivery=B.DELIVERY_TILE))
+    loop.run(steps)
+    assert np.array_equal(loop.fire_count(), ref["fire_count"])
+    assert loop.info().events_total == eng.info().events_total
