@@ -142,6 +142,7 @@ static uint32_t f2u(float f)
 
 static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab);
 static bool wants_tiles(const bsim_options &o, int32_t D);
+static int many_cycles(const Engine &e);
 static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, const int32_t *src,
                             const int32_t *dst, const float *weight, const int32_t *delay, int64_t s);
 
@@ -512,6 +513,7 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     if (a.n_tiles > 0 && e.opt.delivery == BSIM_DELIVERY_TILE) a.delivery = BSIM_DELIVERY_TILE;
     // every cycle of a tiled-only engine overwrites all planes of the parity it
     // delivers into, so the LIF phase need not clear them; any other mode adds
+    a.mean_outdeg = e.N ? (float)((double)e.S / (double)e.N) : 0.0f;
     a.acc_clear = a.delivery == BSIM_DELIVERY_TILE ? 0 : 1;
     // launch shape: all blocks resident (occupancy-sized grid), so the grid-stride
     // loops of both phases see every SM
@@ -603,6 +605,25 @@ static bool wants_tiles(const bsim_options &o, int32_t D)
 {
     return o.accumulate == BSIM_ACC_EXACT && D <= 64 && o.build_tiles >= 0 &&
            (o.build_tiles > 0 || o.delivery == BSIM_DELIVERY_TILE || o.delivery == BSIM_DELIVERY_AUTO);
+}
+
+// Push delivery of a large network holds the tiled copy too, and delivers its busy cycles from it: the
+// sums are the same, and one L2 reduction per event (~1.5e11/s) is what bounds a pushed cycle. The
+// line: a tiled cycle costs ~35 us + 2 to 3 ps per event, a pushed one ~10 us + 6.5 to 11 ps (us per
+// cycle, pushed / tiled: 1.5e7 events 121 / 79, 3.0e7 with 50-step delays 331 / 127, 6.4e7 440 / 160,
+// 4.8e8 with 50-step delays 3,040 / 1,280), so cycles above TILE_MIN_EVENTS. Tiled shares follow the
+// previous cycle, most of whose spikes are delivered again with another delay: delays of at least 4
+// steps. Only for generated networks (the copy is made on the GPU, in about the time of the rows) and
+// where a quarter of the device's memory stays free; build_tiles = -1 keeps the rows alone.
+#define TILE_MIN_EVENTS 7.0e6f
+static bool push_holds_tiles(const Engine &e)
+{
+    if (e.opt.accumulate != BSIM_ACC_EXACT || e.opt.delivery != BSIM_DELIVERY_PUSH || e.opt.build_tiles != 0 ||
+        e.D < 4 || e.D > 64 || e.S < 50000000 || many_cycles(e))
+        return false;
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+    return (double)free - (18.0 * (double)e.S + 24.0 * (double)e.N * e.D) > 0.25 * (double)total;
 }
 
 // Host-side description of the tiled copy.
@@ -1420,7 +1441,9 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         E.a.csc_d = d_cd;
     }
     // target-tiled copy
-    const bool tiles = wants_tiles(E.opt, D);
+    const bool busy_tiles = push_holds_tiles(E);
+    const bool tiles = wants_tiles(E.opt, D) || busy_tiles;
+    E.a.tile_events = busy_tiles ? TILE_MIN_EVENTS : 0.0f;
     if (tiles) {
         // target ranges follow population boundaries
         std::vector<int64_t> runs;
@@ -2305,6 +2328,8 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
     if (e.a.row_off) modes.push_back(BSIM_DELIVERY_PUSH);
     if (e.a.n_tiles > 0) modes.push_back(BSIM_DELIVERY_TILE);
     const int saved_block = e.block, saved_grid = e.grid, saved_del = e.a.delivery;
+    const float saved_events = e.a.tile_events;
+    e.a.tile_events = 0.0f;  // a trial of push pushes every cycle
     cudaEvent_t ev0, ev1;
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
@@ -2363,6 +2388,7 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
     }
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
+    e.a.tile_events = saved_events;
     e.block = best_b;
     e.grid = best_g;
     // an AUTO engine keeps choosing per cycle; a fixed one takes the fastest mode

@@ -1161,6 +1161,7 @@ template <int ACC>
 __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel(const __grid_constant__ StepArgs a)
 {
     __shared__ unsigned long long s_ev;
+    __shared__ int s_dm;
     // tiled delivery: whether the block is a tile's first finisher ([1]), the best part to join ([2..3]),
     // the share's scan and bounds
     __shared__ __align__(8) int s_part[4];
@@ -1177,18 +1178,24 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     const unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
     const int p = (int)(t & 1ull);
     const int cur = (int)(t % (unsigned long long)a.R);
-    int dm = a.deliv_sel ? *a.deliv_sel : a.delivery;
-    if (dm == BSIM_DELIVERY_AUTO) dm = a.pstats ? auto_delivery(a, t) : BSIM_DELIVERY_PUSH;
-    if (dm == BSIM_DELIVERY_TILE && a.n_tiles == 0) dm = BSIM_DELIVERY_PUSH;
+    // the cycle's delivery mode, by one warp (the spike counts it reads are a hot spot when every warp
+    // of the GPU reads them)
+    if (threadIdx.x < 32) {
+        int dm = a.deliv_sel ? *a.deliv_sel : a.delivery;
+        if (dm == BSIM_DELIVERY_AUTO) dm = a.pstats ? auto_delivery(a, t) : BSIM_DELIVERY_PUSH;
+        else if (dm == BSIM_DELIVERY_PUSH && a.tile_events > 0.0f)
+            dm = window_spikes(a, t) * a.mean_outdeg > a.tile_events * (float)a.D ? BSIM_DELIVERY_TILE : BSIM_DELIVERY_PUSH;
+        if (dm == BSIM_DELIVERY_TILE && a.n_tiles == 0) dm = BSIM_DELIVERY_PUSH;
+        if (threadIdx.x == 0) s_dm = dm;
+        if (ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_PUSH)
+            delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
+    }
     if (a.mlp && blockIdx.x == 0 && threadIdx.x == 32) {
         // slot t+2 is next written by cycle t+1's prediction
         a.pred_sum[((t + 2) & 3) * 2 + 0] = 0.0f;
         a.pred_sum[((t + 2) & 3) * 2 + 1] = 0.0f;
     }
-    const bool push = ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_PUSH;
-    const bool tiled = ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_TILE;
     if (threadIdx.x == 0) s_ev = 0;
-    if (push && threadIdx.x < 32) delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // slot t+1 is neither written (LIF writes slot t) nor read (delivery reads t-1..t-D) now
         a.ring_cnt[(t + 1) % (unsigned long long)a.R] = 0;
@@ -1198,7 +1205,9 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_pops; i += gridDim.x * blockDim.x) nxt[i] = 0;
     }
     record_phase(a, t);
-    __syncthreads();  // publishes s_cum and s_ev
+    __syncthreads();  // publishes s_dm, s_cum and s_ev
+    const bool push = ACC != BSIM_ACC_ORDERED && s_dm == BSIM_DELIVERY_PUSH;
+    const bool tiled = ACC != BSIM_ACC_ORDERED && s_dm == BSIM_DELIVERY_TILE;
     unsigned long long ev;
     if (push) {
         ev = push_phase(a, t, p ^ 1, s_cum, s_seg + (threadIdx.x >> 5) * PUSH_CHUNK,

@@ -75,8 +75,9 @@ typedef struct bsim_options {
     int32_t graph_steps;   /* steps captured per CUDA graph by bsim_run (0: plain launches) */
     int32_t block_threads; /* threads per block of the step kernel (0: autotuned) */
     int32_t grid_blocks;   /* blocks of the step kernel (0: autotuned) */
-    int32_t build_tiles;   /* 1: also build the target-tiled copy; 0: only for TILE/AUTO; -1: never
-                              (an AUTO engine then pushes every cycle; saves ~8 B per synapse) */
+    int32_t build_tiles;   /* 1: also build the target-tiled copy; 0: for TILE/AUTO, and for large generated
+                              PUSH networks (their busy cycles are delivered from it); -1: never (an AUTO
+                              engine then pushes every cycle; saves ~8 B per synapse) */
     int32_t tile_size;     /* target neurons per tile (0: chosen from the network size and delays, <= 5000) */
     int32_t reserved[7];
 } bsim_options;

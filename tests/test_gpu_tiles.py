@@ -109,3 +109,25 @@ def test_segment_lengths_and_small_populations_in_one_tile(length):
     loop.run(steps)
     assert np.array_equal(loop.fire_count(), ref["fire_count"])
     assert loop.info().events_total == eng.info().events_total
+
+
+def test_busy_cycles_of_a_large_pushed_network():
+    """A generated network large enough to hold the tiled copy beside its push rows: quiet cycles are
+    pushed, busy ones tiled, with the spikes, state and events of the rows alone (build_tiles = -1)."""
+    from bsim_b200 import workloads as W
+    sp = W.cuba(12, 6500, 2000, 6, seed=5)
+    out = []
+    for bt in (0, -1):
+        eng = B.Engine.generated(sp, DT, opts=B.options(build_tiles=bt))
+        per = []
+        for n in [1] * 8 + [10] * 12:  # the first cycles' deliveries grow from nothing
+            e0 = eng.info().events_total
+            eng.run(n)
+            per.append((eng.info().events_total - e0) / n)
+        out.append((eng.fire_count(), eng.state(), per, eng.info().device_bytes))
+        eng.close()
+    (fa, sa, pa, ba), (fb, sb, pb, bb) = out
+    assert ba > 1.5 * bb  # both copies were held
+    assert min(pa) < 3e6 and max(pa) > 9e6  # both modes ran
+    assert pa == pb and np.array_equal(fa, fb)
+    assert all(np.array_equal(sa[k], sb[k]) for k in sa)
