@@ -456,9 +456,8 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     StepArgs &a = e.a;
     a.N = e.N;
     a.D = e.D;
-    // small networks run many cycles per launch; the push form clears two cycles' counters ahead
-    e.loop = many_cycles(e);
-    a.R = e.D + (e.loop == 1 ? 4 : 2);
+    e.loop = many_cycles(e);  // small networks run many cycles per launch
+    a.R = e.D + (e.loop ? LOOP_EXTRA_SLOTS : 2);
     a.cap = e.N;
     a.W = (e.N + 31) / 32;
     ClassParams *d_ctab;

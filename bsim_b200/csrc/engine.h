@@ -15,6 +15,11 @@ namespace bsim {
 // own zero weight is stored as +0.0f there).
 constexpr uint32_t TILE_PAD_W = 0x80000000u;
 
+// Ring slots beyond the longest delay in a many-cycle engine: an interval of two cycles t, t + 1
+// clears the counters of t + 2 and t + 3 while a slower block may still copy the spikes of t - 2 and
+// t - 1 into the recording, so t + 3 and t - 2 need slots of their own also with 1-step delays.
+constexpr int LOOP_EXTRA_SLOTS = 5;
+
 // One neuron class. For LIF_brian neurons: a folded parameter tuple, the
 // per-population part of LIFENeuron::reset's output (src/neuron/lif/LIFENeuron.cpp:68-112);
 // v_tmp depends on i_offset and is kept per neuron. Input-drive neurons
