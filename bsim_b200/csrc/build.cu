@@ -1705,7 +1705,7 @@ static int enter_loop(Engine &e)
 {
     if (e.in_loop) return BSIM_OK;
     if (e.a.rec && e.a.rec_ids) CK(launch_record_flush(e));
-    if (e.loop == 1) CK(launch_loop_enter(e));
+    CK(launch_loop_enter(e));
     e.in_loop = true;
     return BSIM_OK;
 }

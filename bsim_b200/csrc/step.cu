@@ -440,66 +440,115 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
 // row order with warp shuffles, so the fp32 sum is formed in exactly the order
 // of the reference's loop over pSynapses.
 // ---------------------------------------------------------------------------
-// bitmap: [R][W] fired flags (global memory, or a copy of them in shared memory);
-// warp_lin of n_warps: this warp's number among those that deliver.
+// The scan waits for its loads, so a warp has those of PULL_LOADS chunks in flight (40 x 5,000
+// neurons, 1e8 synapses: 770 -> 465 us per cycle EXACT, 720 -> 475 ORDERED).
+// ---------------------------------------------------------------------------
+#ifndef PULL_LOADS
+#define PULL_LOADS 4
+#endif
+#define PULL_NO_DELAY (1 << 20)  // of a lane past the row's end
+
+// One target's input: the active weights of consecutive entries, a chunk of 32 at a time.
 template <int ACC>
-static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &a, unsigned long long t, int pw,
-                                                                const uint32_t *bitmap, long long warp_lin,
-                                                                long long n_warps)
-{
-    const int lane = threadIdx.x & 31;
-    const int W = (int)a.W, R = a.R, cur = (int)(t % (unsigned long long)a.R);
-    const int d_max = (long long)t < a.D ? (int)t : a.D;  // cycles before the first fired nothing
-    unsigned long long ev = 0;
-    for (long long j = warp_lin; j < a.N; j += n_warps) {
-        const int64_t c0 = a.col_off[j], c1 = a.col_off[j + 1];
-        const float sc = (ACC == BSIM_ACC_EXACT) ? __ldg(&a.ctab[a.cls[j]].scale_up) : 0.0f;
-        long long sE = 0, sI = 0;
-        float fE = 0.0f, fI = 0.0f;
-        for (int64_t k0 = c0; k0 < c1; k0 += 32) {
-            const int64_t e = k0 + lane;
-            bool act = false;
-            float w = 0.0f;
-            if (e < c1) {
-                const uint32_t s = __ldcs(a.csc_src + e);
-                const int d = (int)__ldcs(a.csc_d + e) + 1;
-                w = __ldcs(a.csc_w + e);
-                if (d <= d_max) {
-                    const int slot = cur >= d ? cur - d : cur - d + R;
-                    act = (bitmap[(int64_t)slot * W + (s >> 5)] >> (s & 31)) & 1u;
-                }
+struct PullSum {
+    long long qE = 0, qI = 0;    // EXACT: this lane's part
+    float fE = 0.0f, fI = 0.0f;  // ORDERED: the sums, in every lane
+
+    __device__ __forceinline__ int add(bool act, float w, float sc)
+    {
+        unsigned m = __ballot_sync(0xffffffffu, act);
+        const int n = __popc(m);
+        if (ACC == BSIM_ACC_EXACT) {
+            if (act) {
+                const long long q = __float2ll_rn(__fmul_rn(w, sc));
+                if (w >= 0.0f) qE += q;
+                else qI += q;
             }
-            unsigned m = __ballot_sync(0xffffffffu, act);
-            ev += __popc(m);
-            if (ACC == BSIM_ACC_EXACT) {
-                if (act) {
-                    const long long q = __float2ll_rn(__fmul_rn(w, sc));
-                    if (w >= 0.0f) sE += q;
-                    else sI += q;
-                }
-            } else {
-                while (m) {
-                    const int b = __ffs(m) - 1;
-                    const float wb = __shfl_sync(0xffffffffu, w, b);
-                    if (wb >= 0.0f) fE = __fadd_rn(fE, wb);
-                    else fI = __fadd_rn(fI, wb);
-                    m &= m - 1;
-                }
+        } else {
+            while (m) {
+                const int b = __ffs(m) - 1;
+                const float wb = __shfl_sync(0xffffffffu, w, b);
+                if (wb >= 0.0f) fE = __fadd_rn(fE, wb);
+                else fI = __fadd_rn(fI, wb);
+                m &= m - 1;
             }
         }
+        return n;
+    }
+    // Target i's input, by lane 0.
+    __device__ __forceinline__ void store(void *acc, int64_t i)
+    {
         if (ACC == BSIM_ACC_EXACT) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                sE += __shfl_xor_sync(0xffffffffu, sE, o);
-                sI += __shfl_xor_sync(0xffffffffu, sI, o);
+                qE += __shfl_xor_sync(0xffffffffu, qE, o);
+                qI += __shfl_xor_sync(0xffffffffu, qI, o);
             }
-            if (lane == 0)
-                reinterpret_cast<longlong2 *>(a.acc)[(int64_t)pw * a.N + j] = make_longlong2(sE, sI);
-        } else {
-            if (lane == 0) reinterpret_cast<float2 *>(a.acc)[(int64_t)pw * a.N + j] = make_float2(fE, fI);
         }
+        if ((threadIdx.x & 31) != 0) return;
+        if (ACC == BSIM_ACC_EXACT) reinterpret_cast<longlong2 *>(acc)[i] = make_longlong2(qE, qI);
+        else reinterpret_cast<float2 *>(acc)[i] = make_float2(fE, fI);
     }
-    return lane == 0 ? ev : 0ull;
+};
+
+// Whether source `src` fired `d` cycles before the cycle in ring slot `slot`; d_max: later cycles only.
+static __device__ __forceinline__ unsigned pull_fired(const uint32_t *bitmap, int W, int R, int slot, int d_max,
+                                                      uint32_t src, int d)
+{
+    if (d > d_max) return 0u;
+    const int s = slot >= d ? slot - d : slot - d + R;
+    return (bitmap[(int64_t)s * W + (src >> 5)] >> (src & 31)) & 1u;
+}
+
+// The entries [c0, c1) of the pull rows, one per lane and chunk: test(source, delay) of several
+// chunks, then add(what test returned, weight, chunk's first entry) chunk by chunk.
+template <typename Test, typename Add>
+static __device__ __forceinline__ void pull_entries(const StepArgs &a, int64_t c0, int64_t c1, Test test, Add add)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t k0 = c0; k0 < c1; k0 += 32 * PULL_LOADS) {
+        uint32_t src[PULL_LOADS];
+        int d[PULL_LOADS];
+        float w[PULL_LOADS];
+        unsigned r[PULL_LOADS];
+#pragma unroll
+        for (int u = 0; u < PULL_LOADS; u++) {
+            const int64_t e = k0 + u * 32 + lane;
+            src[u] = 0;
+            d[u] = PULL_NO_DELAY;
+            w[u] = 0.0f;
+            if (e < c1) {
+                src[u] = __ldcs(a.csc_src + e);
+                d[u] = (int)__ldcs(a.csc_d + e) + 1;
+                w[u] = __ldcs(a.csc_w + e);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PULL_LOADS; u++) r[u] = test(src[u], d[u]);
+#pragma unroll
+        for (int u = 0; u < PULL_LOADS; u++)
+            if (k0 + u * 32 < c1) add(r[u], w[u], k0 + u * 32);
+    }
+}
+
+template <int ACC>
+static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &a, unsigned long long t, int pw)
+{
+    const long long warp_lin = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int W = (int)a.W, R = a.R, cur = (int)(t % (unsigned long long)R);
+    const int d_max = (long long)t < a.D ? (int)t : a.D;  // cycles before the first fired nothing
+    const int64_t plane = (int64_t)pw * a.N;
+    unsigned long long ev = 0;
+    for (long long j = warp_lin; j < a.N; j += n_warps) {
+        const float sc = (ACC == BSIM_ACC_EXACT) ? __ldg(&a.ctab[a.cls[j]].scale_up) : 0.0f;
+        PullSum<ACC> x;
+        pull_entries(a, a.col_off[j], a.col_off[j + 1],
+                     [&](uint32_t src, int d) { return pull_fired(a.bitmap, W, R, cur, d_max, src, d); },
+                     [&](unsigned act, float w, int64_t) { ev += x.add(act != 0, w, sc); });
+        x.store(a.acc, plane + j);
+    }
+    return (threadIdx.x & 31) == 0 ? ev : 0ull;
 }
 
 // ---------------------------------------------------------------------------
@@ -1218,8 +1267,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
                         reinterpret_cast<char *>(s_dyn + 2 * a.tile_max), s_part,
                         s_dyn + 2 * a.tile_max, s_share);  // (the share's scan is done before the rings are used)
     } else {
-        ev = pull_phase<ACC>(a, t, p ^ 1, a.bitmap, ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                             ((long long)gridDim.x * blockDim.x) >> 5);
+        ev = pull_phase<ACC>(a, t, p ^ 1);
     }
     if (ev) atomicAdd(&s_ev, ev);
     lif_phase<ACC>(a, t, p, cur, s_wcnt);
@@ -1270,9 +1318,14 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 //     that a population that fires together spreads over the GPU.
 //     10 x 1,000 neurons (100 Hz): 10.2 -> 3.3 us per cycle; 5,000 neurons behind
 //     Poisson drives 13.7 -> 3.9; 20 x 1,000 all-to-all 18.1 -> 6.2.
-//   * Pull (and the ORDERED sums): one cycle per barrier; the update's owners and
-//     the target rows run side by side, with the delay window's fired flags in
-//     shared memory. 10 x 1,000 neurons: 12.8 -> 10.0 us per cycle.
+//   * Pull (and the ORDERED sums): a block sums the input of its own neurons, so the update
+//     follows without a barrier and again two cycles are run between barriers: the input of
+//     cycle t takes the spikes up to t - 2, that of t + 1 those up to t - 1, and one scan of
+//     the rows tests both. The delay window's fired flags and the rows (8 bytes an entry,
+//     as far as they fit) stay in shared memory. 10 x 1,000 neurons, ORDERED: 11.6 -> 5.1
+//     us per cycle (9.2 with one cycle per barrier and the rows read from L2); 36 x 1,000
+//     31.9 -> 13.2; 12 x 3,000 at 2 kHz 107 -> 57. What is left of the first is the scan's
+//     instructions (110 entries a row, two tests each), the barrier and the flags' exchange.
 //
 // The fire ring, its counts and the fired flags are kept as step_kernel keeps them,
 // so the two can follow one another (loop_enter_kernel, loop_leave_kernel). Data that
@@ -1298,7 +1351,12 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 #ifndef LOOP_WAIT_SPINS
 #define LOOP_WAIT_SPINS (1u << 22)  // seconds: a cycle takes microseconds
 #endif
-#define LOOP_MAX_SMEM ((size_t)160 * 1024)  // pull: bitmaps kept in shared memory
+#define LOOP_MAX_SMEM ((size_t)160 * 1024)
+// Pull: the fired flags, and the rows of the block's neurons as far as they fit (none for a launch of
+// fewer cycles than PULL_LOOP_HOLD, which would read most of them once).
+#define PULL_LOOP_SMEM ((size_t)216 * 1024)
+#define PULL_LOOP_WORDS (LOOP_WARPS / 2)  // words of fired flags per block at most (loop_form)
+#define PULL_LOOP_HOLD 3
 #define LOOP_ERR (1ull << 40)  // one block's error in a barrier counter; arrivals are below
 
 static __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
@@ -1667,80 +1725,198 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
 }
 
 template <int ACC>
-__global__ void __launch_bounds__(PULL_LOOP_THREADS, 1) pull_loop_kernel(const __grid_constant__ StepArgs a, int steps)
+__global__ void __launch_bounds__(PULL_LOOP_THREADS, 1)
+    pull_loop_kernel(const __grid_constant__ StepArgs a, int steps, int room)
 {
     __shared__ bool s_stop, s_err;
-    extern __shared__ __align__(16) unsigned long long s_dyn[];  // [R][W] the fired flags
+    __shared__ longlong2 s_in[LOOP_CYCLES][PULL_LOOP_WORDS * 32];  // input of cycles t, t + 1 of this block's neurons
+    extern __shared__ __align__(16) unsigned long long s_dyn[];    // [R][W] the fired flags, then the warps' rows
     uint32_t *s_bm = reinterpret_cast<uint32_t *>(s_dyn);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = (int)a.W, R = a.R, D = a.D;
+    uint2 *rows = reinterpret_cast<uint2 *>(s_dyn + ((size_t)R * W + 1) / 2) + (size_t)warp * room;
     if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
     unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
-    // owners: warp w of block b owns word w * grid + b of the fired flags, if there is one
+    // the block's neurons: words i * grid + block of the fired flags. Warp i updates word i's; warp w
+    // sums the input of neuron w of every word.
+    const int words = blockIdx.x < W ? (int)((W - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
     const int64_t word = (int64_t)warp * gridDim.x + blockIdx.x;
-    const bool owner = word < a.W;
+    const bool owner = warp < words;
     const int64_t j = word * 32 + lane;
     const bool mine = owner && j < a.N;
     const ClassParams *c = a.ctab;
     float4 st = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float scale_down = 0.0f;
-    int pop = -1, fires = 0;
+    float scale_down = 0.0f, vt = 0.0f, vt_alt = 0.0f;
+    int pop = -1, fires = 0, kind = BSIM_NEURON_LIF;
+    LifConst lif{};
     if (mine) {
         c += a.cls[j];
         st = a.state[j];
         scale_down = __ldg(&c->scale_down);
         pop = __ldg(&c->pop);
+        kind = __ldg(&c->kind);
+        lif = lif_const(c);
+        vt = a.vtmp[j];
+        if (a.drive_half > 0) vt_alt = a.vtmp_alt[j];
+        const int64_t i = (int64_t)(t & 1ull) * a.N + j;  // cycle t's input
+        if (ACC == BSIM_ACC_EXACT) {
+            longlong2 *q = reinterpret_cast<longlong2 *>(a.acc) + i;
+            s_in[0][threadIdx.x] = *q;
+            if (a.acc_clear) *q = make_longlong2(0, 0);  // as step_kernel leaves it
+        } else {
+            reinterpret_cast<float2 *>(s_in[0])[threadIdx.x] = reinterpret_cast<const float2 *>(a.acc)[i];
+        }
     }
     if (threadIdx.x == 0) s_err = false;
-    for (int64_t i = threadIdx.x; i < (int64_t)a.R * a.W; i += PULL_LOOP_THREADS) s_bm[i] = a.bitmap[i];
+    for (int64_t i = threadIdx.x; i < (int64_t)R * W; i += PULL_LOOP_THREADS) s_bm[i] = __ldcg(&a.bitmap[i]);
+    // the rows, lane i holding the bounds of the warp's i-th; the first ones stay in shared memory as
+    // {source, delay - 1, weight} as far as there is room
+    int64_t row0 = 0, row_at = 0;
+    long long row_len = 0;
+    float row_scale = 0.0f;
+    {
+        const int64_t tgt = ((int64_t)lane * gridDim.x + blockIdx.x) * 32 + warp;
+        if (lane < words && tgt < a.N) {
+            row0 = a.col_off[tgt];
+            row_len = a.col_off[tgt + 1] - row0;
+            if (ACC == BSIM_ACC_EXACT) row_scale = __ldg(&a.ctab[a.cls[tgt]].scale_up);
+        }
+        row_at = row_len;
+        for (int o = 1; o < PULL_LOOP_WORDS; o <<= 1) {
+            const long long v = __shfl_up_sync(0xffffffffu, (long long)row_at, o);
+            if (lane >= o) row_at += v;
+        }
+        row_at -= row_len;
+    }
+    const unsigned held = __ballot_sync(0xffffffffu, steps >= PULL_LOOP_HOLD && row_at + row_len <= room);
+    for (int i = 0; i < words; i++)
+        if ((held >> i) & 1u) {
+            const int64_t c0 = __shfl_sync(0xffffffffu, (long long)row0, i);
+            const int64_t c1 = c0 + __shfl_sync(0xffffffffu, row_len, i);
+            uint2 *to = rows + (int)__shfl_sync(0xffffffffu, (int)row_at, i);
+            pull_entries(a, c0, c1, [](uint32_t src, int d) { return src | (unsigned)(d - 1) << 16; },
+                         [&](unsigned sd, float w, int64_t k) {
+                             if (k + lane < c1) to[k + lane - c0] = make_uint2(sd, __float_as_uint(w));
+                         });
+        }
     unsigned long long ev = 0;
+    int cur = (int)(t % (unsigned long long)R);  // ring slot of cycle t
+    bool have = true;                            // cycle t's input is in s_in[0] already
     LoopBar bar = loop_bar_begin(a);
     LoopRec rec = loop_record_begin(a, t);
     bool stop = false;
-    for (int k = 0; k < steps && !stop; k++) {
-        const int p = (int)(t & 1ull);
-        const int cur = (int)(t % (unsigned long long)a.R);
-        if (blockIdx.x == 0 && warp == PULL_LOOP_WARPS - 1) loop_clear_counts(a, t + 1, cur + 1 < a.R ? cur + 1 : 0, 1);
-        if (owner) {
-            bool fired = false;
-            if (mine) {
-                float inE, inI;
-                if (ACC == BSIM_ACC_EXACT) {
-                    longlong2 *q = reinterpret_cast<longlong2 *>(a.acc) + (int64_t)p * a.N + j;
-                    const longlong2 in = __ldcg(q);
-                    if (a.acc_clear) __stcg(q, make_longlong2(0, 0));  // as step_kernel leaves it
-                    inE = __fmul_rn(__ll2float_rn(in.x), scale_down);
-                    inI = __fmul_rn(__ll2float_rn(in.y), scale_down);
-                } else {
-                    const float2 in = __ldcg(reinterpret_cast<const float2 *>(a.acc) + (int64_t)p * a.N + j);
-                    inE = in.x;
-                    inI = in.y;
+    for (int k = 0; k < steps && !stop;) {
+        // the last interval has one cycle: the input of the cycle after the launch is then at hand
+        const int m = steps - k == 1 || (k == 0 && (steps & 1) == 0) ? 1 : LOOP_CYCLES;
+        const int cur1 = cur + 1 < R ? cur + 1 : 0, prev = cur > 0 ? cur - 1 : R - 1;
+        __syncthreads();
+        // ---- the inputs: cycle t's from the spikes up to t - 2, cycle t + 1's from those up to t - 1
+        const int d1 = (long long)t < D ? (int)t : D;  // cycles before the first fired nothing
+        const int d0 = have ? 0 : (long long)t - 1 < D ? (int)t - 1 : D;
+        for (int i = 0; i < words; i++) {
+            const float sc = ACC == BSIM_ACC_EXACT ? __shfl_sync(0xffffffffu, row_scale, i) : 0.0f;
+            PullSum<ACC> x0, x1;
+            int n = 0;
+            auto test = [&](uint32_t src, int d) {
+                return pull_fired(s_bm, W, R, cur, d1, src, d) | pull_fired(s_bm, W, R, prev, d0, src, d) << 1;
+            };
+            auto add = [&](unsigned act, float w, int64_t) {
+                n += x1.add(act & 1u, w, sc);
+                if (!have) n += x0.add(act >> 1, w, sc);
+            };
+            if ((held >> i) & 1u) {
+                const int len = (int)__shfl_sync(0xffffffffu, row_len, i);
+                const uint2 *row = rows + (int)__shfl_sync(0xffffffffu, (int)row_at, i);
+                for (int e0 = 0; e0 < len; e0 += 32) {
+                    const uint2 v = e0 + lane < len ? row[e0 + lane] : make_uint2(0u, 0u);
+                    const int d = e0 + lane < len ? (int)(v.x >> 16) + 1 : PULL_NO_DELAY;
+                    add(test(v.x & 0xffffu, d), __uint_as_float(v.y), 0);
                 }
-                neuron_update(a, c, j, (int)t, drive_vtmp(a, t), inE, inI, st, fired);
-                if (a.trace) trace_neuron(a, trace_row(a, t), j, st, inE, inI);
-                fires += fired;
+            } else {
+                const int64_t c0 = __shfl_sync(0xffffffffu, (long long)row0, i);
+                pull_entries(a, c0, c0 + __shfl_sync(0xffffffffu, row_len, i), test, add);
             }
-            const unsigned mask = __ballot_sync(0xffffffffu, fired);
-            if (lane == 0) a.bitmap[(int64_t)cur * a.W + word] = mask;
-            loop_append(a, t, cur, mask, loop_reserve(a, cur, mask), j, pop);
-        }
-        if (k > 0) {  // the previous cycle's fired flags
-            const int prev = cur > 0 ? cur - 1 : a.R - 1;
-            for (int64_t i = threadIdx.x; i < a.W; i += PULL_LOOP_THREADS)
-                s_bm[(int64_t)prev * a.W + i] = __ldcg(&a.bitmap[(int64_t)prev * a.W + i]);
+            ev += n;
+            x1.store(s_in[1], i * 32 + warp);
+            if (!have) x0.store(s_in[0], i * 32 + warp);
         }
         __syncthreads();
-        ev += pull_phase<ACC>(a, t, p ^ 1, s_bm, (long long)warp * gridDim.x + blockIdx.x,
-                              (long long)PULL_LOOP_WARPS * gridDim.x);
+        // ---- the updates of cycles t .. t+m-1
+        if (owner) {
+            unsigned mask[LOOP_CYCLES];
+            int place[LOOP_CYCLES];
+#pragma unroll
+            for (int i = 0; i < LOOP_CYCLES; i++) {
+                bool fired = false;
+                if (mine && i < m) {
+                    float inE, inI;
+                    if (ACC == BSIM_ACC_EXACT) {
+                        const longlong2 in = s_in[i][threadIdx.x];
+                        inE = __fmul_rn(__ll2float_rn(in.x), scale_down);
+                        inI = __fmul_rn(__ll2float_rn(in.y), scale_down);
+                    } else {
+                        const float2 in = reinterpret_cast<const float2 *>(s_in[i])[threadIdx.x];
+                        inE = in.x;
+                        inI = in.y;
+                    }
+                    if (kind == BSIM_NEURON_LIF) {
+                        const bool alt = a.drive_half > 0 && (((t + i) / (unsigned long long)a.drive_half) & 1ull);
+                        lif_update(lif, alt ? vt_alt : vt, inE, inI, st, fired);
+                    } else {
+                        drive_update(kind, (int)(t + i), st, fired, [&](int fc) { return poisson_gap(a, c, j, st, fc); });
+                    }
+                    if (a.trace) trace_neuron(a, trace_row(a, t + i), j, st, inE, inI);
+                    fires += fired;
+                }
+                mask[i] = __ballot_sync(0xffffffffu, fired);
+                place[i] = i < m ? loop_reserve(a, i == 0 ? cur : cur1, mask[i]) : 0;
+            }
+            if (mine && m == 1) {  // the next cycle's input
+                if (k + 1 < steps) {
+                    if (ACC == BSIM_ACC_EXACT) s_in[0][threadIdx.x] = s_in[1][threadIdx.x];
+                    else
+                        reinterpret_cast<float2 *>(s_in[0])[threadIdx.x] =
+                            reinterpret_cast<const float2 *>(s_in[1])[threadIdx.x];
+                } else {
+                    const int64_t i = (int64_t)((t & 1ull) ^ 1ull) * a.N + j;
+                    if (ACC == BSIM_ACC_EXACT) reinterpret_cast<longlong2 *>(a.acc)[i] = s_in[1][threadIdx.x];
+                    else
+                        reinterpret_cast<float2 *>(a.acc)[i] = reinterpret_cast<const float2 *>(s_in[1])[threadIdx.x];
+                }
+            }
+            for (int i = 0; i < m; i++) {
+                const unsigned mk = i == 0 ? mask[0] : mask[1];
+                const int rs = i == 0 ? cur : cur1;
+                if (lane == 0) a.bitmap[(int64_t)rs * W + word] = mk;
+                loop_append(a, t + i, rs, mk, i == 0 ? place[0] : place[1], j, pop);
+            }
+        }
+        if (blockIdx.x == 0 && warp == PULL_LOOP_WARPS - 1) loop_clear_counts(a, t + m, (cur + m) % R, LOOP_CYCLES);
         stop = loop_barrier(a, bar, &s_err, &s_stop, [] {});
-        if (rec.on) loop_record(a, rec, t, t + 1, cur);
-        t++;
+        for (int i = 0; i < m; i++) {  // their fired flags
+            const int64_t at = (int64_t)(i == 0 ? cur : cur1) * W;
+            for (int x = threadIdx.x; x < W; x += PULL_LOOP_THREADS) s_bm[at + x] = __ldcg(&a.bitmap[at + x]);
+        }
+        if (rec.on) loop_record(a, rec, t, t + m, cur);
+        have = m == 1;
+        t += m;
+        k += m;
+        cur = (cur + m) % R;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.step_ctr = t;
     if (mine) {
         a.state[j] = st;
         if (fires) a.fire_count[j] += fires;
     }
-    if (ev) atomicAdd(a.events, ev);
+    if (lane == 0 && ev) atomicAdd(a.events, ev);
+}
+
+// Before the first of these launches: step_kernel cleared cycle t's counters only.
+__global__ void loop_clear_kernel(const __grid_constant__ StepArgs a)
+{
+    if (*reinterpret_cast<volatile int32_t *>(a.err) != 0) return;
+    const unsigned long long t = *a.step_ctr;
+    loop_clear_counts(a, t + 1, (int)((t + 1) % (unsigned long long)a.R), 1);
 }
 
 // From step_kernel's input accumulators to the ring of push_loop_kernel: the input of the next
@@ -1872,15 +2048,14 @@ int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
     if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
     if (o.accumulate != BSIM_ACC_ORDERED && (o.delivery == BSIM_DELIVERY_PUSH || o.delivery == BSIM_DELIVERY_TILE))
         return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
-    const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + 2) * W;
-    return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps <= LOOP_MAX_SMEM ? 2 : 0;
+    const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + LOOP_EXTRA_SLOTS) * W;
+    return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps + 8 <= PULL_LOOP_SMEM ? 2 : 0;
 }
 
 cudaError_t launch_loop(Engine &e, int steps)
 {
-    void *args[] = {&e.a, &steps};
-    if (e.loop == 1)
-    {
+    if (e.loop == 1) {
+        void *args[] = {&e.a, &steps};
         const cudaError_t st = cudaFuncSetAttribute((const void *)push_loop_kernel,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOOP_MAX_SMEM);
         if (st != cudaSuccess) return st;
@@ -1889,14 +2064,21 @@ cudaError_t launch_loop(Engine &e, int steps)
     }
     const void *f = e.opt.accumulate == BSIM_ACC_ORDERED ? (const void *)pull_loop_kernel<BSIM_ACC_ORDERED>
                                                          : (const void *)pull_loop_kernel<BSIM_ACC_EXACT>;
-    const cudaError_t st = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOOP_MAX_SMEM);
+    const cudaError_t st = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PULL_LOOP_SMEM);
     if (st != cudaSuccess) return st;
-    return cudaLaunchCooperativeKernel(f, dim3(e.sm_count), dim3(PULL_LOOP_THREADS), args,
-                                       sizeof(uint32_t) * (size_t)e.a.R * e.a.W, e.stream);
+    const size_t flags = (sizeof(uint32_t) * (size_t)e.a.R * e.a.W + 7) / 8 * 8;
+    // a held entry has 16 bits for its source
+    int room = e.N <= 65536 ? (int)((PULL_LOOP_SMEM - flags) / (PULL_LOOP_WARPS * sizeof(uint2))) : 0;
+    void *args[] = {&e.a, &steps, &room};
+    return cudaLaunchCooperativeKernel(f, dim3(e.sm_count), dim3(PULL_LOOP_THREADS), args, PULL_LOOP_SMEM, e.stream);
 }
 
 cudaError_t launch_loop_enter(Engine &e)
 {
+    if (e.loop == 2) {
+        loop_clear_kernel<<<1, 32, 0, e.stream>>>(e.a);
+        return cudaGetLastError();
+    }
     cudaError_t st = cudaMemsetAsync(e.a.acc_ring, 0, sizeof(longlong2) * (size_t)e.a.acc_R * e.N, e.stream);
     if (st == cudaSuccess)
         st = cudaMemsetAsync(e.a.loop_ev, 0, sizeof(unsigned long long) * e.a.acc_R, e.stream);

@@ -102,3 +102,26 @@ def test_trace_and_statistics_equal_one_launch_per_cycle(ordered):
     assert all(np.array_equal(ta[k], tb[k]) for k in ta) and ta["v"].shape == (40, 900)
     assert np.array_equal(ca, cb) and ca.sum() > 0 and ea == eb
     assert all(np.array_equal(sa[k], sb[k]) for k in sa)
+
+
+@pytest.mark.parametrize("ordered", [False, True])
+@pytest.mark.parametrize("n,D,degree", [(33, 3, 3000), (9473, 2, 700), (1500, 40, 40), (150, 1, 5)])
+def test_rows_held_in_part_or_not_at_all(n, D, degree, ordered):
+    """Pull: rows that stay in shared memory, that do in part, and that are too long; launches of one,
+    two, an even and an odd number of cycles."""
+    net = network(n, D, degree, seed=n)
+    net[3][:] *= np.float32(20.0 / degree)
+    out = []
+    for gs in (0, 64):
+        o = B.options(graph_steps=gs, delivery=B.DELIVERY_PULL,
+                      accumulate=B.ACC_ORDERED if ordered else B.ACC_EXACT)
+        eng = B.Engine.from_arrays(*net, DT, opts=o)
+        eng.record(60, n * 60)
+        for k in (1, 2, 3, 4, 1, 30, 19):
+            eng.run(k)
+        out.append((eng.raster(), eng.state(), eng.fire_count(), eng.info().events_total))
+        eng.close()
+    (ra, sa, fa, ea), (rb, sb, fb, eb) = out
+    assert fa.sum() > 0 and ea == eb and np.array_equal(fa, fb)
+    assert all(np.array_equal(x, y) for x, y in zip(ra, rb))
+    assert all(np.array_equal(sa[k], sb[k]) for k in sa)
