@@ -1110,19 +1110,6 @@ static __device__ __forceinline__ void predict_phase(const StepArgs &a, unsigned
     }
 }
 
-// Spikes of the cycles a step delivers (t-1 .. t-D), from the ring counts; every
-// lane of the calling warp gets the sum.
-static __device__ __forceinline__ float window_spikes(const StepArgs &a, unsigned long long t)
-{
-    const int lane = threadIdx.x & 31;
-    float c = 0.0f;
-    for (int d = 1 + lane; d <= a.D; d += 32)
-        if ((long long)t - d >= 0) c += (float)a.ring_cnt[(t - d) % (unsigned long long)a.R];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    return c;
-}
-
 // The delivery mode of cycle t under BSIM_DELIVERY_AUTO: the cost model of each
 // mode (fixed ns per cycle + ns per event) on the cycle's work.
 //  * exact schedule (no predictor attached): the work is the exact spike count of
@@ -1132,16 +1119,16 @@ static __device__ __forceinline__ float window_spikes(const StepArgs &a, unsigne
 //    times the mean out-degree, or the exact count of cycle t-1 when the prediction
 //    for that cycle missed by more than the tolerance (the fallback).
 // Every block computes the same choice from the same device words.
-static __device__ __forceinline__ int auto_delivery(const StepArgs &a, unsigned long long t)
+static __device__ __forceinline__ int auto_delivery(const StepArgs &a, unsigned long long t, float window_spikes)
 {
     if (!a.mlp) {
-        const float work = window_spikes(a, t) * a.mean_outdeg / (float)a.D;
+        const float work = window_spikes * a.mean_outdeg / (float)a.D;
         const int dm = (a.n_tiles > 0 && a.cost_tile_a + a.cost_tile_b * work < a.cost_push_a + a.cost_push_b * work)
                            ? BSIM_DELIVERY_TILE
                            : BSIM_DELIVERY_PUSH;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
-            a.pstats->cycles += 1;
-            a.pstats->tile_cycles += dm == BSIM_DELIVERY_TILE ? 1 : 0;
+            atomicAdd(&a.pstats->cycles, 1ull);  // (not waited for, as a read and a write would be)
+            if (dm == BSIM_DELIVERY_TILE) atomicAdd(&a.pstats->tile_cycles, 1ull);
         }
         return dm;
     }
@@ -1231,13 +1218,16 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     // of the GPU reads them)
     if (threadIdx.x < 32) {
         int dm = a.deliv_sel ? *a.deliv_sel : a.delivery;
-        if (dm == BSIM_DELIVERY_AUTO) dm = a.pstats ? auto_delivery(a, t) : BSIM_DELIVERY_PUSH;
-        else if (dm == BSIM_DELIVERY_PUSH && a.tile_events > 0.0f)
-            dm = window_spikes(a, t) * a.mean_outdeg > a.tile_events * (float)a.D ? BSIM_DELIVERY_TILE : BSIM_DELIVERY_PUSH;
+        if (ACC != BSIM_ACC_ORDERED && (dm == BSIM_DELIVERY_PUSH || dm == BSIM_DELIVERY_AUTO)) {
+            // the window's counts are read once: for the push walk and for the choice
+            delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
+            __syncwarp();
+            const float spikes = (float)s_cum[a.D];
+            if (dm == BSIM_DELIVERY_AUTO) dm = a.pstats ? auto_delivery(a, t, spikes) : BSIM_DELIVERY_PUSH;
+            else if (a.tile_events > 0.0f && spikes * a.mean_outdeg > a.tile_events * (float)a.D) dm = BSIM_DELIVERY_TILE;
+        }
         if (dm == BSIM_DELIVERY_TILE && a.n_tiles == 0) dm = BSIM_DELIVERY_PUSH;
         if (threadIdx.x == 0) s_dm = dm;
-        if (ACC != BSIM_ACC_ORDERED && dm == BSIM_DELIVERY_PUSH)
-            delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
     }
     if (a.mlp && blockIdx.x == 0 && threadIdx.x == 32) {
         // slot t+2 is next written by cycle t+1's prediction
