@@ -243,6 +243,7 @@ class Engine:
     def __init__(self, handle):
         self._h = handle
         self._rec_steps = None  # steps of the current recording (sizes the offsets read back)
+        self._neurons = None
 
     @classmethod
     def from_arrays(cls, params, src, dst, weight, delay_steps, dt, pop=None, instance=None, opts=None,
@@ -333,8 +334,14 @@ class Engine:
                                      _p(out["in_I"]), ctypes.byref(ns)))
         return {k: v[:ns.value] for k, v in out.items()}
 
+    def _n(self):
+        """Neurons of the engine (asked of the library once)."""
+        if self._neurons is None:
+            self._neurons = self.info().n_neurons
+        return self._neurons
+
     def state(self):
-        n = self.info().n_neurons
+        n = self._n()
         v = np.zeros(n, np.float32)
         ie = np.zeros(n, np.float32)
         ii = np.zeros(n, np.float32)
@@ -393,7 +400,7 @@ class Engine:
     def fire_count(self, out=None):
         """Spikes per neuron since creation; into `out` (a C-contiguous int32 array of
         n_neurons, e.g. in page-locked memory, reused across reads) when given."""
-        n = self.info().n_neurons
+        n = self._n()
         if (out is not None and out.dtype == np.int32 and out.ndim == 1 and out.flags.c_contiguous
                 and out.shape[0] == n):
             c = out

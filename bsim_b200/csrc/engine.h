@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -200,6 +201,12 @@ struct Engine {
     // staging for state uploads and read-backs: four planes of N words (v, i_E,
     // i_I, refrac), so the host's arrays move with one copy each, no host repacking
     float *stage = nullptr;
+    // page-locked (ensure_host): the error flag as the last synchronisation saw it and, for small
+    // engines, five planes of N words for the state's fields and the spike counts (a copy into the
+    // caller's pageable memory waits for each piece by itself)
+    std::once_flag host_once;
+    int32_t *h_err = nullptr;
+    float *h_stage = nullptr;
     // schedule state: predictor statistics and the MLP's parameters (a.pstats / a.mlp
     // point here while a schedule / a predictor is attached)
     PredStats *pstats_mem = nullptr;
