@@ -1746,9 +1746,9 @@ int bsim_run_async(bsim_engine *eh, int64_t steps)
     int64_t left = steps;
     const int gl = e.opt.graph_steps;
     const bool ordered = e.opt.accumulate == BSIM_ACC_ORDERED;
-    const bool same_mode = e.loop == 1 ? e.a.delivery == BSIM_DELIVERY_PUSH || e.a.delivery == BSIM_DELIVERY_TILE
+    const bool same_mode = e.loop == 1 ? e.a.delivery != BSIM_DELIVERY_PULL
                                        : e.loop == 2 && (ordered || e.a.delivery == BSIM_DELIVERY_PULL);
-    if (left > 0 && gl > 0 && same_mode && !e.a.mlp && !e.a.pstats) {
+    if (left > 0 && gl > 0 && same_mode && !e.a.mlp && (!e.a.pstats || e.a.delivery == BSIM_DELIVERY_AUTO)) {
         TRY(enter_loop(e));
         for (int k; left > 0; left -= k) {  // bounded, so that a launch ends within a second
             k = (int)std::min<int64_t>(left, LOOP_STEPS);

@@ -1110,6 +1110,13 @@ static __device__ __forceinline__ void predict_phase(const StepArgs &a, unsigned
     }
 }
 
+// The exact schedule's choice for a cycle that delivers `window_spikes` spikes.
+static __device__ __forceinline__ bool exact_tiled(const StepArgs &a, float window_spikes)
+{
+    const float work = window_spikes * a.mean_outdeg / (float)a.D;
+    return a.n_tiles > 0 && a.cost_tile_a + a.cost_tile_b * work < a.cost_push_a + a.cost_push_b * work;
+}
+
 // The delivery mode of cycle t under BSIM_DELIVERY_AUTO: the cost model of each
 // mode (fixed ns per cycle + ns per event) on the cycle's work.
 //  * exact schedule (no predictor attached): the work is the exact spike count of
@@ -1122,10 +1129,7 @@ static __device__ __forceinline__ void predict_phase(const StepArgs &a, unsigned
 static __device__ __forceinline__ int auto_delivery(const StepArgs &a, unsigned long long t, float window_spikes)
 {
     if (!a.mlp) {
-        const float work = window_spikes * a.mean_outdeg / (float)a.D;
-        const int dm = (a.n_tiles > 0 && a.cost_tile_a + a.cost_tile_b * work < a.cost_push_a + a.cost_push_b * work)
-                           ? BSIM_DELIVERY_TILE
-                           : BSIM_DELIVERY_PUSH;
+        const int dm = exact_tiled(a, window_spikes) ? BSIM_DELIVERY_TILE : BSIM_DELIVERY_PUSH;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             atomicAdd(&a.pstats->cycles, 1ull);  // (not waited for, as a read and a write would be)
             if (dm == BSIM_DELIVERY_TILE) atomicAdd(&a.pstats->tile_cycles, 1ull);
@@ -1563,6 +1567,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
     }
     __syncthreads();
     unsigned long long ev = 0;  // thread 0: events delivered
+    // the exact schedule's choices, as step_kernel counts them
+    const bool choices = a.pstats && blockIdx.x == 0 && warp == LOOP_WARPS - 2;
+    unsigned long long tile_choices = 0;
+    const unsigned long long t_first = t;
     int slot = (int)(t % (unsigned long long)Ra);         // accumulator slot of cycle t
     int rslot = (int)(t % (unsigned long long)a.R);       // ring slot of cycle t
     LoopBar bar = loop_bar_begin(a);
@@ -1698,6 +1706,16 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
                 s_ev[sl] = 0ull;
             }
         }
+        if (choices)
+            for (int i = 0; i < m; i++) {
+                int n_spikes = 0;  // delivered in cycle t + i
+                for (int d = 1 + lane; d <= D; d += 32) {
+                    const int sl = rslot + i - d;
+                    if ((long long)t + i - d >= 0) n_spikes += __ldcg(&a.ring_cnt[sl < 0 ? sl + a.R : sl < a.R ? sl : sl - a.R]);
+                }
+                n_spikes = __reduce_add_sync(0xffffffffu, n_spikes);
+                tile_choices += exact_tiled(a, (float)n_spikes);
+            }
         if (rec.on) loop_record(a, rec, t, t + m, rslot);
         t += m;
         k += m;
@@ -1706,6 +1724,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
         __syncthreads();
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.step_ctr = t;
+    if (choices && lane == 0) {
+        atomicAdd(&a.pstats->cycles, t - t_first);
+        atomicAdd(&a.pstats->tile_cycles, tile_choices);
+    }
     if (threadIdx.x < Ra && s_ev[threadIdx.x]) atomicAdd(&a.loop_ev[threadIdx.x], s_ev[threadIdx.x]);  // still in flight
     if (mine) {
         a.state[j] = st;
@@ -2030,13 +2052,14 @@ cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream
 // Whether an engine of these sizes can run many cycles per launch (0: no, 1: push form, 2: pull
 // form): half of a block's warps own neurons at most. An engine asked to deliver tiled takes the push
 // form too: the spikes are the same, and at these sizes a tiled cycle is a launch and a chain of
-// dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.3). AUTO delivery and longer delays
-// take one launch per cycle.
+// dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.3), and so does an AUTO engine
+// until a predictor is attached (38 x 874 neurons, 1-step delays: 13.0 us against 5.5): the choices of
+// the exact schedule are counted, the delivery is the push form's. Longer delays take one launch per cycle.
 int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
 {
     const int64_t W = (N + 31) / 32;
     if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
-    if (o.accumulate != BSIM_ACC_ORDERED && (o.delivery == BSIM_DELIVERY_PUSH || o.delivery == BSIM_DELIVERY_TILE))
+    if (o.accumulate != BSIM_ACC_ORDERED && o.delivery != BSIM_DELIVERY_PULL)
         return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
     const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + LOOP_EXTRA_SLOTS) * W;
     return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps + 8 <= PULL_LOOP_SMEM ? 2 : 0;

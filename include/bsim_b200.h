@@ -301,7 +301,8 @@ int bsim_set_predictor(bsim_engine *e, const float *params, float tolerance, con
 typedef struct bsim_pred_stats {
     int64_t cycles;          /* cycles scheduled by the predictor */
     int64_t fallbacks;       /* cycles whose choice was recomputed from exact counts */
-    int64_t tile_cycles;     /* cycles delivered with the tiled mode */
+    int64_t tile_cycles;     /* cycles for which the schedule chose the tiled mode (small engines, which run
+                                many cycles per launch, count the choice and deliver in their own form) */
     double abs_err_sum;      /* sum over cycles and populations of |predicted - actual| spikes */
     double actual_sum;       /* sum of actual spikes over the same cycles and populations */
 } bsim_pred_stats;

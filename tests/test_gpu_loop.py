@@ -125,3 +125,22 @@ def test_rows_held_in_part_or_not_at_all(n, D, degree, ordered):
     assert fa.sum() > 0 and ea == eb and np.array_equal(fa, fb)
     assert all(np.array_equal(x, y) for x, y in zip(ra, rb))
     assert all(np.array_equal(sa[k], sb[k]) for k in sa)
+
+
+@pytest.mark.parametrize("D", [1, 6, 40])
+def test_auto_schedule_counts_its_choices(D):
+    """Small AUTO engines under the exact schedule: the spikes, events and statistics of one launch per
+    cycle, with a choice that changes along the run."""
+    net = network(1500, D, 30, seed=D, burst=True)
+    out = []
+    for gs in (0, 64):
+        eng = B.Engine.from_arrays(*net, DT, opts=B.options(graph_steps=gs, delivery=B.DELIVERY_AUTO))
+        eng.set_predictor(None, 0.25, (10.0, 6.5), (10000.0, 3.0))
+        for k in (1, 2, 40, 7, 50):
+            eng.run(k)
+        out.append((eng.fire_count(), eng.state(), eng.info().events_total, eng.predictor_stats()))
+        eng.close()
+    (fa, sa, ea, pa), (fb, sb, eb, pb) = out
+    assert fa.sum() > 0 and ea == eb and np.array_equal(fa, fb)
+    assert all(np.array_equal(sa[k], sb[k]) for k in sa)
+    assert pa.cycles == pb.cycles == 100 and pa.tile_cycles == pb.tile_cycles and 0 < pa.tile_cycles < 100
