@@ -615,7 +615,7 @@ static bool wants_tiles(const bsim_options &o, int32_t D)
 // 4.8e8 with 50-step delays 3,040 / 1,280), so cycles above TILE_MIN_EVENTS. Tiled shares follow the
 // previous cycle, most of whose spikes are delivered again with another delay: delays of at least 4
 // steps. Only for generated networks (the copy is made on the GPU, in about the time of the rows) and
-// where half of the device's memory stays free; build_tiles = -1 keeps the rows alone.
+// where a quarter of the device's memory stays free; build_tiles = -1 keeps the rows alone.
 #define TILE_MIN_EVENTS 7.0e6f
 static bool push_holds_tiles(const Engine &e)
 {
@@ -624,7 +624,7 @@ static bool push_holds_tiles(const Engine &e)
         return false;
     size_t free = 0, total = 0;
     if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
-    return (double)free - (18.0 * (double)e.S + 24.0 * (double)e.N * e.D) > 0.5 * (double)total;
+    return (double)free - (18.0 * (double)e.S + 24.0 * (double)e.N * e.D) > 0.25 * (double)total;
 }
 
 // Host-side description of the tiled copy.
