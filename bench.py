@@ -34,11 +34,10 @@ HBM_FALLBACK_GBS = 6650.0
 BYTES_PER_NEURON_STEP = 52.0   # read/write v, i_E, i_I, refrac (32), v_tmp (4), read+clear E/I input (16)
 BYTES_PER_EVENT = 8.0          # int32 target + fp32 weight of one delivered synapse
 BYTES_PER_SPIKE = 8.0          # fired id written once, read once
-# Delivery mode per workload when --delivery is not given: the fastest measured on
-# a B200 (1e6-neuron network at ~545 Hz: tiled 0.223 ms per cycle, push ~0.44 ms).
-# fastest measured delivery per workload (steady state): tiled on the 1e6-neuron network
-# (-51 % against push); on the dense one tiled and push are level (2.95-3.11 ms against
-# 3.03-3.08 ms per cycle over several boxes), and push varies less
+# Delivery mode per workload when --delivery is not given: the fastest measured on a B200 in the
+# steady state. Tiled on the 1e6-neuron network (0.164 ms per cycle; rows alone 0.43 ms); elsewhere push,
+# whose engine delivers the busy cycles of a network of this size from a tiled copy too (dense: 1.31 ms
+# per cycle, rows alone 3.04 ms).
 DEFAULT_DELIVERY = {"plain_1m": "tile"}
 
 
@@ -449,7 +448,10 @@ def predicted_vs_plain(steps, device, settle=1000, chunk=50):
     t_train = time.perf_counter() - t_train
 
     def run_mode(deliv, setup=None):
-        eng = B.Engine.generated(specs, DT, opts=B.options(device=device, delivery=deliv, graph_steps=chunk))
+        # (plain push is the rows alone: with the tiled copy beside them its busy cycles would be tiled)
+        bt = -1 if deliv == B.DELIVERY_PUSH else 0
+        eng = B.Engine.generated(specs, DT, opts=B.options(device=device, delivery=deliv, graph_steps=chunk,
+                                                           build_tiles=bt))
         if setup:
             setup(eng)
         eng.run(settle)

@@ -59,7 +59,8 @@ extern "C" {
                               reference's StaticSynapse::update loop (src/net/Network.cpp:320-325):
                               bit-identical to the reference CPU simulator. Pull delivery only. */
 
-#define BSIM_DELIVERY_PUSH 0 /* source-ordered rows, one warp per (spike, delay) segment */
+#define BSIM_DELIVERY_PUSH 0 /* source-ordered rows, one warp per (spike, delay) segment; large generated
+                                networks deliver their busy cycles tiled (build_tiles) */
 #define BSIM_DELIVERY_PULL 1 /* target-ordered rows scanned against per-step fired bitmaps */
 #define BSIM_DELIVERY_AUTO 2 /* per step, by the firing predictor (EXACT accumulation only) */
 #define BSIM_DELIVERY_TILE 3 /* target tiles summed in shared memory, sources filtered by their
@@ -72,7 +73,8 @@ typedef struct bsim_options {
     int32_t accumulate;    /* BSIM_ACC_* */
     int32_t delivery;      /* BSIM_DELIVERY_* */
     int32_t build_pull;    /* also build the target-ordered copy (forced on for PULL and ORDERED) */
-    int32_t graph_steps;   /* steps captured per CUDA graph by bsim_run (0: plain launches) */
+    int32_t graph_steps;   /* steps captured per CUDA graph by bsim_run; networks of a few ten thousand neurons run
+                              many steps per launch instead (0: one plain launch per step) */
     int32_t block_threads; /* threads per block of the step kernel (0: autotuned) */
     int32_t grid_blocks;   /* blocks of the step kernel (0: autotuned) */
     int32_t build_tiles;   /* 1: also build the target-tiled copy; 0: for TILE/AUTO, and for large generated
