@@ -1316,9 +1316,10 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 //     follows without a barrier and again two cycles are run between barriers: the input of
 //     cycle t takes the spikes up to t - 2, that of t + 1 those up to t - 1, and one scan of
 //     the rows tests both. The delay window's fired flags and the rows (8 bytes an entry,
-//     as far as they fit) stay in shared memory. 10 x 1,000 neurons, ORDERED: 11.6 -> 5.1
-//     us per cycle (9.2 with one cycle per barrier and the rows read from L2); 36 x 1,000
-//     31.9 -> 13.2; 12 x 3,000 at 2 kHz 107 -> 57. What is left of the first is the scan's
+//     as far as they fit) stay in shared memory. 10 x 1,000 neurons, ORDERED: 11.6 -> 4.4
+//     us per cycle (9.2 with one cycle per barrier and the rows read from L2, 5.1 with two
+//     separate looks at the flags per entry); 36 x 1,000 31.9 -> 11.1; 12 x 3,000 at 2 kHz
+//     107 -> 58. What is left of the first is the scan's
 //     instructions (110 entries a row, two tests each), the barrier and the flags' exchange.
 //
 // The fire ring, its counts and the fired flags are kept as step_kernel keeps them,
@@ -1742,11 +1743,12 @@ __global__ void __launch_bounds__(PULL_LOOP_THREADS, 1)
 {
     __shared__ bool s_stop, s_err;
     __shared__ longlong2 s_in[LOOP_CYCLES][PULL_LOOP_WORDS * 32];  // input of cycles t, t + 1 of this block's neurons
-    extern __shared__ __align__(16) unsigned long long s_dyn[];    // [R][W] the fired flags, then the warps' rows
-    uint32_t *s_bm = reinterpret_cast<uint32_t *>(s_dyn);
+    extern __shared__ __align__(16) unsigned long long s_dyn[];    // [1 + R][W] the fired flags, then the warps' rows
+    // slot -1 holds what slot R - 1 does, so the slot of the cycle before is always W words back
+    uint32_t *s_bm = reinterpret_cast<uint32_t *>(s_dyn) + a.W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int W = (int)a.W, R = a.R, D = a.D;
-    uint2 *rows = reinterpret_cast<uint2 *>(s_dyn + ((size_t)R * W + 1) / 2) + (size_t)warp * room;
+    uint2 *rows = reinterpret_cast<uint2 *>(s_dyn + ((size_t)(R + 1) * W + 1) / 2) + (size_t)warp * room;
     if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t *>(a.err) != 0)) return;
     unsigned long long t = *reinterpret_cast<volatile unsigned long long *>(a.step_ctr);
     // the block's neurons: words i * grid + block of the fired flags. Warp i updates word i's; warp w
@@ -1780,7 +1782,11 @@ __global__ void __launch_bounds__(PULL_LOOP_THREADS, 1)
         }
     }
     if (threadIdx.x == 0) s_err = false;
-    for (int64_t i = threadIdx.x; i < (int64_t)R * W; i += PULL_LOOP_THREADS) s_bm[i] = __ldcg(&a.bitmap[i]);
+    for (int64_t i = threadIdx.x; i < (int64_t)R * W; i += PULL_LOOP_THREADS) {
+        const uint32_t v = __ldcg(&a.bitmap[i]);
+        s_bm[i] = v;
+        if (i >= (int64_t)(R - 1) * W) s_bm[i - (int64_t)R * W] = v;
+    }
     // the rows, lane i holding the bounds of the warp's i-th; the first ones stay in shared memory as
     // {source, delay - 1, weight} as far as there is room
     int64_t row0 = 0, row_at = 0;
@@ -1820,19 +1826,22 @@ __global__ void __launch_bounds__(PULL_LOOP_THREADS, 1)
     for (int k = 0; k < steps && !stop;) {
         // the last interval has one cycle: the input of the cycle after the launch is then at hand
         const int m = steps - k == 1 || (k == 0 && (steps & 1) == 0) ? 1 : LOOP_CYCLES;
-        const int cur1 = cur + 1 < R ? cur + 1 : 0, prev = cur > 0 ? cur - 1 : R - 1;
+        const int cur1 = cur + 1 < R ? cur + 1 : 0;
         __syncthreads();
         // ---- the inputs: cycle t's from the spikes up to t - 2, cycle t + 1's from those up to t - 1
         const int d1 = (long long)t < D ? (int)t : D;  // cycles before the first fired nothing
-        const int d0 = have ? 0 : (long long)t - 1 < D ? (int)t - 1 : D;
         for (int i = 0; i < words; i++) {
             const float sc = ACC == BSIM_ACC_EXACT ? __shfl_sync(0xffffffffu, row_scale, i) : 0.0f;
             PullSum<ACC> x0, x1;
             int n = 0;
             auto test = [&](uint32_t src, int d) {
-                return pull_fired(s_bm, W, R, cur, d1, src, d) | pull_fired(s_bm, W, R, prev, d0, src, d) << 1;
+                if (d > d1) return 0u;
+                const uint32_t *f = s_bm + (cur >= d ? cur - d : cur - d + R) * W + (src >> 5);
+                // (d cycles before t - 1 may be cycle -1, whose flags are zero)
+                return ((f[0] >> (src & 31)) & 1u) | ((f[-W] >> (src & 31)) & 1u) << 1;
             };
             auto add = [&](unsigned act, float w, int64_t) {
+                if (!__any_sync(0xffffffffu, act)) return;
                 n += x1.add(act & 1u, w, sc);
                 if (!have) n += x0.add(act >> 1, w, sc);
             };
@@ -1907,7 +1916,12 @@ __global__ void __launch_bounds__(PULL_LOOP_THREADS, 1)
         stop = loop_barrier(a, bar, &s_err, &s_stop, [] {});
         for (int i = 0; i < m; i++) {  // their fired flags
             const int64_t at = (int64_t)(i == 0 ? cur : cur1) * W;
-            for (int x = threadIdx.x; x < W; x += PULL_LOOP_THREADS) s_bm[at + x] = __ldcg(&a.bitmap[at + x]);
+            const bool twice = at == (int64_t)(R - 1) * W;
+            for (int x = threadIdx.x; x < W; x += PULL_LOOP_THREADS) {
+                const uint32_t v = __ldcg(&a.bitmap[at + x]);
+                s_bm[at + x] = v;
+                if (twice) s_bm[x - W] = v;
+            }
         }
         if (rec.on) loop_record(a, rec, t, t + m, cur);
         have = m == 1;
@@ -2061,7 +2075,7 @@ int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
     if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
     if (o.accumulate != BSIM_ACC_ORDERED && o.delivery != BSIM_DELIVERY_PULL)
         return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
-    const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + LOOP_EXTRA_SLOTS) * W;
+    const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + LOOP_EXTRA_SLOTS + 1) * W;
     return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps + 8 <= PULL_LOOP_SMEM ? 2 : 0;
 }
 
@@ -2079,7 +2093,7 @@ cudaError_t launch_loop(Engine &e, int steps)
                                                          : (const void *)pull_loop_kernel<BSIM_ACC_EXACT>;
     const cudaError_t st = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PULL_LOOP_SMEM);
     if (st != cudaSuccess) return st;
-    const size_t flags = (sizeof(uint32_t) * (size_t)e.a.R * e.a.W + 7) / 8 * 8;
+    const size_t flags = (sizeof(uint32_t) * (size_t)(e.a.R + 1) * e.a.W + 7) / 8 * 8;
     // a held entry has 16 bits for its source
     int room = e.N <= 65536 ? (int)((PULL_LOOP_SMEM - flags) / (PULL_LOOP_WARPS * sizeof(uint2))) : 0;
     void *args[] = {&e.a, &steps, &room};
