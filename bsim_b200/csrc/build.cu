@@ -1797,7 +1797,9 @@ int bsim_stall_tile(bsim_engine *eh, int32_t tile)
 {
     if (!eh) return fail(BSIM_ERR_ARG, "null engine");
     Engine &e = *H(eh);
-    if (!e.a.tile_arrive || tile < 0 || tile >= e.a.n_tiles)
+    // a push engine that was not asked for a tiled copy has none to stall
+    if (!e.a.tile_arrive || (e.opt.delivery == BSIM_DELIVERY_PUSH && e.opt.build_tiles == 0) || tile < 0 ||
+        tile >= e.a.n_tiles)
         return fail(BSIM_ERR_ARG, "bsim_stall_tile: the engine has no such tile");
     CK(cudaSetDevice(e.device));
     TRY(leave_loop(e));  // the wait is in the cycle-by-cycle form: a small engine keeps to it from here on
