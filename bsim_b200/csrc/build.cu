@@ -2141,27 +2141,56 @@ __global__ void pop_in_from_counts_kernel(StepArgs a, const int32_t *indeg, doub
         atomicAdd(&in_sum[a.ctab[a.cls[j]].pop], (double)indeg[j]);
 }
 
+// Population of the target whose counter an entry of a tile of T targets names (E or I).
+static __device__ __forceinline__ int entry_pop(const StepArgs &a, uint2 e, int tb, int T)
+{
+    const int c = (int)(e.x >> 2);
+    return __ldg(&a.ctab[a.cls[tb + (c >= 2 * T ? c - 2 * T : c)]].pop);
+}
+
+// One block per tile: the entries of each (run, source) give the out-degree of the source and the
+// in-degrees of the tile's populations. Consecutive small populations share a tile, so in such a tile
+// every entry is looked at; one of a single population takes the segments' lengths alone.
 __global__ void pop_degree_tiles_kernel(StepArgs a, double *in_sum, double *out_sum, int want_in, int want_out)
 {
-    // one block per tile: entries per (run, source) give out-degree of the source and in-degree of the tile
     for (int q = blockIdx.x; q < a.n_tiles; q += gridDim.x) {
         const uint2 *ent = a.ent + 2 * a.tile_seg0[q];
+        const int tb = a.tile_beg[q], T = a.tile_beg[q + 1] - tb;
+        const int pop0 = a.ctab[a.cls[tb]].pop;
+        bool other = false;
+        for (int i = threadIdx.x; i < T; i += blockDim.x) other |= a.ctab[a.cls[tb + i]].pop != pop0;
+        const bool shared = __syncthreads_or(other) != 0;
         for (int r = a.tile_run_off[q]; r < a.tile_run_off[q + 1]; r++) {
             const int n_r = a.run_n[r], chunks = (n_r + 31) >> 5;
             const int units = (r + 1 < a.tile_run_off[q + 1] ? a.run_unit0[r + 1] : a.tile_units[q]) - a.run_unit0[r];
             const int D_r = units / chunks;
             for (int i = threadIdx.x; i < n_r; i += blockDim.x) {
                 int64_t real = 0;
+                int pop = pop0;
+                int64_t of_pop = 0;  // entries of `pop` not yet added
                 for (int d = 0; d < D_r; d++) {
                     const uint32_t *so = a.seg_off + a.run_seg0[r] + (int64_t)d * n_r + i;
                     const int64_t x1 = 2 * (int64_t)so[1];
                     const int64_t x0 = 2 * (int64_t)so[0];
-                    if (x1 > x0) real += x1 - x0 - (ent[x1 - 1].y == TILE_PAD_W ? 1 : 0);
+                    if (x1 <= x0) continue;
+                    const int64_t n = x1 - x0 - (ent[x1 - 1].y == TILE_PAD_W ? 1 : 0);
+                    real += n;
+                    if (!shared) {
+                        of_pop += n;
+                        continue;
+                    }
+                    for (int64_t x = x0; x < x0 + n; x++) {
+                        const int p = entry_pop(a, ent[x], tb, T);
+                        if (p != pop) {
+                            if (want_in && of_pop) atomicAdd(&in_sum[pop], (double)of_pop);
+                            pop = p;
+                            of_pop = 0;
+                        }
+                        of_pop++;
+                    }
                 }
-                const double c = (double)real;
-                const uint32_t src = a.run_src0[r] + i;
-                if (want_out) atomicAdd(&out_sum[a.ctab[a.cls[src]].pop], c);
-                if (want_in) atomicAdd(&in_sum[a.ctab[a.cls[a.tile_beg[q]]].pop], c);
+                if (want_in && of_pop) atomicAdd(&in_sum[pop], (double)of_pop);
+                if (want_out) atomicAdd(&out_sum[a.ctab[a.cls[a.run_src0[r] + i]].pop], (double)real);
             }
         }
     }
