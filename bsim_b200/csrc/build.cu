@@ -494,6 +494,7 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     a.step_ctr = d_ctr;
     a.events = d_ctr + 1;
     a.ticket = reinterpret_cast<unsigned int *>(d_ctr + 2);
+    a.tile_cycles = d_ctr + 3;
     a.loop_bar = d_ctr + 16;
     if (e.loop == 1) {
         a.acc_R = e.D + 3;
@@ -1738,6 +1739,15 @@ static int leave_loop(Engine &e)
     return BSIM_OK;
 }
 
+// The many-cycle form bsim_run takes now (0: one launch per cycle).
+static int loop_now(const Engine &e)
+{
+    const bool ordered = e.opt.accumulate == BSIM_ACC_ORDERED;
+    const bool same_mode = e.loop == 1 ? e.a.delivery != BSIM_DELIVERY_PULL
+                                       : e.loop == 2 && (ordered || e.a.delivery == BSIM_DELIVERY_PULL);
+    return e.opt.graph_steps > 0 && same_mode && !e.a.mlp && (!e.a.pstats || e.a.delivery == BSIM_DELIVERY_AUTO) ? e.loop : 0;
+}
+
 int bsim_run_async(bsim_engine *eh, int64_t steps)
 {
     if (!eh || steps < 0) return fail(BSIM_ERR_ARG, "bsim_run: invalid arguments");
@@ -1745,10 +1755,7 @@ int bsim_run_async(bsim_engine *eh, int64_t steps)
     CK(cudaSetDevice(e.device));
     int64_t left = steps;
     const int gl = e.opt.graph_steps;
-    const bool ordered = e.opt.accumulate == BSIM_ACC_ORDERED;
-    const bool same_mode = e.loop == 1 ? e.a.delivery != BSIM_DELIVERY_PULL
-                                       : e.loop == 2 && (ordered || e.a.delivery == BSIM_DELIVERY_PULL);
-    if (left > 0 && gl > 0 && same_mode && !e.a.mlp && (!e.a.pstats || e.a.delivery == BSIM_DELIVERY_AUTO)) {
+    if (left > 0 && loop_now(e)) {
         TRY(enter_loop(e));
         for (int k; left > 0; left -= k) {  // bounded, so that a launch ends within a second
             k = (int)std::min<int64_t>(left, LOOP_STEPS);
@@ -2490,7 +2497,7 @@ int bsim_get_info(bsim_engine *eh, bsim_info *info)
     info->n_instances = e.n_inst;
     info->n_classes = e.n_cls;
     info->n_pops = e.n_pops;
-    unsigned long long ctr[2];
+    unsigned long long ctr[4];  // cycle, events, ticket, tiled cycles
     CK(cudaMemcpy(ctr, e.a.step_ctr, sizeof(ctr), cudaMemcpyDeviceToHost));
     info->steps_done = (int64_t)ctr[0];
     info->events_total = ctr[1];
@@ -2500,6 +2507,8 @@ int bsim_get_info(bsim_engine *eh, bsim_info *info)
     info->accumulate = e.opt.accumulate;
     info->delivery = e.opt.delivery;
     info->sm_count = e.sm_count;
+    info->many_cycles = loop_now(e);
+    info->tile_cycles = (int64_t)ctr[3];
     return BSIM_OK;
 }
 

@@ -95,6 +95,7 @@ struct StepArgs {
     unsigned long long *step_ctr;  // current cycle t (device-side, advanced by the last block)
     unsigned int *ticket;          // end-of-step block counter
     unsigned long long *events;    // synaptic events delivered
+    unsigned long long *tile_cycles;  // cycles delivered from the tiled copy
     // many cycles per launch (small networks)
     unsigned long long *loop_bar;     // [2] barrier counters, 128 bytes apart (small networks only)
     void *acc_ring;                   // [acc_R][N] longlong2: input of cycle c in slot c mod acc_R (push form)

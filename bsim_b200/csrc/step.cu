@@ -1283,6 +1283,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
         for (int i = threadIdx.x; i < a.n_items; i += blockDim.x)
             a.item_clocks[(int64_t)((t + 1ull) & 1ull) * a.n_items + i] = 0u;
         if (threadIdx.x == 0) {
+            if (tiled) *a.tile_cycles += 1ull;
             // advance the cycle
             record_advance(a, t);
             *a.ticket = 0u;

@@ -118,7 +118,11 @@ typedef struct bsim_info {
     int32_t grid_blocks, block_threads;
     int32_t accumulate, delivery;
     int32_t sm_count;
-    int32_t reserved[7];
+    int32_t many_cycles;     /* how bsim_run advances the engine as it stands: 0 one launch per cycle, 1 many cycles
+                                per launch with the spikes pushed (whatever EXACT delivery was asked for), 2 many
+                                cycles per launch with the rows scanned (PULL, ORDERED) */
+    int64_t tile_cycles;     /* cycles delivered from the tiled copy so far */
+    int32_t reserved[4];
 } bsim_info;
 
 /* Fills *opt with defaults: EXACT accumulation, PUSH delivery, graphs of 64 steps. */
