@@ -62,7 +62,7 @@ class Info(ctypes.Structure):
                 ("device_bytes", ctypes.c_int64), ("grid_blocks", ctypes.c_int32),
                 ("block_threads", ctypes.c_int32), ("accumulate", ctypes.c_int32),
                 ("delivery", ctypes.c_int32), ("sm_count", ctypes.c_int32), ("many_cycles", ctypes.c_int32),
-                ("tile_cycles", ctypes.c_int64), ("reserved", ctypes.c_int32 * 4)]
+                ("tile_cycles", ctypes.c_int64), ("n_tiles", ctypes.c_int32), ("reserved", ctypes.c_int32 * 3)]
 
 
 EXPORTS = [

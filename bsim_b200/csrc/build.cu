@@ -513,9 +513,8 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     a.n_pops = e.n_pops;
     a.hist_len = 0;
     if (a.n_tiles > 0 && e.opt.delivery == BSIM_DELIVERY_TILE) a.delivery = BSIM_DELIVERY_TILE;
-    // every cycle of a tiled-only engine overwrites all planes of the parity it
-    // delivers into, so the LIF phase need not clear them; any other mode adds
-    a.mean_outdeg = e.N ? (float)((double)e.S / (double)e.N) : 0.0f;
+    // every cycle of a tiled-only engine overwrites the plane of the parity it
+    // delivers into, so the LIF phase need not clear it; any other mode adds
     a.acc_clear = a.delivery == BSIM_DELIVERY_TILE ? 0 : 1;
     // launch shape: all blocks resident (occupancy-sized grid), so the grid-stride
     // loops of both phases see every SM
@@ -609,23 +608,48 @@ static bool wants_tiles(const bsim_options &o, int32_t D)
            (o.build_tiles > 0 || o.delivery == BSIM_DELIVERY_TILE || o.delivery == BSIM_DELIVERY_AUTO);
 }
 
-// Push delivery of a large network holds the tiled copy too, and delivers its busy cycles from it: the
-// sums are the same, and one L2 reduction per event (~1.5e11/s) is what bounds a pushed cycle. The
-// line: a tiled cycle costs ~35 us + 2 to 3 ps per event, a pushed one ~10 us + 6.5 to 11 ps (us per
-// cycle, pushed / tiled: 1.5e7 events 121 / 79, 3.0e7 with 50-step delays 331 / 127, 6.4e7 440 / 160,
-// 4.8e8 with 50-step delays 3,040 / 1,280), so cycles above TILE_MIN_EVENTS. Tiled shares follow the
-// previous cycle, most of whose spikes are delivered again with another delay: delays of at least 4
-// steps. Only for generated networks (the copy is made on the GPU, in about the time of the rows) and
-// where a quarter of the device's memory stays free; build_tiles = -1 keeps the rows alone.
-#define TILE_MIN_EVENTS 7.0e6f
-static bool push_holds_tiles(const Engine &e)
+// Push delivery of a large network may hold the tiled copy too, and deliver its busy cycles from it: the
+// sums are the same, and one L2 reduction per event (~1.5e11/s) is what bounds a pushed cycle. Tiled
+// shares follow the previous cycle, most of whose spikes are delivered again with another delay: delays
+// of at least 4 steps. Only for generated networks (the copy is made on the GPU, in about the time of the
+// rows); build_tiles = -1 keeps the rows alone.
+static bool push_may_hold_tiles(const Engine &e)
 {
-    if (e.opt.accumulate != BSIM_ACC_EXACT || e.opt.delivery != BSIM_DELIVERY_PUSH || e.opt.build_tiles != 0 ||
-        e.D < 4 || e.D > 64 || e.S < 50000000 || many_cycles(e))
-        return false;
+    return e.opt.accumulate == BSIM_ACC_EXACT && e.opt.delivery == BSIM_DELIVERY_PUSH && e.opt.build_tiles == 0 &&
+           e.D >= 4 && e.D <= 64 && e.S >= 50000000 && !many_cycles(e);
+}
+
+// The spikes of the delay window above which a cycle of such a network is cheaper tiled, 0 if it never is.
+// Pushed, a cycle costs PUSH_ITEM_NS per (spike, delay) row and ~6 ps per event; tiled, TILE_START_NS more
+// at the start, TILE_UNIT_NS per 32-source unit scanned, TILE_SEGMENT_NS per segment listed (one per spike,
+// delay and tile that the source reaches, empty ones too) and ~2 ps per event. Fitted to 90 networks of 8e5
+// and 1e6 neurons with 6e7 to 2.4e9 synapses (us per cycle, tiled / pushed): 200 x 5,000 with 6-step delays,
+// 1.5e7 events 109 / 208, 3.9e6 50 / 45; 50 x 20,000 with 50-step delays, 4.3e8 events 1,280 / 2,606, 2.5e7
+// 207 / 133; 4 x 200,000 (40 tiles each) with 20-step delays, 4.4e8 events 2,113 / 2,654, 1.4e8 1,798 / 940,
+// 2e7 2,196 / 668. Held against ten others: 25 x 10,000, 4.3e7 events 135 / 292; 8 x 50,000 with 30-step
+// delays, 5.6e7 events 486 / 402; 16 x 30,000 with 60-step delays, 2.1e8 events 767 / 1,297.
+#define PUSH_ITEM_NS 0.08
+#define TILE_START_NS 30000.0
+#define TILE_UNIT_NS 0.025
+#define TILE_SEGMENT_NS 0.010
+#define TILE_EVENT_GAIN_NS 0.004  // pushed less tiled, per event
+static float tiled_from_spikes(const Engine &e, int64_t n_seg, int64_t units)
+{
+    const double window = (double)e.N * e.D;  // (spike, delay) rows if every neuron fires in every cycle
+    const double gain = PUSH_ITEM_NS - TILE_SEGMENT_NS * (double)n_seg / window + TILE_EVENT_GAIN_NS * (double)e.S / window;
+    if (!(gain > 0.0)) return 0.0f;
+    const double spikes = (TILE_START_NS + TILE_UNIT_NS * (double)units) / gain;
+    return spikes < 0.5 * window ? (float)spikes : 0.0f;
+}
+
+// Whether the tiled copy of n_seg segment starts (4 bytes each; 8 per entry, an entry of padding per odd
+// segment) leaves a quarter of the device's memory free, the rows being there already.
+static bool tiles_leave_room(const Engine &e, int64_t n_seg)
+{
     size_t free = 0, total = 0;
     if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
-    return (double)free - (18.0 * (double)e.S + 24.0 * (double)e.N * e.D) > 0.25 * (double)total;
+    const double bytes = 8.0 * ((double)e.S + (double)std::min(e.S, n_seg)) + 4.0 * (double)n_seg;
+    return (double)free - bytes > 0.25 * (double)total;
 }
 
 // Host-side description of the tiled copy.
@@ -1278,6 +1302,159 @@ static int check_spec(const bsim_gen_spec &g)
     return BSIM_OK;
 }
 
+// The tiled copy of generated networks: tiles, their (source population, target range) segments and
+// where the starts of their (delay, source) segments lie.
+struct GenTiles {
+    TileHost th;
+    std::vector<TileSeg> segs;
+    std::vector<TileRun> runs;
+    std::vector<int64_t> tile_idx0;  // [tiles + 1] index in seg_off
+    int64_t pairs = 0, n_seg = 0;
+};
+
+static GenTiles plan_gen_tiles(const Engine &E, const std::vector<GenInst> &gi, const std::vector<GenPlan> &plans)
+{
+    // target ranges follow population boundaries
+    std::vector<int64_t> runs;
+    std::vector<int32_t> net;
+    for (size_t k = 0; k < gi.size(); k++)
+        for (int pp = 0; pp < gi[k].P; pp++) {
+            runs.push_back(gi[k].nbase + (int64_t)pp * gi[k].n);
+            net.push_back((int32_t)k);
+        }
+    runs.push_back(E.N);
+    GenTiles gt;
+    TileHost &th = gt.th;
+    plan_tiles(runs, net, auto_tile_size(E.opt, E.N, E.sm_count, E.D), th.tile_beg, th.tile_max);
+    const std::vector<int32_t> &tile_beg = th.tile_beg;
+    const int32_t nt = (int32_t)tile_beg.size() - 1;
+    th.n_u = nt;
+    th.tile_scale.resize(nt);
+    th.tile_run_off.assign(nt + 1, 0);
+    int64_t &pairs = gt.pairs, &n_seg = gt.n_seg;
+    gt.tile_idx0.assign(nt + 1, 0);
+    size_t k = 0;
+    for (int32_t q = 0; q < nt; q++) {
+        while (k + 1 < gi.size() && gi[k + 1].nbase <= tile_beg[q]) k++;
+        const GenInst &x = gi[k];
+        const GenPlan &pl = plans[k];
+        th.tile_units.push_back(0);
+        th.tile_run_off[q + 1] = th.tile_run_off[q];
+        th.tile_scale[q] = ldexpf(1.0f, E.qexp[k]);
+        const int64_t lb = tile_beg[q] - x.nbase, le = tile_beg[q + 1] - x.nbase;
+        for (int64_t pp = lb / x.n; pp <= (le - 1) / x.n; pp++) {
+            const int64_t pop_beg = pp * x.n;
+            const int32_t j0 = (int32_t)(std::max(lb, pop_beg) - pop_beg);
+            const int32_t j1 = (int32_t)(std::min(le, pop_beg + x.n) - pop_beg);
+            for (int id : pl.in[pp]) {
+                TileSeg sg;
+                sg.pair_start = pairs;
+                sg.seg0 = n_seg;
+                sg.base = 0;
+                sg.pseed = pl.proj[id].pseed;
+                sg.src_base = x.nbase + (int64_t)pl.proj[id].src_pop * x.n;
+                sg.j0 = j0;
+                sg.j1 = j1;
+                sg.tgt_off = (int32_t)(pop_beg + j0 - lb);
+                sg.n_src = x.n;
+                sg.p24 = x.p24;
+                sg.exc24 = x.exc24;
+                sg.w_exc = x.w_exc;
+                sg.w_inh = x.w_inh;
+                sg.d_inst = x.D;
+                sg.T = tile_beg[q + 1] - tile_beg[q];
+                sg.scale = th.tile_scale[q];
+                gt.segs.push_back(sg);
+                gt.runs.push_back(TileRun{pairs, n_seg, 0, x.n, x.D, sg.T});
+                add_run(th, (uint32_t)sg.src_base, x.n, n_seg, x.D);  // the network's own delay range
+                pairs += x.n;
+                n_seg += (int64_t)x.n * x.D + 1;
+            }
+        }
+        gt.tile_idx0[q + 1] = n_seg;
+    }
+    return gt;
+}
+
+// Device memory that is freed with the scope.
+struct Scratch {
+    std::vector<void *> p;
+    ~Scratch()
+    {
+        for (void *q : p) cudaFree(q);
+    }
+    template <typename T>
+    int get(T **out, size_t count)
+    {
+        if (cudaMalloc((void **)out, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(BSIM_ERR_NOMEM, "build scratch allocation failed");
+        }
+        p.push_back(*out);
+        return BSIM_OK;
+    }
+};
+
+static int build_gen_tiles(Engine &E, const GenTiles &gt)
+{
+    const TileHost &th = gt.th;
+    std::vector<TileSeg> segs = gt.segs;
+    std::vector<TileRun> runs = gt.runs;
+    const int64_t pairs = gt.pairs, n_seg = gt.n_seg;
+    const int32_t nt = th.n_u;
+    const int gb = E.sm_count * 8;
+    TileSeg *d_segs;
+    int64_t *d_idx0;
+    unsigned long long *d_total;
+    Scratch tmp;
+    TRY(tmp.get(&d_segs, segs.size()));
+    TRY(tmp.get(&d_idx0, nt + 1));
+    TRY(tmp.get(&d_total, nt));
+    if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(d_idx0, gt.tile_idx0.data(), sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice);
+    uint32_t *d_seg;
+    int64_t *d_seg0;
+    TRY(dalloc(E, &d_seg, n_seg));
+    TRY(dalloc(E, &d_seg0, nt));
+    cudaMemsetAsync(d_seg, 0, sizeof(uint32_t) * n_seg, E.stream);
+    cudaMemsetAsync(d_total, 0, sizeof(unsigned long long) * nt, E.stream);
+    gen_tile_kernel<0><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, d_seg, nullptr, nullptr);
+    tile_total_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_total);
+    std::vector<unsigned long long> total(nt, 0);
+    cudaMemcpyAsync(total.data(), d_total, sizeof(unsigned long long) * nt, cudaMemcpyDeviceToHost, E.stream);
+    if (cudaStreamSynchronize(E.stream) != cudaSuccess) return fail(BSIM_ERR_CUDA, "generator: tiled copy sizes");
+    std::vector<int64_t> tile_seg0(nt, 0);
+    int64_t ent_pairs = 0;
+    for (int32_t q = 0; q < nt; q++) {
+        if (total[q] > (unsigned long long)UINT32_MAX)
+            return fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries");
+        tile_seg0[q] = ent_pairs;
+        ent_pairs += (int64_t)total[q];
+        for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++)
+            segs[r].base = runs[r].base = tile_seg0[q];
+    }
+    cudaMemcpy(d_seg0, tile_seg0.data(), sizeof(int64_t) * nt, cudaMemcpyHostToDevice);
+    if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
+    if (n_seg > 0) {  // starts from the counts, wrapping at 2^32, then relative to the tile
+        size_t tb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tb, d_seg, d_seg, n_seg, E.stream);
+        char *d_tb;
+        TRY(tmp.get(&d_tb, tb));
+        cub::DeviceScan::ExclusiveSum(d_tb, tb, d_seg, d_seg, n_seg, E.stream);
+        tile_rebase_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_seg0);
+    }
+    uint2 *d_ent;
+    TRY(dalloc(E, &d_ent, 2 * ent_pairs));
+    gen_tile_kernel<1><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, nullptr, d_seg, d_ent);
+    if (cudaStreamSynchronize(E.stream) != cudaSuccess) return fail(BSIM_ERR_CUDA, "generator: tiled copy");
+    E.a.seg_off = d_seg;
+    E.a.tile_seg0 = d_seg0;
+    E.a.ent = d_ent;
+    TRY(spread_tiles(E, runs, pairs));
+    TRY(upload_tiles(E, th));
+    return BSIM_OK;
+}
+
 static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, const bsim_options *opt, Engine **out)
 {
     if (!specs || ns < 1 || !(dt > 0) || !out) return fail(BSIM_ERR_ARG, "bsim_create_generated: invalid arguments");
@@ -1442,132 +1619,8 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         E.a.csc_w = d_cw;
         E.a.csc_d = d_cd;
     }
-    // target-tiled copy
-    const bool busy_tiles = push_holds_tiles(E);
-    const bool tiles = wants_tiles(E.opt, D) || busy_tiles;
-    E.a.tile_events = busy_tiles ? TILE_MIN_EVENTS : 0.0f;
-    if (tiles) {
-        // target ranges follow population boundaries
-        std::vector<int64_t> runs;
-        std::vector<int32_t> net;
-        for (int k = 0; k < ns; k++)
-            for (int pp = 0; pp < gi[k].P; pp++) {
-                runs.push_back(gi[k].nbase + (int64_t)pp * gi[k].n);
-                net.push_back(k);
-            }
-        runs.push_back(N);
-        std::vector<int32_t> tile_beg;
-        int32_t tile_max = 0;
-        plan_tiles(runs, net, auto_tile_size(E.opt, N, E.sm_count, D), tile_beg, tile_max);
-        const int32_t nu = (int32_t)tile_beg.size() - 1, nt = nu;
-        std::vector<TileSeg> segs;
-        TileHost th;
-        th.n_u = nu;
-        th.tile_beg = tile_beg;
-        th.tile_max = tile_max;
-        th.tile_scale.resize(nt);
-        th.tile_run_off.assign(nt + 1, 0);
-        int64_t pairs = 0, n_seg = 0;
-        std::vector<int64_t> tile_idx0(nt + 1, 0);
-        std::vector<TileRun> runs_d;
-        for (int32_t q = 0; q < nt; q++) {
-            const int32_t qu = q;
-            int k = 0;
-            while (k + 1 < ns && gi[k + 1].nbase <= tile_beg[qu]) k++;
-            const GenInst &x = gi[k];
-            const GenPlan &pl = plans[k];
-            th.tile_units.push_back(0);
-            th.tile_run_off[q + 1] = th.tile_run_off[q];
-            th.tile_scale[q] = ldexpf(1.0f, E.qexp[k]);
-            const int64_t lb = tile_beg[qu] - x.nbase, le = tile_beg[qu + 1] - x.nbase;
-            for (int64_t pp = lb / x.n; pp <= (le - 1) / x.n; pp++) {
-                const int64_t pop_beg = pp * x.n;
-                const int32_t j0 = (int32_t)(std::max(lb, pop_beg) - pop_beg);
-                const int32_t j1 = (int32_t)(std::min(le, pop_beg + x.n) - pop_beg);
-                for (int id : pl.in[pp]) {
-                    TileSeg sg;
-                    sg.pair_start = pairs;
-                    sg.seg0 = n_seg;
-                    sg.base = 0;
-                    sg.pseed = pl.proj[id].pseed;
-                    sg.src_base = x.nbase + (int64_t)pl.proj[id].src_pop * x.n;
-                    sg.j0 = j0;
-                    sg.j1 = j1;
-                    sg.tgt_off = (int32_t)(pop_beg + j0 - lb);
-                    sg.n_src = x.n;
-                    sg.p24 = x.p24;
-                    sg.exc24 = x.exc24;
-                    sg.w_exc = x.w_exc;
-                    sg.w_inh = x.w_inh;
-                    sg.d_inst = x.D;
-                    sg.T = tile_beg[qu + 1] - tile_beg[qu];
-                    sg.scale = th.tile_scale[q];
-                    segs.push_back(sg);
-                    runs_d.push_back(TileRun{pairs, n_seg, 0, x.n, x.D, sg.T});
-                    add_run(th, (uint32_t)sg.src_base, x.n, n_seg, x.D);  // the network's own delay range
-                    pairs += x.n;
-                    n_seg += (int64_t)x.n * x.D + 1;
-                }
-            }
-            tile_idx0[q + 1] = n_seg;
-        }
-        TileSeg *d_segs;
-        int64_t *d_idx0;
-        unsigned long long *d_total;
-        if ((rc = talloc((void **)&d_segs, sizeof(TileSeg) * std::max<size_t>(1, segs.size()))) ||
-            (rc = talloc((void **)&d_idx0, sizeof(int64_t) * (nt + 1))) ||
-            (rc = talloc((void **)&d_total, sizeof(unsigned long long) * nt))) { free_tmp(); return bail(rc); }
-        if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
-        cudaMemcpy(d_idx0, tile_idx0.data(), sizeof(int64_t) * (nt + 1), cudaMemcpyHostToDevice);
-        uint32_t *d_seg;
-        int64_t *d_seg0;
-        if ((rc = dalloc(E, &d_seg, n_seg)) || (rc = dalloc(E, &d_seg0, nt))) { free_tmp(); return bail(rc); }
-        cudaMemsetAsync(d_seg, 0, sizeof(uint32_t) * n_seg, E.stream);
-        cudaMemsetAsync(d_total, 0, sizeof(unsigned long long) * nt, E.stream);
-        gen_tile_kernel<0><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, d_seg, nullptr, nullptr);
-        tile_total_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_total);
-        std::vector<unsigned long long> total(nt, 0);
-        cudaMemcpyAsync(total.data(), d_total, sizeof(unsigned long long) * nt, cudaMemcpyDeviceToHost, E.stream);
-        if (cudaStreamSynchronize(E.stream) != cudaSuccess) {
-            free_tmp();
-            return bail(fail(BSIM_ERR_CUDA, "generator: tiled copy sizes"));
-        }
-        std::vector<int64_t> tile_seg0(nt, 0);
-        int64_t ent_pairs = 0;
-        for (int32_t q = 0; q < nt; q++) {
-            if (total[q] > (unsigned long long)UINT32_MAX) {
-                free_tmp();
-                return bail(fail(BSIM_ERR_LIMIT, "tiled delivery: a tile with more than 2^33 entries"));
-            }
-            tile_seg0[q] = ent_pairs;
-            ent_pairs += (int64_t)total[q];
-            for (int32_t r = th.tile_run_off[q]; r < th.tile_run_off[q + 1]; r++)
-                segs[r].base = runs_d[r].base = tile_seg0[q];
-        }
-        cudaMemcpy(d_seg0, tile_seg0.data(), sizeof(int64_t) * nt, cudaMemcpyHostToDevice);
-        if (!segs.empty()) cudaMemcpy(d_segs, segs.data(), sizeof(TileSeg) * segs.size(), cudaMemcpyHostToDevice);
-        if (n_seg > 0) {  // starts from the counts, wrapping at 2^32, then relative to the tile
-            size_t tb = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, tb, d_seg, d_seg, n_seg, E.stream);
-            void *d_tb;
-            if ((rc = talloc(&d_tb, tb))) { free_tmp(); return bail(rc); }
-            cub::DeviceScan::ExclusiveSum(d_tb, tb, d_seg, d_seg, n_seg, E.stream);
-            tile_rebase_kernel<<<nt, 256, 0, E.stream>>>(d_seg, d_idx0, nt, d_seg0);
-        }
-        uint2 *d_ent;
-        if ((rc = dalloc(E, &d_ent, 2 * ent_pairs))) { free_tmp(); return bail(rc); }
-        gen_tile_kernel<1><<<gb, 256, 0, E.stream>>>(d_segs, (int)segs.size(), pairs, nullptr, d_seg, d_ent);
-        if (cudaStreamSynchronize(E.stream) != cudaSuccess) {
-            free_tmp();
-            return bail(fail(BSIM_ERR_CUDA, "generator: tiled copy"));
-        }
-        E.a.seg_off = d_seg;
-        E.a.tile_seg0 = d_seg0;
-        E.a.ent = d_ent;
-        if ((rc = spread_tiles(E, runs_d, pairs))) { free_tmp(); return bail(rc); }
-        if ((rc = upload_tiles(E, th))) { free_tmp(); return bail(rc); }
-    }
     // push rows (not needed when every step uses the tiled copy)
+    const bool tiles = wants_tiles(E.opt, D);
     if (!(tiles && E.opt.delivery == BSIM_DELIVERY_TILE) || many_cycles(E) == 1) {
         const int64_t nrows = N * (int64_t)D;
         int64_t *d_row; uint2 *d_syn;
@@ -1577,6 +1630,32 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
         gen_push_kernel<1><<<gb, 256, 0, E.stream>>>(gd, N, d_row, d_syn);
         E.a.row_off = d_row;
         E.a.syn = d_syn;
+    }
+    // target-tiled copy
+    if (tiles) {
+        const GenTiles plan = plan_gen_tiles(E, gi, plans);
+        if ((rc = build_gen_tiles(E, plan))) { free_tmp(); return bail(rc); }
+    } else if (push_may_hold_tiles(E)) {
+        // an addition: where it does not pay or fit, the engine has the rows alone
+        const GenTiles plan = plan_gen_tiles(E, gi, plans);
+        int64_t units = 0;
+        for (int32_t u : plan.th.tile_units) units += u;
+        const float from = tiled_from_spikes(E, plan.n_seg, units);
+        if (from > 0.0f && tiles_leave_room(E, plan.n_seg)) {
+            const size_t n_allocs = E.allocs.size();
+            const int64_t bytes = E.device_bytes;
+            rc = build_gen_tiles(E, plan);
+            if (rc == BSIM_OK) {
+                E.a.tile_spikes = from;
+            } else if (rc == BSIM_ERR_NOMEM || rc == BSIM_ERR_LIMIT) {
+                for (; E.allocs.size() > n_allocs; E.allocs.pop_back()) cudaFree(E.allocs.back());
+                E.device_bytes = bytes;
+                E.a.n_tiles = E.a.n_items = 0;
+            } else {
+                free_tmp();
+                return bail(rc);
+            }
+        }
     }
     cudaError_t st = cudaStreamSynchronize(E.stream);
     if (st == cudaSuccess) st = cudaGetLastError();
@@ -1805,8 +1884,7 @@ int bsim_stall_tile(bsim_engine *eh, int32_t tile)
     if (!eh) return fail(BSIM_ERR_ARG, "null engine");
     Engine &e = *H(eh);
     // a push engine that was not asked for a tiled copy has none to stall
-    if (!e.a.tile_arrive || (e.opt.delivery == BSIM_DELIVERY_PUSH && e.opt.build_tiles == 0) || tile < 0 ||
-        tile >= e.a.n_tiles)
+    if (!e.a.tile_arrive || e.a.tile_spikes > 0.0f || tile < 0 || tile >= e.a.n_tiles)
         return fail(BSIM_ERR_ARG, "bsim_stall_tile: the engine has no such tile");
     CK(cudaSetDevice(e.device));
     TRY(leave_loop(e));  // the wait is in the cycle-by-cycle form: a small engine keeps to it from here on
@@ -2399,10 +2477,11 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
     }
     std::vector<int> modes;
     if (e.a.row_off) modes.push_back(BSIM_DELIVERY_PUSH);
-    if (e.a.n_tiles > 0) modes.push_back(BSIM_DELIVERY_TILE);
+    // (the copy that a push engine holds for its busy cycles is not a mode that was asked for)
+    if (e.a.n_tiles > 0 && !(e.a.tile_spikes > 0.0f)) modes.push_back(BSIM_DELIVERY_TILE);
     const int saved_block = e.block, saved_grid = e.grid, saved_del = e.a.delivery;
-    const float saved_events = e.a.tile_events;
-    e.a.tile_events = 0.0f;  // a trial of push pushes every cycle
+    const float saved_spikes = e.a.tile_spikes;
+    e.a.tile_spikes = 0.0f;  // a trial of push pushes every cycle
     cudaEvent_t ev0, ev1;
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
@@ -2461,7 +2540,7 @@ int bsim_autotune(bsim_engine *eh, int32_t trial_steps, bsim_tune_result *out)
     }
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
-    e.a.tile_events = saved_events;
+    e.a.tile_spikes = saved_spikes;
     e.block = best_b;
     e.grid = best_g;
     // an AUTO engine keeps choosing per cycle; a fixed one takes the fastest mode
@@ -2509,6 +2588,7 @@ int bsim_get_info(bsim_engine *eh, bsim_info *info)
     info->sm_count = e.sm_count;
     info->many_cycles = loop_now(e);
     info->tile_cycles = (int64_t)ctr[3];
+    info->n_tiles = e.a.n_tiles;
     return BSIM_OK;
 }
 

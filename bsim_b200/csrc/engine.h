@@ -162,7 +162,8 @@ struct StepArgs {
     float *pred_ring;                // [4][n_pops] predicted spikes of cycle s at slot s % 4
     float *pred_sum;                 // [4][2] predicted spikes and events of cycle s at slot s % 4
     PredStats *pstats;
-    float tile_events;               // push delivery: cycles with more events than this go tiled (0: none do)
+    float tile_spikes;               // push delivery: cycles with more spikes in their delay window than this
+                                     // go tiled (0: none do)
     float pred_tol, mean_outdeg;
     float cost_push_a, cost_push_b, cost_tile_a, cost_tile_b;  // ns per cycle, ns per event
 };

@@ -1228,7 +1228,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
             __syncwarp();
             const float spikes = (float)s_cum[a.D];
             if (dm == BSIM_DELIVERY_AUTO) dm = a.pstats ? auto_delivery(a, t, spikes) : BSIM_DELIVERY_PUSH;
-            else if (a.tile_events > 0.0f && spikes * a.mean_outdeg > a.tile_events * (float)a.D) dm = BSIM_DELIVERY_TILE;
+            else if (a.tile_spikes > 0.0f && spikes > a.tile_spikes) dm = BSIM_DELIVERY_TILE;
         }
         if (dm == BSIM_DELIVERY_TILE && a.n_tiles == 0) dm = BSIM_DELIVERY_PUSH;
         if (threadIdx.x == 0) s_dm = dm;

@@ -122,7 +122,8 @@ typedef struct bsim_info {
                                 per launch with the spikes pushed (whatever EXACT delivery was asked for), 2 many
                                 cycles per launch with the rows scanned (PULL, ORDERED) */
     int64_t tile_cycles;     /* cycles delivered from the tiled copy so far */
-    int32_t reserved[4];
+    int32_t n_tiles;         /* tiles of the tiled copy held (0: none) */
+    int32_t reserved[3];
 } bsim_info;
 
 /* Fills *opt with defaults: EXACT accumulation, PUSH delivery, graphs of 64 steps. */
