@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libbsim_b200.so")
 SOURCES = ["csrc/step.cu", "csrc/build.cu", "csrc/noalloc.cu", "csrc/predictor.cu"]
-HEADERS = ["csrc/engine.h", "csrc/netgen.h", "../include/bsim_b200.h"]
+HEADERS = ["csrc/engine.h", "csrc/netgen.h", "csrc/drive.h", "csrc/loop_barrier.h", "../include/bsim_b200.h"]
 
 
 def nvcc():

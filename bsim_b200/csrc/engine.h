@@ -9,6 +9,7 @@
 
 #include "../../include/bsim_b200.h"
 #include "drive.h"
+#include "loop_barrier.h"
 
 namespace bsim {
 
@@ -191,6 +192,7 @@ struct Engine {
     // (the push form then has the spikes in flight in acc_ring, not in step_kernel's accumulators)
     int loop = 0;
     bool in_loop = false;
+    LoopBarriers loop_barriers;
     // recording
     int64_t rec_cap_alloc = 0, rec_steps_alloc = 0;
     bool rec_dirty = false;

@@ -1353,7 +1353,6 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 #define PULL_LOOP_SMEM ((size_t)216 * 1024)
 #define PULL_LOOP_WORDS (LOOP_WARPS / 2)  // words of fired flags per block at most (loop_form)
 #define PULL_LOOP_HOLD 3
-#define LOOP_ERR (1ull << 40)  // one block's error in a barrier counter; arrivals are below
 
 static __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
 {
@@ -2082,6 +2081,10 @@ int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
 
 cudaError_t launch_loop(Engine &e, int steps)
 {
+    if (e.loop_barriers.start_over(steps)) {  // (one barrier per cycle at most)
+        const cudaError_t st = cudaMemsetAsync(e.a.loop_bar, 0, sizeof(unsigned long long) * 32, e.stream);
+        if (st != cudaSuccess) return st;
+    }
     if (e.loop == 1) {
         void *args[] = {&e.a, &steps};
         const cudaError_t st = cudaFuncSetAttribute((const void *)push_loop_kernel,
