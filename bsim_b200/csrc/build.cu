@@ -1768,25 +1768,27 @@ int bsim_synapse_reset(const float *delay_s, const float *weight, const float *t
 // Engines of up to this many neurons read back through page-locked memory (1.3 MB): one copy and one
 // wait for all arrays (1,007 neurons: state 81 -> 24 us, counts 33 -> 13, through the Python binding).
 #define PINNED_MAX_NEURONS 65536
-static int ensure_host(Engine &e)
+static void ensure_host(Engine &e)
 {
-    cudaError_t st = cudaSuccess;
     std::call_once(e.host_once, [&] {
-        st = cudaHostAlloc((void **)&e.h_err, sizeof(int32_t), cudaHostAllocDefault);
-        if (st == cudaSuccess && e.N <= PINNED_MAX_NEURONS)
-            st = cudaHostAlloc((void **)&e.h_stage, 5 * sizeof(float) * (size_t)e.N, cudaHostAllocDefault);
+        if (cudaHostAlloc((void **)&e.h_err, sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) e.h_err = nullptr;
+        if (e.N <= PINNED_MAX_NEURONS &&
+            cudaHostAlloc((void **)&e.h_stage, 5 * sizeof(float) * (size_t)e.N, cudaHostAllocDefault) != cudaSuccess)
+            e.h_stage = nullptr;
+        cudaGetLastError();  // without page-locked memory the copies go to the caller's
     });
-    if (st != cudaSuccess) cudaGetLastError();
-    return e.h_err ? BSIM_OK : fail(BSIM_ERR_NOMEM, "page-locked host memory");
 }
 
-// Waits for the engine's stream; the error flag comes with the same wait.
+// Waits for the engine's stream; the error flag comes with the same wait. (Threads may wait at the same
+// time: the flag never changes once it is set, so each reads its own wait's value or a later one.)
 static int sync_and_check(Engine &e)
 {
-    TRY(ensure_host(e));
-    CK(cudaMemcpyAsync(e.h_err, e.a.err, sizeof(int32_t), cudaMemcpyDeviceToHost, e.stream));
+    ensure_host(e);
+    int32_t pageable = 0;
+    int32_t *flag = e.h_err ? e.h_err : &pageable;
+    CK(cudaMemcpyAsync(flag, e.a.err, sizeof(int32_t), cudaMemcpyDeviceToHost, e.stream));
     CK(cudaStreamSynchronize(e.stream));
-    const int32_t err = *e.h_err;
+    const int32_t err = *flag;
     if (err) {
         static const char *names[] = {"", "row offsets not ascending", "synapse target outside the network",
                                       "class index or kind out of range", "row offsets do not span the synapses",
@@ -2106,11 +2108,12 @@ int bsim_read_state(bsim_engine *eh, float *v, float *iE, float *iI, int32_t *re
     if (!eh) return fail(BSIM_ERR_ARG, "null engine");
     Engine &e = *H(eh);
     CK(cudaSetDevice(e.device));
+    std::lock_guard<std::mutex> lock(e.stage_mutex);  // until the caller's arrays hold this moment's state
     TRY(ensure_stage(e));
     state_unpack_kernel<<<state_grid(e), 256, 0, e.stream>>>(e.a.state, e.stage, e.N);
     CK(cudaGetLastError());
     void *dst[4] = {v, iE, iI, refrac};
-    TRY(ensure_host(e));
+    ensure_host(e);
     if (e.h_stage) {
         const size_t bytes = sizeof(float) * (size_t)e.N;
         CK(cudaMemcpyAsync(e.h_stage, e.stage, 4 * bytes, cudaMemcpyDeviceToHost, e.stream));
@@ -2132,6 +2135,7 @@ int bsim_write_state(bsim_engine *eh, const float *v, const float *iE, const flo
     if (!eh) return fail(BSIM_ERR_ARG, "null engine");
     Engine &e = *H(eh);
     CK(cudaSetDevice(e.device));
+    std::lock_guard<std::mutex> lock(e.stage_mutex);
     TRY(ensure_stage(e));
     const void *src[4] = {v, iE, iI, refrac};
     for (int k = 0; k < 4; k++)
@@ -2181,8 +2185,9 @@ int bsim_read_fire_count(bsim_engine *eh, int32_t *count)
     if (!eh || !count) return fail(BSIM_ERR_ARG, "invalid arguments");
     Engine &e = *H(eh);
     CK(cudaSetDevice(e.device));
-    TRY(ensure_host(e));
+    ensure_host(e);
     if (e.h_stage) {
+        std::lock_guard<std::mutex> lock(e.count_mutex);
         float *h = e.h_stage + 4 * (size_t)e.N;
         CK(cudaMemcpyAsync(h, e.a.fire_count, sizeof(int32_t) * e.N, cudaMemcpyDeviceToHost, e.stream));
         CK(cudaStreamSynchronize(e.stream));

@@ -207,8 +207,10 @@ struct Engine {
     float *stage = nullptr;
     // page-locked (ensure_host): the error flag as the last synchronisation saw it and, for small
     // engines, five planes of N words for the state's fields and the spike counts (a copy into the
-    // caller's pageable memory waits for each piece by itself)
+    // caller's pageable memory waits for each piece by itself). The state's planes here and in `stage`
+    // belong to the thread that holds stage_mutex, the counts' to that which holds count_mutex.
     std::once_flag host_once;
+    std::mutex stage_mutex, count_mutex;
     int32_t *h_err = nullptr;
     float *h_stage = nullptr;
     // schedule state: predictor statistics and the MLP's parameters (a.pstats / a.mlp
