@@ -903,11 +903,12 @@ static int spread_tiles(Engine &e, const std::vector<TileRun> &runs, int64_t n_p
     return BSIM_OK;
 }
 
-// {counter offset, scaled weight} of one synapse onto target `tgt` of a tile of T targets.
+// {counter offset, scaled weight} of one synapse onto target `tgt` of a tile of T targets. A weight that is
+// zero, or underflows to it, is stored as +0.0f: TILE_PAD_W marks padding.
 static inline uint2 tile_entry(int64_t tgt, int32_t T, float w, float scale)
 {
     const float ws = w * scale;  // a power of two
-    return make_uint2(4u * (uint32_t)(tgt + (w >= 0.0f ? 0 : 2 * (int64_t)T)), w == 0.0f ? 0u : f2u(ws));
+    return make_uint2(4u * (uint32_t)(tgt + (w >= 0.0f ? 0 : 2 * (int64_t)T)), ws == 0.0f ? 0u : f2u(ws));
 }
 
 // Host construction of the tiled copy: target ranges follow population (and
@@ -1274,8 +1275,9 @@ __global__ void gen_tile_kernel(const TileSeg *segs, int n_segs, int64_t n_pairs
                 const long long at = cur[sd.d - 1] + __popc(same & ((1u << lane) - 1u));
                 if (PASS == 1) {
                     const unsigned tgt = (unsigned)(sg.tgt_off + (j - sg.j0));
+                    const float ws = __fmul_rn(sd.w, sg.scale);
                     ent[at] = make_uint2(4u * (tgt + (sd.w >= 0.0f ? 0u : 2u * (unsigned)sg.T)),
-                                         sd.w == 0.0f ? 0u : __float_as_uint(__fmul_rn(sd.w, sg.scale)));
+                                         ws == 0.0f ? 0u : __float_as_uint(ws));
                 }
                 __syncwarp(same);
                 if (lane == leader) cur[sd.d - 1] += __popc(same);
