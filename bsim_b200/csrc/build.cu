@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <map>
+#include <tuple>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -911,6 +912,50 @@ static inline uint2 tile_entry(int64_t tgt, int32_t T, float w, float scale)
     return make_uint2(4u * (uint32_t)(tgt + (w >= 0.0f ? 0 : 2 * (int64_t)T)), ws == 0.0f ? 0u : f2u(ws));
 }
 
+// The limit on host networks: 65,535 synapses (each delay's counted to an even number) of one source into
+// one range of targets, a population's near-equal part of at most `limit_range` neurons. The copy itself
+// has no such limit; the ranges are not its tiles, so that larger tiles and tiles that small populations
+// share refuse nothing more.
+static int64_t limit_range(const bsim_options &o, int64_t N, int sm_count, int32_t D)
+{
+    if (o.tile_size > 0) return std::min<int64_t>(o.tile_size, 12288);
+    int64_t t = std::max<int64_t>((int64_t)std::ceil((double)N / (2.0 * sm_count)), (int64_t)(1700.0 * std::sqrt((double)D / 6.0)));
+    t = std::min<int64_t>(t, (2 * N + sm_count - 1) / sm_count);
+    return std::max<int64_t>(256, std::min<int64_t>(5000, t));
+}
+
+static bool source_over_limit(const Engine &e, const std::vector<int64_t> &pop_beg, const int32_t *src, const int32_t *dst,
+                              const int32_t *delay, int64_t s)
+{
+    const int64_t limit = 65535;
+    std::vector<int64_t> out(e.N, 0);
+    for (int64_t k = 0; k < s; k++) out[src[k]]++;
+    std::vector<int64_t> order;  // of the sources that could be over it (padding at most doubles a count)
+    for (int64_t k = 0; k < s; k++)
+        if (2 * out[src[k]] > limit) order.push_back(k);
+    if (order.empty()) return false;
+    std::vector<int32_t> range_of(e.N);
+    const int64_t size = limit_range(e.opt, e.N, e.sm_count, e.D);
+    int32_t ranges = 0;
+    for (size_t r = 0; r + 1 < pop_beg.size(); r++) {
+        const int64_t b = pop_beg[r], len = pop_beg[r + 1] - b, parts = (len + size - 1) / size;
+        for (int64_t i = 0; i < parts; i++, ranges++)
+            for (int64_t j = b + len * i / parts; j < b + len * (i + 1) / parts; j++) range_of[j] = ranges;
+    }
+    auto key = [&](int64_t k) { return std::make_tuple(src[k], range_of[dst[k]], delay[k]); };
+    std::sort(order.begin(), order.end(), [&](int64_t x, int64_t y) { return key(x) < key(y); });
+    int64_t sum = 0;
+    for (size_t i = 0; i < order.size();) {
+        size_t j = i + 1;
+        while (j < order.size() && key(order[j]) == key(order[i])) j++;
+        const bool same = i > 0 && src[order[i]] == src[order[i - 1]] && range_of[dst[order[i]]] == range_of[dst[order[i - 1]]];
+        sum = (same ? sum : 0) + (((int64_t)(j - i) + 1) & ~1ll);
+        if (sum > limit) return true;
+        i = j;
+    }
+    return false;
+}
+
 // Host construction of the tiled copy: target ranges follow population (and
 // network) boundaries; synapses sorted by (tile of the target, source, delay);
 // one pair per distinct (tile, source), runs of consecutive sources.
@@ -925,6 +970,8 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
     std::vector<int32_t> net;
     for (int64_t b : runs) net.push_back(inst ? inst[b] : 0);
     runs.push_back(n);
+    if (source_over_limit(e, runs, src, dst, delay, s))
+        return fail(BSIM_ERR_LIMIT, "tiled delivery: a source has more than 65535 synapses into one tile");
     TileHost th;
     plan_tiles(runs, net, auto_tile_size(e.opt, n, e.sm_count, D), th.tile_beg, th.tile_max);
     th.n_u = (int32_t)th.tile_beg.size() - 1;
@@ -999,14 +1046,6 @@ static int build_tiles_host(Engine &e, const int32_t *inst, const int32_t *pop, 
         }
     };
     for_each([&](size_t r, int32_t, int64_t k) { seg_off[seg_at(runs_d[r], th.run_src0[r], k)]++; });
-    bool pair_overflow = false;
-    for (const TileRun &rn : runs_d)
-        for (int64_t i = 0; i < rn.n; i++) {
-            int64_t c = 0;
-            for (int32_t d = 0; d < rn.D; d++) c += (seg_off[rn.seg0 + (int64_t)d * rn.n + i] + 1) & ~1u;
-            pair_overflow |= c > 65535;
-        }
-    if (pair_overflow) return fail(BSIM_ERR_LIMIT, "tiled delivery: a source has more than 65535 synapses into one tile");
     std::vector<int64_t> tile_seg0(nt, 0);
     int64_t at = 0;
     for (int32_t q = 0; q < nt; q++) {
