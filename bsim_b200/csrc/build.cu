@@ -24,7 +24,8 @@ namespace bsim {
 
 cudaError_t launch_step(Engine &e);
 cudaError_t launch_record_flush(Engine &e);
-int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count);
+int loop_form(const bsim_options &o, int64_t N, int32_t D, int64_t S, int64_t max_indeg, int sm_count);
+int64_t loop_launch_cycles(const Engine &e);
 cudaError_t launch_loop(Engine &e, int steps);
 cudaError_t launch_loop_enter(Engine &e);
 cudaError_t launch_loop_leave(Engine &e);
@@ -35,9 +36,6 @@ cudaError_t step_set_smem(int accumulate, size_t bytes);
 
 #ifndef TILE_MAX_DEPTH
 #define TILE_MAX_DEPTH 3
-#endif
-#ifndef LOOP_STEPS
-#define LOOP_STEPS 4096  // cycles of one many-cycle launch at most
 #endif
 
 static thread_local std::string g_err;
@@ -253,6 +251,7 @@ static int create_from_arrays(const float *params, const uint8_t *kind, int64_t 
     if (rc != BSIM_OK) { free_engine(e); return rc; }
     e->N = n;
     e->S = s;
+    e->max_indeg = *std::max_element(maxdeg.begin(), maxdeg.end());
     e->D = D;
     e->dt = dt;
     e->n_inst = n_inst;
@@ -450,7 +449,7 @@ static int create_from_arrays(const float *params, const uint8_t *kind, int64_t 
 // launch shape gets one launch per cycle.
 static int many_cycles(const Engine &e)
 {
-    return e.opt.block_threads > 0 || e.opt.grid_blocks > 0 ? 0 : loop_form(e.opt, e.N, e.D, e.sm_count);
+    return e.opt.block_threads > 0 || e.opt.grid_blocks > 0 ? 0 : loop_form(e.opt, e.N, e.D, e.S, e.max_indeg, e.sm_count);
 }
 
 // Ring, bitmaps, accumulators, counters; launch shape. Shared by both builders.
@@ -1641,6 +1640,7 @@ static int create_generated(const bsim_gen_spec *specs, int32_t ns, float dt, co
     cudaMemcpyAsync(maxw.data(), d_maxw, 4 * ns, cudaMemcpyDeviceToHost, E.stream);
     if (cudaStreamSynchronize(E.stream) != cudaSuccess) { free_tmp(); return bail(fail(BSIM_ERR_CUDA, std::string("generator: ") + cudaGetErrorString(cudaGetLastError()))); }
     E.S = S;
+    E.max_indeg = (int64_t)*std::max_element(maxdeg.begin(), maxdeg.end());
     E.qexp.resize(ns);
     for (int k = 0; k < ns; k++) {
         float mw;
@@ -1879,8 +1879,8 @@ int bsim_run_async(bsim_engine *eh, int64_t steps)
     const int gl = e.opt.graph_steps;
     if (left > 0 && loop_now(e)) {
         TRY(enter_loop(e));
-        for (int k; left > 0; left -= k) {  // bounded, so that a launch ends within a second
-            k = (int)std::min<int64_t>(left, LOOP_STEPS);
+        for (int k; left > 0; left -= k) {
+            k = (int)std::min(left, loop_launch_cycles(e));
             CK(launch_loop(e, k));
         }
     }

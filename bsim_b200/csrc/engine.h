@@ -175,6 +175,7 @@ struct Engine {
     bsim_options opt{};
     int sm_count = 0;
     int64_t N = 0, S = 0;
+    int64_t max_indeg = 0;  // longest row by target
     int32_t D = 1;
     float dt = 0.0f;
     int32_t n_inst = 1, n_cls = 0, n_pops = 1;

@@ -1644,18 +1644,11 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
             }
             int slot0 = slot + sp.cycle + 2;  // of delay 1
             if (slot0 >= Ra) slot0 -= Ra;
-            auto add = [&](int64_t e, uint32_t tgt, uint32_t wbits) {
+            auto add = [&](int d, uint32_t tgt, uint32_t wbits) {  // d: delay - 1
                 if ((int64_t)tgt >= a.N) {  // a target outside the network: flag it, touch nothing
                     raise_error(a, BSIM_DEVERR_TARGET);
                     s_err = true;
                     return;
-                }
-                const unsigned x = (unsigned)(e - r0);
-                int d = 0, top = D - 1;  // delay - 1: the segment that holds entry x
-                while (d < top) {
-                    const int mid = (d + top + 1) >> 1;
-                    if (off[mid] <= x) d = mid;
-                    else top = mid - 1;
                 }
                 int sl = slot0 + d;
                 if (sl >= Ra) sl -= Ra;
@@ -1664,24 +1657,53 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
                 red_add_u64(reinterpret_cast<unsigned long long *>(acc + (int64_t)sl * a.N + tgt) + (w >= 0.0f ? 0 : 1),
                             (unsigned long long)q);
             };
+            // the segments that hold entries e and e + 1, one search for both
+            auto add_pair = [&](int64_t e, uint4 v) {
+                int d = 0;
+                if (D > 1) {
+                    const unsigned x = (unsigned)(max(e, lo) - r0);
+                    int top = D - 1;
+                    while (d < top) {
+                        const int mid = (d + top + 1) >> 1;
+                        if (off[mid] <= x) d = mid;
+                        else top = mid - 1;
+                    }
+                }
+                if (e >= lo) add(d, v.x, v.y);
+                if (e + 1 < hi) {
+                    if (D > 1)
+                        while (off[d + 1] <= (unsigned)(e + 1 - r0)) d++;
+                    add(d, v.z, v.w);
+                }
+            };
             if (it % split == 0)  // delivered in cycle t+i+d: counted when that cycle has run
                 for (int d = lane; d < D; d += 32) {
                     int sl = slot + sp.cycle + 1 + d;
                     if (sl >= Ra) sl -= Ra;
                     if (off[d + 1] != off[d]) atomicAdd(&s_ev[sl], (unsigned long long)(off[d + 1] - off[d]));
                 }
-            // pairs of entries from even positions; the rows are read again within cycles, so they
-            // stay in L2 (the array has room for the pair that holds its last entry)
-            for (int64_t e0 = (lo & ~1ll) + 2 * lane; e0 < hi; e0 += 4 * 64) {
+            // Pairs of entries from even positions; the rows are read again within cycles, so they
+            // stay in L2 (the array has room for the pair that holds its last entry). Each row is
+            // walked from a point of its own, wrapping around, so that blocks whose rows hit the same
+            // targets do not add into the same addresses in lockstep, and one search finds the delays
+            // of both entries of a pair (us per cycle, before / after: 2 x 6,000 neurons at p = 0.5,
+            // 2 kHz, 1-step delays 79 / 64, 50-step delays 80 / 60; 10 x 1,000 all-to-all, 500 Hz,
+            // 10.4 / 10.1 and 16.2 / 12.6).
+            const int64_t even = lo & ~1ll;
+            const int n_pairs = (int)((hi - even + 1) >> 1);
+            const int rot = (int)__umulhi((unsigned)sp.who * 2654435769u + blockIdx.x * 2246822519u, (unsigned)n_pairs);
+            for (int q0 = lane; q0 < n_pairs; q0 += 4 * 32) {
                 uint4 v[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (e0 + u * 64 < hi) v[u] = __ldg(reinterpret_cast<const uint4 *>(a.syn + e0 + u * 64));
+                for (int u = 0; u < 4; u++) {
+                    const int q = q0 + u * 32 + rot;
+                    if (q0 + u * 32 < n_pairs) v[u] = __ldg(reinterpret_cast<const uint4 *>(a.syn + even + 2 * (q < n_pairs ? q : q - n_pairs)));
+                }
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const int64_t e = e0 + u * 64;
-                    if (e < hi && e >= lo) add(e, v[u].x, v[u].y);
-                    if (e + 1 < hi) add(e + 1, v[u].z, v[u].w);
+                    const int q = q0 + u * 32 + rot;
+                    const int64_t e = even + 2 * (q < n_pairs ? q : q - n_pairs);
+                    if (q0 + u * 32 < n_pairs) add_pair(e, v[u]);
                 }
             }
         }
@@ -2063,20 +2085,47 @@ cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream
     return cudaGetLastError();
 }
 
-// Whether an engine of these sizes can run many cycles per launch (0: no, 1: push form, 2: pull
-// form): half of a block's warps own neurons at most. An engine asked to deliver tiled takes the push
-// form too: the spikes are the same, and at these sizes a tiled cycle is a launch and a chain of
-// dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.3), and so does an AUTO engine
-// until a predictor is attached (38 x 874 neurons, 1-step delays: 13.0 us against 5.5): the choices of
-// the exact schedule are counted, the delivery is the push form's. Longer delays take one launch per cycle.
-int loop_form(const bsim_options &o, int64_t N, int32_t D, int sm_count)
+// Whether an engine of these sizes runs many cycles per launch (0: no, 1: push form, 2: pull form): half of
+// a block's warps own neurons at most. Longer delays take one launch per cycle.
+//
+// An engine asked to deliver tiled takes the push form too: the spikes are the same, and at these sizes
+// a tiled cycle is a launch and a chain of dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.2),
+// and so does an AUTO engine until a predictor is attached (38 x 874 neurons, 1-step delays: 13.0 us against
+// 5.5): the choices of the exact schedule are counted, the delivery is the push form's.
+//
+// Rows: a spike's whole row is one block's, so networks with many synapses in long rows are better spread
+// over the GPU by step_kernel, pushed or tiled. Up to LOOP_MAX_SYNAPSES, with rows of up to LOOP_LONG_ROW on
+// average where there are more than LOOP_ANY_ROW, the push form was faster than a pushed cycle or level on 20
+// networks of 100 Hz to 2 kHz with delays to 1, 6 and 50 steps (us per cycle, 500 Hz, 50 steps, push form /
+// pushed: 36 x 1,000 all-to-all, 4.2e7 synapses, 27 / 28; 15 x 1,500, 3.8e7, 30 / 30; 4 x 9,000 at 0.1,
+// 3.2e7, 18 / 25; 2 x 5,000, 2.5e7, 36 / 44; one population of 3,000, 9e6, 9 / 15), beyond it was not (12 x 3,000
+// at 0.5, 5.9e7, 37 / 34; 3 x 3,000 all-to-all, 2.7e7 in rows of 3,000, 17 / 15 and at 2 kHz 55 / 45).
+//
+// The pull form scans every row, half as often as step_kernel; a row is one warp's, so that one of
+// PULL_LOOP_MAX_ROW entries takes some 50 ms, far from the bound of the barrier's wait.
+#define LOOP_MAX_SYNAPSES 45000000
+#define LOOP_ANY_ROW 20000000
+#define LOOP_LONG_ROW 2500
+#define PULL_LOOP_MAX_ROW (1 << 22)
+int loop_form(const bsim_options &o, int64_t N, int32_t D, int64_t S, int64_t max_indeg, int sm_count)
 {
     const int64_t W = (N + 31) / 32;
     if (D > LOOP_MAX_DELAY || W > (int64_t)(LOOP_WARPS / 2) * sm_count) return 0;
     if (o.accumulate != BSIM_ACC_ORDERED && o.delivery != BSIM_DELIVERY_PULL)
-        return push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM ? 1 : 0;
+        return S <= LOOP_MAX_SYNAPSES && (S <= LOOP_ANY_ROW || S <= LOOP_LONG_ROW * N) &&
+                       push_loop_smem(N, D, sm_count) <= LOOP_MAX_SMEM
+                   ? 1
+                   : 0;
     const size_t bitmaps = sizeof(uint32_t) * (size_t)(D + LOOP_EXTRA_SLOTS + 1) * W;
-    return (o.accumulate == BSIM_ACC_ORDERED || o.delivery == BSIM_DELIVERY_PULL) && bitmaps + 8 <= PULL_LOOP_SMEM ? 2 : 0;
+    return max_indeg <= PULL_LOOP_MAX_ROW && bitmaps + 8 <= PULL_LOOP_SMEM ? 2 : 0;
+}
+
+// Cycles of one launch at most, so that it ends within about a second: 4,096 cycles of a few to 300 us
+// pushed; 4e11 row entries scanned.
+int64_t loop_launch_cycles(const Engine &e)
+{
+    const int64_t most = 4096;
+    return e.loop == 2 ? std::max<int64_t>(16, std::min(most, (int64_t)4e11 / std::max<int64_t>(e.S, 1))) : most;
 }
 
 cudaError_t launch_loop(Engine &e, int steps)
