@@ -495,6 +495,8 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     a.events = d_ctr + 1;
     a.ticket = reinterpret_cast<unsigned int *>(d_ctr + 2);
     a.tile_cycles = d_ctr + 3;
+    a.tile_prev = reinterpret_cast<unsigned int *>(d_ctr + 4);
+    a.cost_shift = e.D == 1 ? 3 : 0;
     a.loop_bar = d_ctr + 16;
     if (e.loop == 1) {
         a.acc_R = e.D + 3;

@@ -134,6 +134,8 @@ struct StepArgs {
     const int4 *items;               // [n_items] {tile, first unit, units, targets of the tile (its first item)}
     const int2 *run_item;            // [runs] first item of each run, delays per item
     unsigned int *item_clocks;       // [2][n_items] warp clocks spent, by cycle parity
+    int32_t cost_shift;              // item_clocks and tile_pairs keep 1 - 2^-cost_shift of the cycle before's (0: none)
+    unsigned int *tile_prev;         // whether the last cycle was delivered tiled
     unsigned int *tile_arrive;       // [2][n_tiles]: blocks that finished a piece of the tile this
                                      // cycle, and whether the first one's store is done (reset by
                                      // the last block)

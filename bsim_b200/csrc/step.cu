@@ -725,10 +725,18 @@ static __device__ __forceinline__ unsigned tile_unit_count(const StepArgs &a, in
 }
 // Cost of an item in warp clocks: what its chunks took in the previous cycle, a floor for its units'
 // scan, and for a tile's first item the start, the last warp and the flush of one part.
+//
+// With 1-step delays a cycle's spikes are those of the cycle before alone, and populations that fire
+// together every few cycles make each cycle unlike the last: there the clocks, and the pairs listed, are
+// means over the last cycles instead (each cycle keeps 1 - 2^-cost_shift of what was there, so that they
+// hold 2^cost_shift cycles' worth). At 2 kHz, us per cycle with the last cycle's alone / the means: 100 x
+// 10,000 670 / 375, 100 x 4,000 296 / 171, 20 x 5,000 all-to-all 802 / 355, 12 x 3,000 all-to-all 386 / 176;
+// at 500 Hz level. Of the costs alone, without the pairs that size the chunks and decide where blocks
+// help: 100 x 4,000 288.
 static __device__ __forceinline__ unsigned long long item_cost(const StepArgs &a, const unsigned *prev, int i)
 {
     const int4 it = a.items[i];  // {tile, first unit, units, targets of the tile in its first item}
-    return (unsigned long long)prev[i] + (unsigned long long)(TILE_UNIT_CLOCKS * it.z) +
+    return (unsigned long long)(prev[i] >> a.cost_shift) + (unsigned long long)(TILE_UNIT_CLOCKS * it.z) +
            (it.w ? (unsigned long long)(TILE_PART_CLOCKS + TILE_FLUSH_CLOCKS * it.w) : 0ull);
 }
 
@@ -832,7 +840,8 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
                 const unsigned hp = *reinterpret_cast<volatile unsigned *>(a.part_help + i);
                 // entry pairs left, about 8 per unit to scan, for each block then on it
                 const unsigned flush = (unsigned)(a.tile_beg[q + 1] - a.tile_beg[q]);
-                const float left = (float)(end - nx) * ((float)prev[q] / (float)tile_unit_count(a, q) + 8.0f) / (float)(hp + 2u);
+                const float per_unit = (float)(prev[q] >> a.cost_shift) / (float)tile_unit_count(a, q) + 8.0f;
+                const float left = (float)(end - nx) * per_unit / (float)(hp + 2u);
                 if (left < (float)flush) continue;
                 const unsigned long long key = ((unsigned long long)__float2uint_rz(left) << 32) | (unsigned)i;
                 best = key > best ? key : best;
@@ -858,9 +867,10 @@ static __device__ __forceinline__ unsigned long long tile_phase(const StepArgs &
         // free: 32 units (one per lane), fewer where the tile listed many entry pairs per unit in
         // the previous cycle, so that a hot chunk does not hold up the block for long
         unsigned *pairs_cnt = a.tile_pairs + (int64_t)(t & 1ull) * a.n_tiles + q;
-        const int cs = prev[q] == 0u ? 32
+        const unsigned prev_q = prev[q] >> a.cost_shift;
+        const int cs = prev_q == 0u ? 32
                                      : (int)max(TILE_MIN_CHUNK, min(32ll, (long long)TILE_CHUNK_PAIRS * a.tile_units[q] /
-                                                                              (long long)prev[q]));
+                                                                              (long long)prev_q));
         unsigned listed = 0;
         int pads = 0;
         // ring: the slot being filled and how far (64 pairs: two per lane), slots filled and not yet added
@@ -1238,7 +1248,11 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
         a.pred_sum[((t + 2) & 3) * 2 + 0] = 0.0f;
         a.pred_sum[((t + 2) & 3) * 2 + 1] = 0.0f;
     }
-    if (threadIdx.x == 0) s_ev = 0;
+    unsigned measured = 0;  // thread 0: whether the last cycle was delivered tiled
+    if (threadIdx.x == 0) {
+        s_ev = 0;
+        if (a.n_tiles > 0) measured = *reinterpret_cast<volatile unsigned *>(a.tile_prev);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // slot t+1 is neither written (LIF writes slot t) nor read (delivery reads t-1..t-D) now
         a.ring_cnt[(t + 1) % (unsigned long long)a.R] = 0;
@@ -1270,20 +1284,29 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     if (threadIdx.x == 0) {
         if (s_ev) atomicAdd(a.events, s_ev);
         __threadfence();
-        s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1 ? 1 + (int)measured : 0;
     }
     __syncthreads();
     if (s_last) {
         // every other block has finished this cycle: the tiles' finisher counts start over, and the
-        // next cycle counts its listed pairs from zero (whichever delivery this cycle used)
+        // next cycle counts its listed pairs and clocks from what cost_shift keeps of this one's (its
+        // places hold those of the cycle before this one, if that was delivered tiled, else nothing new)
         if (tiled)
             for (int i = threadIdx.x; i < 2 * a.n_tiles; i += blockDim.x) a.tile_arrive[i] = 0u;
-        for (int i = threadIdx.x; i < a.n_tiles; i += blockDim.x)
-            a.tile_pairs[(int64_t)((t + 1ull) & 1ull) * a.n_tiles + i] = 0u;
-        for (int i = threadIdx.x; i < a.n_items; i += blockDim.x)
-            a.item_clocks[(int64_t)((t + 1ull) & 1ull) * a.n_items + i] = 0u;
+        if (s_last == 2) {
+            const unsigned now = (unsigned)(t & 1ull), next = now ^ 1u;
+            auto keep = [&](unsigned *v, int n) {
+                for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                    const unsigned c = a.cost_shift ? __ldcg(v + (int64_t)now * n + i) : 0u;
+                    v[(int64_t)next * n + i] = c - (c >> a.cost_shift);
+                }
+            };
+            keep(a.tile_pairs, a.n_tiles);
+            keep(a.item_clocks, a.n_items);
+        }
         if (threadIdx.x == 0) {
-            if (tiled) *a.tile_cycles += 1ull;
+            if (a.n_tiles > 0) *a.tile_prev = tiled;
+            if (tiled) atomicAdd(a.tile_cycles, 1ull);
             // advance the cycle
             record_advance(a, t);
             *a.ticket = 0u;
