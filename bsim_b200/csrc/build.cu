@@ -26,6 +26,7 @@ cudaError_t launch_step(Engine &e);
 cudaError_t launch_record_flush(Engine &e);
 int loop_form(const bsim_options &o, int64_t N, int32_t D, int64_t S, int64_t max_indeg, int sm_count);
 int64_t loop_launch_cycles(const Engine &e);
+int push_split_of(int64_t S, int64_t N, int32_t D);
 cudaError_t launch_loop(Engine &e, int steps);
 cudaError_t launch_loop_enter(Engine &e);
 cudaError_t launch_loop_leave(Engine &e);
@@ -518,6 +519,7 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     // every cycle of a tiled-only engine overwrites the plane of the parity it
     // delivers into, so the LIF phase need not clear it; any other mode adds
     a.acc_clear = a.delivery == BSIM_DELIVERY_TILE ? 0 : 1;
+    a.push_split = push_split_of(e.S, e.N, e.D);
     // launch shape: all blocks resident (occupancy-sized grid), so the grid-stride
     // loops of both phases see every SM
     e.block = e.opt.block_threads > 0 ? e.opt.block_threads : 512;

@@ -104,6 +104,7 @@ struct StepArgs {
     int32_t acc_R;                    // D + 3
     int32_t *err;                  // device error flag (0 = ok)
     const int32_t *deliv_sel;      // per-step delivery choice written by the predictor (may be NULL)
+    int32_t push_split;            // pieces of one row at most, in pushed cycles with few spikes
     int32_t delivery;              // BSIM_DELIVERY_PUSH / _PULL when deliv_sel is NULL
     // raster recording (control words in device memory so a captured graph stays valid)
     int32_t *rec_ids;           // [rec->cap]

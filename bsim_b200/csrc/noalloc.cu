@@ -28,6 +28,7 @@
 namespace bsim {
 cudaError_t step_occupancy(int block, int accumulate, int *blocks_per_sm);
 cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream_t stream);
+int push_split_of(int64_t S, int64_t N, int32_t D);
 int record_error(int code, const std::string &msg);
 }  // namespace bsim
 
@@ -171,6 +172,7 @@ extern "C" int bsim_run_noalloc(int64_t n, int32_t max_delay, void *state_dev, c
     a.delivery = BSIM_DELIVERY_PUSH;
     a.n_pops = 1;
     a.acc_clear = 1;
+    a.push_split = push_split_of(n_synapses, n, max_delay);
 
     // The previous call's contents are still in the array: clear what must
     // start at zero (input accumulators of both parities, ring counts, bitmaps,

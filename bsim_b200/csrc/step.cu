@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "engine.h"
 
@@ -270,9 +271,8 @@ static __device__ __forceinline__ void push_one(const StepArgs &a, unsigned long
 #ifndef PUSH_CHUNK
 #define PUSH_CHUNK 8
 #endif
-#ifndef PUSH_MAX_SPLIT
-#define PUSH_MAX_SPLIT 32  // pieces of one row at most, in cycles with few long rows
-#endif
+#define PUSH_MAX_SPLIT 32   // pieces of one row at most, in cycles with few long rows
+#define PUSH_PASS 256       // entries a warp takes at once
 // resident blocks of STEP_MAX_THREADS threads the step kernel is compiled for
 // (together they set its register budget: 65,536 / (2 x 512) = 64 per thread)
 #ifndef STEP_MAX_THREADS
@@ -314,6 +314,13 @@ static __device__ __forceinline__ void delay_window_prefix(const StepArgs &a, un
     if (lane == 0) s_cum[0] = 0;
 }
 
+// Pieces that rows of a push cycle are cut into at most (S synapses in N rows of D segments).
+int push_split_of(int64_t S, int64_t N, int32_t D)
+{
+    const double mean = N > 0 ? (double)S / ((double)N * (double)D) : 0.0;
+    return (int)std::min((double)PUSH_MAX_SPLIT, std::max(1.0, std::floor(mean / PUSH_PASS + 0.5)));
+}
+
 // warp_lin of n_warps: this warp's number among those that deliver; s_seg: the warp's table.
 static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &a, unsigned long long t, int pw,
                                                                 const long long *s_cum, PushSeg *seg,
@@ -330,8 +337,11 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
     // block c % grid), so a cycle with few chunks still spreads over every SM.
     int pc = PUSH_CHUNK;
     while (pc > 1 && total < (long long)pc * n_warps) pc >>= 1;
-    // fewer segments than warps: each is cut into `split` pieces of whole pairs
-    const int split = total > 0 && 2 * total <= n_warps ? (int)min(n_warps / total, (long long)PUSH_MAX_SPLIT) : 1;
+    // fewer segments than warps: each is cut into `split` pieces of whole pairs, where rows are longer than
+    // one pass of a warp takes (push_split: cutting short ones only repeats the look-ups; us per cycle at 100
+    // Hz, 1-step delays, uncut / cut: rows of 120 entries, 20 x 1,000 neurons 8.9 / 11.3, 100 x 1,000
+    // 10.9 / 13.2; of 1,200, 25 x 10,000 20.7 / 16.5; of 5,700, 20 x 5,000 57.7 / 24.2)
+    const int split = a.push_split > 1 && total > 0 && 2 * total <= n_warps ? min((int)n_warps / (int)total, a.push_split) : 1;
     const long long n_chunks = split > 1 ? total * split : (total + pc - 1) / pc;
     for (long long ch = warp_lin; ch < n_chunks; ch += n_warps) {
         // Lanes 0..PUSH_CHUNK-1 each resolve one (spike, delay) segment: its row
@@ -339,7 +349,7 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
         // and an odd tail entry.
         int64_t r0 = 0, r1 = 0;
         float sc = 0.0f;
-        const long long item = split > 1 ? ch / split + lane : ch * pc + lane;
+        const long long item = split > 1 ? (int)ch / split + lane : ch * pc + lane;  // (split: n_chunks <= n_warps)
         if (lane < pc && item < total) {
             int lo = 1, hi = D;
             while (lo < hi) {
@@ -359,7 +369,7 @@ static __device__ __forceinline__ unsigned long long push_phase(const StepArgs &
             sc = __ldg(&a.ctab[a.cls[s]].scale_up);
             if (split > 1 && r1 > r0) {  // piece ch % split; inner cuts lie on 16-byte boundaries
                 const int64_t len = r1 - r0, b = r0;
-                const int k = (int)(ch % split);
+                const int k = (int)ch % split;
                 const int64_t lo = (b + len * k / split + 1) & ~1ll, hi = (b + len * (k + 1) / split + 1) & ~1ll;
                 if (k > 0) r0 = lo < r1 ? lo : r1;
                 if (k + 1 < split) r1 = hi < r1 ? hi : r1;
