@@ -508,7 +508,6 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     }
     a.delivery = (e.opt.delivery == BSIM_DELIVERY_PULL || e.opt.delivery == BSIM_DELIVERY_AUTO) ? e.opt.delivery
                                                                                                  : BSIM_DELIVERY_PUSH;
-    a.deliv_sel = nullptr;
     a.rec_ids = nullptr;
     a.rec_off = nullptr;
     a.rec = nullptr;
@@ -686,11 +685,9 @@ static int upload_tiles(Engine &e, const TileHost &th)
     const int32_t nt = (int32_t)th.tile_scale.size();
     const size_t nr = th.run_src0.size();
     int32_t *d_tb, *d_tro, *d_tu, *d_rn, *d_ru;
-    float *d_ts;
     uint32_t *d_rs;
     int64_t *d_rp;
     TRY(dalloc(e, &d_tb, th.n_u + 1));
-    TRY(dalloc(e, &d_ts, nt));
     TRY(dalloc(e, &d_tro, nt + 1));
     TRY(dalloc(e, &d_tu, nt));
     TRY(dalloc(e, &d_rs, nr));
@@ -698,7 +695,6 @@ static int upload_tiles(Engine &e, const TileHost &th)
     TRY(dalloc(e, &d_rp, nr));
     TRY(dalloc(e, &d_ru, nr));
     CK(cudaMemcpy(d_tb, th.tile_beg.data(), 4 * (th.n_u + 1), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_ts, th.tile_scale.data(), 4 * nt, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_tro, th.tile_run_off.data(), 4 * (nt + 1), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_tu, th.tile_units.data(), 4 * nt, cudaMemcpyHostToDevice));
     if (nr) {
@@ -747,7 +743,6 @@ static int upload_tiles(Engine &e, const TileHost &th)
     a.n_tiles = nt;
     a.tile_max = th.tile_max;
     a.tile_beg = d_tb;
-    a.tile_scale = d_ts;
     a.tile_run_off = d_tro;
     a.tile_units = d_tu;
     a.run_src0 = d_rs;

@@ -68,7 +68,7 @@ struct PredStats {
 struct StepArgs {
     int64_t N;         // neurons
     int32_t D;         // max delay, steps
-    int32_t R;         // ring slots = D + 2
+    int32_t R;         // ring slots: D + 2, D + LOOP_EXTRA_SLOTS in engines that run many cycles per launch
     int64_t cap;       // fired ids per ring slot
     int64_t W;         // bitmap words per ring slot = ceil(N / 32)
     float4 *state;     // [N] LIF: {v, i_E, i_I, refrac_step as int bits}
@@ -103,9 +103,8 @@ struct StepArgs {
     unsigned long long *loop_ev;      // [acc_R] events in flight by the cycle that delivers them
     int32_t acc_R;                    // D + 3
     int32_t *err;                  // device error flag (0 = ok)
-    const int32_t *deliv_sel;      // per-step delivery choice written by the predictor (may be NULL)
     int32_t push_split;            // pieces of one row at most, in pushed cycles with few spikes
-    int32_t delivery;              // BSIM_DELIVERY_PUSH / _PULL when deliv_sel is NULL
+    int32_t delivery;              // BSIM_DELIVERY_*
     // raster recording (control words in device memory so a captured graph stays valid)
     int32_t *rec_ids;           // [rec->cap]
     int64_t *rec_off;           // [rec->steps + 1]
@@ -142,7 +141,6 @@ struct StepArgs {
                                      // the last block)
     int32_t tile_max;                // largest range (neurons): shared-memory accumulator size
     const int32_t *tile_beg;         // [n_tiles + 1] first target of each tile
-    const float *tile_scale;         // [n_tiles] 2^qexp of the tile's network
     const int32_t *tile_run_off;     // [n_tiles + 1] range of runs
     const int32_t *tile_units;       // [n_tiles] work units: sum over runs of ceil(n/32) * D
     const uint32_t *run_src0;        // [runs] first source

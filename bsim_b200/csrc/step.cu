@@ -1241,7 +1241,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
     // the cycle's delivery mode, by one warp (the spike counts it reads are a hot spot when every warp
     // of the GPU reads them)
     if (threadIdx.x < 32) {
-        int dm = a.deliv_sel ? *a.deliv_sel : a.delivery;
+        int dm = a.delivery;
         if (ACC != BSIM_ACC_ORDERED && (dm == BSIM_DELIVERY_PUSH || dm == BSIM_DELIVERY_AUTO)) {
             // the window's counts are read once: for the push walk and for the choice
             delay_window_prefix(a, t, s_cum, [&](int slot) { return __ldcg(&a.ring_cnt[slot]); });
@@ -1527,11 +1527,6 @@ static __device__ __forceinline__ void loop_append(const StepArgs &a, unsigned l
         const unsigned same = __match_any_sync(0xffffffffu, fired ? pop : -1);
         if (fired && lane == __ffs(same) - 1) atomicAdd(&hist[pop], __popc(same));
     }
-}
-
-static __device__ __forceinline__ const float *drive_vtmp(const StepArgs &a, unsigned long long t)
-{
-    return (a.drive_half > 0 && ((t / (unsigned long long)a.drive_half) & 1ull)) ? a.vtmp_alt : a.vtmp;
 }
 
 struct LoopSpike {
