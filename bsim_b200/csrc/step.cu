@@ -10,7 +10,7 @@
 // bandwidth-bound update fills the tail of the delivery.
 //
 // The two halves touch disjoint data (the input accumulators are double
-// buffered by cycle parity, the fire ring has D+2 slots), so they need no
+// buffered by cycle parity, the fire ring has at least D+2 slots), so they need no
 // barrier between them; the kernel boundary orders consecutive cycles.
 // The cycle counter lives on the device and is advanced by the last block to
 // finish, so the same launch can be replayed from a CUDA graph with no host
@@ -637,8 +637,6 @@ static __device__ __forceinline__ unsigned long long pull_phase(const StepArgs &
 
 // Counters are [4][tile]: E low, E high, I low, I high words (word-major, so
 // lanes adding into scattered targets spread over all shared-memory banks).
-// Two entries at once: both low words first, so the second atomic's latency
-// overlaps the first's (a returned value is waited for only where it is used).
 // acc: shared-memory address of the counters; hi: bytes from a low word to its high word. The
 // addresses are 32-bit shared-memory ones throughout: through a generic pointer the compiler
 // emits both kinds of atomic and a compare-and-swap loop, ten shared accesses per addition.
@@ -1344,8 +1342,8 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 //     are run between barriers: both updates, then the rows of both cycles' spikes.
 //     Owners take groups of eight consecutive neurons dealt out over all blocks, so
 //     that a population that fires together spreads over the GPU.
-//     10 x 1,000 neurons (100 Hz): 10.2 -> 3.3 us per cycle; 5,000 neurons behind
-//     Poisson drives 13.7 -> 3.9; 20 x 1,000 all-to-all 18.1 -> 6.2.
+//     10 x 1,000 neurons (100 Hz): 10.2 -> 3.2 us per cycle; 5,000 neurons behind
+//     Poisson drives 13.7 -> 3.7; 20 x 1,000 all-to-all 18.1 -> 6.0.
 //   * Pull (and the ORDERED sums): a block sums the input of its own neurons, so the update
 //     follows without a barrier and again two cycles are run between barriers: the input of
 //     cycle t takes the spikes up to t - 2, that of t + 1 those up to t - 1, and one scan of
@@ -1685,22 +1683,26 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
                 red_add_u64(reinterpret_cast<unsigned long long *>(acc + (int64_t)sl * a.N + tgt) + (w >= 0.0f ? 0 : 1),
                             (unsigned long long)q);
             };
-            // the segments that hold entries e and e + 1, one search for both
-            auto add_pair = [&](int64_t e, uint4 v) {
+            // entries by their places in the row: [from, to) here, in pairs from an even position
+            const int from = (int)(lo - r0), to = (int)(hi - r0), first = (int)((lo & ~1ll) - r0);
+            const int n_pairs = (to - first + 1) >> 1;
+            const uint4 *pairs = reinterpret_cast<const uint4 *>(a.syn + r0 + first);
+            // the segments that hold entries x and x + 1, one search for both
+            auto add_pair = [&](int x, uint4 v) {
                 int d = 0;
                 if (D > 1) {
-                    const unsigned x = (unsigned)(max(e, lo) - r0);
+                    const unsigned y = (unsigned)max(x, from);
                     int top = D - 1;
                     while (d < top) {
                         const int mid = (d + top + 1) >> 1;
-                        if (off[mid] <= x) d = mid;
+                        if (off[mid] <= y) d = mid;
                         else top = mid - 1;
                     }
                 }
-                if (e >= lo) add(d, v.x, v.y);
-                if (e + 1 < hi) {
+                if (x >= from) add(d, v.x, v.y);
+                if (x + 1 < to) {
                     if (D > 1)
-                        while (off[d + 1] <= (unsigned)(e + 1 - r0)) d++;
+                        while (off[d + 1] <= (unsigned)(x + 1)) d++;
                     add(d, v.z, v.w);
                 }
             };
@@ -1717,22 +1719,19 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
             // of both entries of a pair (us per cycle, before / after: 2 x 6,000 neurons at p = 0.5,
             // 2 kHz, 1-step delays 79 / 64, 50-step delays 80 / 60; 10 x 1,000 all-to-all, 500 Hz,
             // 10.4 / 10.1 and 16.2 / 12.6).
-            const int64_t even = lo & ~1ll;
-            const int n_pairs = (int)((hi - even + 1) >> 1);
             const int rot = (int)__umulhi((unsigned)sp.who * 2654435769u + blockIdx.x * 2246822519u, (unsigned)n_pairs);
             for (int q0 = lane; q0 < n_pairs; q0 += 4 * 32) {
                 uint4 v[4];
+                int at[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const int q = q0 + u * 32 + rot;
-                    if (q0 + u * 32 < n_pairs) v[u] = __ldg(reinterpret_cast<const uint4 *>(a.syn + even + 2 * (q < n_pairs ? q : q - n_pairs)));
+                    at[u] = q0 + u * 32 + rot;
+                    if (at[u] >= n_pairs) at[u] -= n_pairs;
+                    if (q0 + u * 32 < n_pairs) v[u] = __ldg(pairs + at[u]);
                 }
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int q = q0 + u * 32 + rot;
-                    const int64_t e = even + 2 * (q < n_pairs ? q : q - n_pairs);
-                    if (q0 + u * 32 < n_pairs) add_pair(e, v[u]);
-                }
+                for (int u = 0; u < 4; u++)
+                    if (q0 + u * 32 < n_pairs) add_pair(first + 2 * at[u], v[u]);
             }
         }
         // ---- history: fired flags and the fire ring (not read by this launch's delivery)
