@@ -523,7 +523,8 @@ static int finish_engine(Engine &e, const std::vector<ClassParams> &ctab)
     // loops of both phases see every SM
     e.block = e.opt.block_threads > 0 ? e.opt.block_threads : 512;
     if (e.block % 32 != 0 || e.block > 512) return fail(BSIM_ERR_ARG, "block_threads must be a multiple of 32 <= 512");
-    // 2 ring slots per warp (4 entry pairs per lane); one where that lets two blocks share an SM, or one fit
+    // ring slots per warp (64 entry pairs each): as many as TILE_MAX_DEPTH, fewer where that lets more
+    // blocks share an SM, or one fit
     int bps = 0;
     for (int depth = TILE_MAX_DEPTH, best = 0; depth >= 1; depth--) {
         StepArgs b = a;

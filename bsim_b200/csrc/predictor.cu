@@ -43,8 +43,9 @@ int fail(int code, const std::string &m, cudaError_t st = cudaSuccess)
 // update and clears the gradients, so a training step is one launch.
 //
 // Measured against one thread per sample and 64 samples per block, with gathering, clearing and
-// the update as launches of their own: one epoch over 65,001 host samples in batches of 8,192, 3.6 ms
-// -> 1.6 ms a call (the rest is allocation and the samples' way to the GPU).
+// the update as launches of their own: one epoch over 65,001 host samples in batches of 8,192, medians
+// of 80 calls 2.9 to 3.3 ms -> 1.5 to 1.7 ms (5th to 95th percentile 2.8 to 3.8 and 1.5 to 1.9 without
+// stragglers; the rest is mostly allocation, the shuffle and the samples' way to the GPU).
 enum { MLP_FORWARD, MLP_LOSS, MLP_GRAD };
 constexpr int GT = 64, LD = H + 4, MLP_THREADS = 256;
 constexpr int64_t MLP_MAX_BLOCKS = 4096;  // blocks of a large pass take several tiles

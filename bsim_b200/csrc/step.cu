@@ -1342,7 +1342,7 @@ __global__ void __launch_bounds__(STEP_MAX_THREADS, STEP_MIN_BLOCKS) step_kernel
 //     are run between barriers: both updates, then the rows of both cycles' spikes.
 //     Owners take groups of eight consecutive neurons dealt out over all blocks, so
 //     that a population that fires together spreads over the GPU.
-//     10 x 1,000 neurons (100 Hz): 10.2 -> 3.2 us per cycle; 5,000 neurons behind
+//     10 x 1,000 neurons (100 Hz): 10.2 -> 3.1 us per cycle; 5,000 neurons behind
 //     Poisson drives 13.7 -> 3.7; 20 x 1,000 all-to-all 18.1 -> 6.0.
 //   * Pull (and the ORDERED sums): a block sums the input of its own neurons, so the update
 //     follows without a barrier and again two cycles are run between barriers: the input of
@@ -1717,8 +1717,8 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) push_loop_kernel(const __grid
             // walked from a point of its own, wrapping around, so that blocks whose rows hit the same
             // targets do not add into the same addresses in lockstep, and one search finds the delays
             // of both entries of a pair (us per cycle, before / after: 2 x 6,000 neurons at p = 0.5,
-            // 2 kHz, 1-step delays 79 / 64, 50-step delays 80 / 60; 10 x 1,000 all-to-all, 500 Hz,
-            // 10.4 / 10.1 and 16.2 / 12.6).
+            // 2 kHz, 1-step delays 79 / 64, 50-step delays 80 / 59; 10 x 1,000 all-to-all, 500 Hz,
+            // 10.4 / 10.0 and 16.2 / 12.3; 10 x 1,000 at 0.1, 100 Hz, 6-step delays 3.19 / 3.05).
             const int rot = (int)__umulhi((unsigned)sp.who * 2654435769u + blockIdx.x * 2246822519u, (unsigned)n_pairs);
             for (int q0 = lane; q0 < n_pairs; q0 += 4 * 32) {
                 uint4 v[4];
@@ -2116,7 +2116,7 @@ cudaError_t launch_step_exact(const StepArgs &a, int grid, int block, cudaStream
 // a block's warps own neurons at most. Longer delays take one launch per cycle.
 //
 // An engine asked to deliver tiled takes the push form too: the spikes are the same, and at these sizes
-// a tiled cycle is a launch and a chain of dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.2),
+// a tiled cycle is a launch and a chain of dependent reads (10 x 1,000 neurons, 100 Hz: 15.5 us against 3.1),
 // and so does an AUTO engine until a predictor is attached (38 x 874 neurons, 1-step delays: 13.0 us against
 // 5.5): the choices of the exact schedule are counted, the delivery is the push form's.
 //

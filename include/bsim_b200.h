@@ -73,13 +73,15 @@ typedef struct bsim_options {
     int32_t accumulate;    /* BSIM_ACC_* */
     int32_t delivery;      /* BSIM_DELIVERY_* */
     int32_t build_pull;    /* also build the target-ordered copy (forced on for PULL and ORDERED) */
-    int32_t graph_steps;   /* steps captured per CUDA graph by bsim_run; networks of a few ten thousand neurons run
-                              many steps per launch instead (0: one plain launch per step) */
+    int32_t graph_steps;   /* steps captured per CUDA graph by bsim_run; networks of a few ten thousand neurons and
+                              million synapses run many steps per launch instead (bsim_info.many_cycles tells;
+                              0: one plain launch per step) */
     int32_t block_threads; /* threads per block of the step kernel (0: autotuned) */
     int32_t grid_blocks;   /* blocks of the step kernel (0: autotuned) */
     int32_t build_tiles;   /* 1: also build the target-tiled copy; 0: for TILE/AUTO, and for large generated
-                              PUSH networks (their busy cycles are delivered from it); -1: never (an AUTO
-                              engine then pushes every cycle; saves ~8 B per synapse) */
+                              PUSH networks whose busy cycles are cheaper delivered from it and where a
+                              quarter of the device's memory stays free (bsim_info.n_tiles tells); -1: never
+                              (an AUTO engine then pushes every cycle; saves ~8 B per synapse) */
     int32_t tile_size;     /* target neurons per tile (0: chosen from the network size and delays, <= 5000) */
     int32_t reserved[7];
 } bsim_options;
