@@ -1,6 +1,7 @@
 """Several host threads on one engine: reads while another thread runs it are of one moment each."""
 import hashlib
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -58,6 +59,8 @@ def test_reads_while_another_thread_runs(n):
         t.start()
     for k in range(steps):
         eng.run(1)
+        while len(seen) < k // 5 and not errors:  # the readers keep up
+            time.sleep(1e-4)
     done.set()
     for t in threads:
         t.join()
